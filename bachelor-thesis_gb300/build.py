@@ -18,7 +18,7 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-O2",
                      "--expt-relaxed-constexpr", "-I" + os.path.join(HERE, "..", "include")]
 
-LIB_SOURCES = ["host.cpp", "limb.cu", "crt.cu", "batch.cpp", "mlp.cu", "pipeline.cpp"]
+LIB_SOURCES = ["host.cpp", "limb.cu", "limb_tc.cu", "crt.cu", "batch.cpp", "mlp.cu", "pipeline.cpp"]
 CLI_SOURCES = ["cli.cpp"]
 
 
@@ -45,7 +45,7 @@ def build(verbose=False, force=False, extra_flags=()):
     """Compiles the library; returns the path of libgbmm.so.  Raises on failure."""
     os.makedirs(OUT, exist_ok=True)
     nvcc = _nvcc()
-    headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".h")]
+    headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh"))]
     headers.append(os.path.join(HERE, "..", "include", "gbmm.h"))
     jobs = []
     objs = []

@@ -86,6 +86,8 @@ gbmm_status launch_split_sizes(const gbmm_mat &x, int h, int32_t *lo, int32_t *h
 gbmm_status launch_add_shifted(const gbmm_mat &w, const gbmm_mat &u, const gbmm_mat &v, int sh, cudaStream_t s);
 // whether the per-entry product kernel handles la x lb limb entries
 bool limb_kernel_fits(int la, int lb);
+// measured rate of that kernel on long sums, in 10^12 32-bit MAC/s, for `entries` results
+double limb_rate(int la, int lb, int64_t entries);
 // whether the batched basecase product stages un x vn limb operands on chip
 bool mpn_basecase_on_chip(int un, int vn);
 
@@ -108,6 +110,16 @@ struct WinoTree {
 gbmm_status launch_wino_sums(const WinoTree &t, int d, cudaStream_t s);
 gbmm_status launch_wino_leaves(const WinoTree &t, cudaStream_t s);
 gbmm_status launch_wino_combine(const WinoTree &t, int d, cudaStream_t s);
+
+// ---- the limb form's product on the tensor cores (limb_tc.cu) -------------------------
+// whether `leaves` products of these shapes run faster there than on the per-entry
+// kernel, their workspace, and the products; *done = false (nothing launched) when the
+// handle's workspace has no room
+bool ltc_pays(int m, int k, int n, int la, int lb, int64_t leaves);
+size_t ltc_ws(int m, int k, int n, int la, int lb, int64_t leaves);
+gbmm_status ltc_matmul(gbmm_handle h, const gbmm_mat &c, const gbmm_mat &a, const gbmm_mat &b, int accumulate,
+                       cudaStream_t s, bool *done);
+gbmm_status ltc_wino_leaves(gbmm_handle h, const WinoTree &t, int64_t leaves, cudaStream_t s, bool *done);
 
 // ---- CRT path (crt.cu) --------------------------------------------------------------
 struct crt_cache;
@@ -221,6 +233,10 @@ gbmm_status wino_crt(gbmm_handle h, const gbmm_mat &c, const gbmm_mat &a, const 
 size_t crt_group_job_ws(const Plan &p, int la, int lb, int m, int k, int n);
 gbmm_status crt_collect(gbmm_handle h, crt_group *g, const gbmm_mat &c, const gbmm_mat &a, const gbmm_mat &b,
                         const Plan &p);
+// extra workspace with which dispatch() runs its limb products on the tensor cores
+size_t limb_tc_extra(const Plan &p, int la, int lb, int m, int k, int n);
+// Reserves `ws` bytes, with `extra` more when they can be had; *got says whether
+gbmm_status arena_reserve_extra(gbmm_handle h, size_t ws, size_t extra, bool *got);
 gbmm_status resolve_plan(gbmm_handle h, const gbmm_mat &a, const gbmm_mat &b, const gbmm_opts &o, Plan &p);
 void invalidate_graphs(gbmm_handle h);
 void batch_state_destroy(gbmm_handle h);
@@ -249,6 +265,9 @@ struct gbmm_handle_s {
     int limb_cutoff = 32;
     // Winograd products as one breadth-first tree (1, default) or depth first (0)
     int wino_breadth_first = 1;
+    // limb products may use the tensor-core form (1 while a call holds a workspace
+    // reserved with room for it; batches, whose streams own fixed slices, leave it 0)
+    int limb_tc = 0;
     // CRT GEMM tile form for the next product (set around each CRT call by dispatch):
     // 0 by size, 1 one-CTA tiles, 2 CTA-pair tiles for the product and reconstruction
     int crt_tiles = 0;

@@ -719,6 +719,19 @@ static unsigned remove_factors(unsigned n, unsigned b) { while (n && n % b == 0)
 
 static gbmm_mat with_limbs(gbmm_mat m, int nl) { m.nlimbs = nl; return m; }
 
+// One product without recursion: on the tensor cores where that is faster and the
+// workspace has room, else the per-entry kernel.
+gbmm_status limb_product(gbmm_handle h, const gbmm_mat &C, const gbmm_mat &A, const gbmm_mat &B, int accumulate,
+                         cudaStream_t s) {
+    if (h->limb_tc && limb_kernel_fits(A.nlimbs, B.nlimbs) &&
+        ltc_pays(A.rows, A.cols, B.cols, A.nlimbs, B.nlimbs, 1)) {
+        bool done = false;
+        GBMM_TRY(ltc_matmul(h, C, A, B, accumulate, s, &done));
+        if (done) return GBMM_OK;
+    }
+    return launch_limb_matmul(C, A, B, accumulate, s);
+}
+
 gbmm_status rec_square(RecCtx &c, int method, gbmm_mat C, gbmm_mat A, gbmm_mat B, int N, int levels, int addmul);
 
 // Winograd's 7-product scheme with 3 temporaries; the operation order is that
@@ -922,7 +935,12 @@ gbmm_status rec_winograd_bf(RecCtx &c, gbmm_mat C, gbmm_mat A, gbmm_mat B, int N
     }
     gbmm_status st = GBMM_OK;
     for (int d = 1; d <= levels && st == GBMM_OK; d++) st = launch_wino_sums(t, d, c.s);
-    if (st == GBMM_OK) st = launch_wino_leaves(t, c.s);
+    if (st == GBMM_OK) {
+        bool done = false;
+        const int hl = N >> levels;
+        if (c.h->limb_tc && ltc_pays(hl, hl, hl, t.capSA, t.capSB, np)) st = ltc_wino_leaves(c.h, t, np, c.s, &done);
+        if (st == GBMM_OK && !done) st = launch_wino_leaves(t, c.s);
+    }
     for (int d = levels; d >= 1 && st == GBMM_OK; d--) st = launch_wino_combine(t, d, c.s);
     arena_release(c.h, mark);
     return st;
@@ -931,17 +949,17 @@ gbmm_status rec_winograd_bf(RecCtx &c, gbmm_mat C, gbmm_mat A, gbmm_mat B, int N
 gbmm_status rec_square(RecCtx &c, int method, gbmm_mat C, gbmm_mat A, gbmm_mat B, int N, int levels, int addmul) {
     // recursion is skipped when the one-limb-longer sums it forms would not fit the per-entry kernel
     if (levels <= 0 || N % 2 != 0 || N / 2 < 1 || !limb_kernel_fits(c.capSA, c.capSB))
-        return launch_limb_matmul(C, A, B, addmul, c.s);
+        return limb_product(c.h, C, A, B, addmul, c.s);
     if (c.breadth_first && wino_bf_ok(method, N, levels, addmul, c.capSA, c.capSB, c.capP))
         return rec_winograd_bf(c, C, A, B, N, levels);
     // depth first from here down (the workspace was sized for that)
     RecCtx dc = c;
     dc.breadth_first = false;
     if (method == GBMM_METHOD_WINOGRAD) return rec_winograd(dc, C, A, B, N, levels, addmul);
-    if (addmul) return launch_limb_matmul(C, A, B, 1, c.s);
+    if (addmul) return limb_product(c.h, C, A, B, 1, c.s);
     if (method == GBMM_METHOD_STRASSEN) return rec_strassen(dc, C, A, B, N, levels);
     if (method == GBMM_METHOD_NAIVE_REC) return rec_naive(dc, C, A, B, N, levels);
-    return launch_limb_matmul(C, A, B, 0, c.s);
+    return limb_product(c.h, C, A, B, 0, c.s);
 }
 
 static int levels_for(int N, int cutoff) {
@@ -975,7 +993,7 @@ gbmm_status squarify(RecCtx &c, int method, gbmm_mat C, gbmm_mat A, gbmm_mat B) 
     if (K == 0 || N == 0) return GBMM_OK;
     if (M == 0) return launch_mat_zero(C, c.s);
     const int base = c.cutoff;
-    if (method == GBMM_METHOD_NAIVE || K <= base || M <= base || N <= base) return launch_limb_matmul(C, A, B, 0, c.s);
+    if (method == GBMM_METHOD_NAIVE || K <= base || M <= base || N <= base) return limb_product(c.h, C, A, B, 0, c.s);
     if (K == M && M == N && remove_factors((unsigned)K, 2) <= (unsigned)base)
         return rec_square(c, method, C, A, B, K, levels_for(K, base), 0);
     int mindim = std::min(std::min(K, M), N);
@@ -1051,7 +1069,7 @@ gbmm_status matmul_limb(gbmm_handle h, const gbmm_mat &c, const gbmm_mat &a, con
                         int accumulate, cudaStream_t s) {
     if (accumulate && (method == GBMM_METHOD_NAIVE || a.rows != a.cols || a.cols != b.cols ||
                        remove_factors((unsigned)a.rows, 2) > (unsigned)cutoff || method != GBMM_METHOD_WINOGRAD))
-        return launch_limb_matmul(c, a, b, 1, s);
+        return limb_product(h, c, a, b, 1, s);
     RecCtx ctx;
     ctx.h = h;
     ctx.s = s;
@@ -1293,6 +1311,46 @@ size_t dispatch_ws(const Plan &p, int la, int lb, int m, int k, int n, int cn, i
     return own + dispatch_ws(q, sa ? hn : la, sa ? lb : hn, sa ? 2 * m : m, k, sa ? n : 2 * n, tn, 0);
 }
 
+// Extra workspace for dispatch()'s limb products on the tensor cores: that of the whole
+// product bounds every sub-product of a recursion, and the breadth-first tree's leaves
+// take what a share of the device allows (several launches when they need more).
+size_t limb_tc_extra(const Plan &p, int la, int lb, int m, int k, int n) {
+    constexpr size_t MAX_BYTES = (size_t)4 << 30, WINO_BYTES = (size_t)1 << 30;
+    if (p.path != GBMM_PATH_LIMB || m == 0 || n == 0 || k == 0) return 0;
+    if (!direct_ok(p, la, lb, k)) {
+        const bool sa = la >= lb;
+        const int xl = sa ? la : lb;
+        if (xl < 2) return 0;
+        Plan q = p;
+        q.split = std::max(0, p.split - 1);
+        const int hn = xl - xl / 2;
+        return limb_tc_extra(q, sa ? hn : la, sa ? lb : hn, sa ? 2 * m : m, k, sa ? n : 2 * n);
+    }
+    const int up = p.method == GBMM_METHOD_NAIVE ? 0 : 1;  // sums have one limb more
+    size_t x = 0;
+    if (ltc_pays(m, k, n, la + up, lb + up, 1)) x = ltc_ws(m, k, n, la + up, lb + up, 1) + 4096;
+    if (p.method == GBMM_METHOD_WINOGRAD && m == k && k == n) {
+        const int L = levels_for(m, p.cutoff), hl = m >> L;
+        if (L >= 1 && L <= WINO_MAX_LEVELS && ltc_pays(hl, hl, hl, la + 1, lb + 1, pow7_h(L))) {
+            const size_t per = ltc_ws(hl, hl, hl, la + 1, lb + 1, 1) + 4096;
+            x = std::max(x, per * (size_t)std::min<int64_t>(pow7_h(L), std::max<int64_t>(64, (int64_t)(WINO_BYTES / per))));
+        }
+    }
+    return x <= MAX_BYTES ? x : 0;
+}
+
+gbmm_status arena_reserve_extra(gbmm_handle h, size_t ws, size_t extra, bool *got) {
+    *got = false;
+    if (extra) {
+        if (arena_reserve(h, ws + extra) == GBMM_OK) {
+            *got = true;
+            return GBMM_OK;
+        }
+        cudaGetLastError();  // a failed allocation: run without the extra
+    }
+    return arena_reserve(h, ws);
+}
+
 // C (+)= A*B with the planned path.  An operand too long for the chosen kernels
 // is split into low and high limb halves, X = X_hi 2^(32h) + X_lo (the
 // Karatsuba-style split of Knuth 4.3.3 without the middle-product trick), and
@@ -1485,8 +1543,13 @@ extern "C" gbmm_status gbmm_matmul(gbmm_handle h, gbmm_mat c, gbmm_mat a, gbmm_m
     if (opts) o = *opts;
     Plan p;
     GBMM_TRY(resolve_plan(h, a, b, o, p));
-    GBMM_TRY(arena_reserve(h, dispatch_ws(p, a.nlimbs, b.nlimbs, a.rows, a.cols, b.cols, c.nlimbs, o.accumulate) + 65536));
-    return dispatch(h, c, a, b, p, o.accumulate, h->stream);
+    bool tc = false;
+    GBMM_TRY(arena_reserve_extra(h, dispatch_ws(p, a.nlimbs, b.nlimbs, a.rows, a.cols, b.cols, c.nlimbs, o.accumulate) + 65536,
+                                 limb_tc_extra(p, a.nlimbs, b.nlimbs, a.rows, a.cols, b.cols), &tc));
+    h->limb_tc = tc;
+    const gbmm_status st = dispatch(h, c, a, b, p, o.accumulate, h->stream);
+    h->limb_tc = 0;
+    return st;
 }
 
 extern "C" gbmm_status gbmm_mpn_mul(gbmm_handle h, uint32_t *rp, const uint32_t *up, int32_t un, const uint32_t *vp,

@@ -24,12 +24,11 @@
 #include <vector>
 
 #include "gbmm_internal.h"
+#include "limb_dev.cuh"
 
 namespace gbmm {
 
 // ---- small device helpers ---------------------------------------------------------
-__device__ __forceinline__ int iabs_d(int x) { return x < 0 ? -x : x; }
-
 // 96-bit column accumulator (c0, c1, c2) += a * b.  One 32x32->64 wide multiply
 // accumulating into c0, then the high word and the carry.
 // The three instructions share the carry flag, so they stay in one asm block.
@@ -39,19 +38,6 @@ __device__ __forceinline__ int iabs_d(int x) { return x < 0 ? -x : x; }
         "addc.u32 %2, %2, 0;"                                                     \
         : "+r"(c0), "+r"(c1), "+r"(c2)                                            \
         : "r"(a), "r"(b))
-
-struct MatArgs {
-    uint32_t *limbs;
-    int32_t *sizes;
-    int64_t rs, ld;
-    int32_t rows, cols, nlimbs;
-};
-__host__ __device__ static inline MatArgs margs(const gbmm_mat &m) {
-    MatArgs a;
-    a.limbs = m.limbs; a.sizes = m.sizes; a.rs = m.rs; a.ld = m.ld;
-    a.rows = m.rows; a.cols = m.cols; a.nlimbs = m.nlimbs;
-    return a;
-}
 
 // ======================================================================================
 // mpn add_n / sub_n with warp-level carry-lookahead.
@@ -1578,57 +1564,6 @@ __global__ void __launch_bounds__(NT, NT <= MM_THREADS ? 2 : 1)
 // Every operand view is computed on the device from the node's index path, so
 // a launch takes no job table and the sequence can be captured in a graph.
 // ======================================================================================
-__device__ __forceinline__ MatArgs wt_quad(MatArgs m, int qr, int qc, int h) {
-    const int64_t off = (int64_t)qr * h * m.rs + (int64_t)qc * h;
-    m.limbs += off;
-    m.sizes += off;
-    m.rows = h;
-    m.cols = h;
-    return m;
-}
-__device__ __forceinline__ MatArgs wt_dense(uint32_t *limbs, int32_t *sizes, int64_t q, int h, int cap) {
-    MatArgs m;
-    const int64_t e = (int64_t)h * h;
-    m.limbs = limbs + q * e * cap;
-    m.sizes = sizes + q * e;
-    m.rs = h;
-    m.ld = e;
-    m.rows = h;
-    m.cols = h;
-    m.nlimbs = cap;
-    return m;
-}
-// Operand `which` (0: A, 1: B) of node `node` at level d.
-__device__ MatArgs wt_operand(const WinoTree &t, int which, int d, int64_t node) {
-    MatArgs v = margs(which ? t.B : t.A);
-    int h = t.N;
-    int64_t pw = 1;
-    for (int l = 1; l < d; l++) pw *= 7;
-    for (int l = 1; l <= d; l++) {
-        const int64_t self = node / pw;  // this node's ancestor at level l
-        const int j = (int)(self % 7);
-        const int64_t parent = self / 7;
-        h >>= 1;
-        int s = -1;
-        if (which == 0) {
-            if (j == 0) v = wt_quad(v, 0, 0, h);
-            else if (j == 1) v = wt_quad(v, 0, 1, h);
-            else if (j == 3) v = wt_quad(v, 1, 1, h);
-            else s = j == 2 ? 3 : j - 4;
-        } else {
-            if (j == 0) v = wt_quad(v, 0, 0, h);
-            else if (j == 1) v = wt_quad(v, 1, 0, h);
-            else if (j == 2) v = wt_quad(v, 1, 1, h);
-            else s = j == 3 ? 3 : j - 4;
-        }
-        if (s >= 0)
-            v = which ? wt_dense(t.sb_limbs[l], t.sb_sizes[l], 4 * parent + s, h, t.capSB)
-                      : wt_dense(t.sa_limbs[l], t.sa_sizes[l], 4 * parent + s, h, t.capSA);
-        pw /= 7;
-    }
-    return v;
-}
-
 // Level d's sums: one thread per (operand side, parent, entry of the h x h quadrants).
 __global__ void k_wino_sums(WinoTree t, int d, int64_t nparents, int h, uint32_t *err) {
     const int64_t hh = (int64_t)h * h;
@@ -1897,6 +1832,16 @@ static void finish_cfg(MMCfg &cfg, int M, int accumulate) {
 bool limb_kernel_fits(int la, int lb) {
     MMCfg cfg;
     return choose_mm(la, lb, cfg);
+}
+
+double limb_rate(int la, int lb, int64_t entries) {
+    MMCfg cfg;
+    if (!choose_mm(la, lb, cfg)) return 1.0;
+    // one thread per entry: it takes about 40 thousand entries to fill the GPU
+    if (cfg.G == 1) return 1.9 * std::min(1.0, entries / 41000.0);
+    const bool thin = cfg.thinA || cfg.thinB;
+    const double rate = cfg.R == 8 ? 4.8 : cfg.R == 4 ? (thin ? 2.7 : 3.4) : (thin ? 1.4 : 1.85);
+    return rate * std::min(1.0, (double)entries * cfg.Gp / (152.0 * 512));
 }
 
 static size_t mm_smem(const MMCfg &c) {

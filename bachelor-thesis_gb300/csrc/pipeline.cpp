@@ -378,8 +378,12 @@ extern "C" gbmm_status gbmm_matmul_host(gbmm_handle h, gbmm_host_job *jobs, int3
             h->stage = &hooks;
         }
         // the plan resolved above runs as is, so the staging decision and the product agree
-        st = arena_reserve(h, dispatch_ws(p, q.a_nlimbs, q.b_nlimbs, q.K, q.M, q.N, q.c_nlimbs, 0) + 65536);
+        bool tc = false;
+        st = arena_reserve_extra(h, dispatch_ws(p, q.a_nlimbs, q.b_nlimbs, q.K, q.M, q.N, q.c_nlimbs, 0) + 65536,
+                                 h->dev_budget ? 0 : limb_tc_extra(p, q.a_nlimbs, q.b_nlimbs, q.K, q.M, q.N), &tc);
+        h->limb_tc = tc;
         if (st == GBMM_OK) st = dispatch(h, C, A, B, p, 0, h->stream);
+        h->limb_tc = 0;
         h->stage = nullptr;
         if (st == GBMM_OK) st = ck(cudaEventRecord(s.computed, h->stream), "cudaEventRecord");
         // download: the whole of C after the compute, or each finished entry range
