@@ -517,15 +517,18 @@ __device__ __forceinline__ void sm_stage_map(uint32_t *dst, int SS, int nchunks,
 // zero-padded), by block product scanning: column block T gathers the 4 x 4
 // blocks (I, T - I); their 7 columns are summed in 96-bit accumulators, the
 // block's four columns absorb the carry from below and go out in ascending
-// order (out(t, limb) for t < 4 (nu4 + nv4)), the upper three seed the next block.
-template <class Out>
-__device__ __forceinline__ void sm_mul4(const uint32_t *u, int nu4, const uint32_t *v, int nv4, Out out) {
+// order (out(T, c, limb): limb 4 T + c), the upper three seed the next block.
+// pre(T) runs before block T's MACs (loads it issues are in flight during them);
+// blocks nu4 + nv4 .. nT - 1 only pass the carry on.
+template <class Pre, class Out>
+__device__ __forceinline__ void sm_mul4_pre(const uint32_t *u, int nu4, const uint32_t *v, int nv4, int nT, Pre pre,
+                                            Out out) {
     uint32_t acc[7][3];
 #pragma unroll
     for (int c = 0; c < 7; c++) acc[c][0] = acc[c][1] = acc[c][2] = 0;
     uint32_t k0 = 0, k1 = 0;  // carry into the next column (64 bits)
-    const int nT = nu4 + nv4;
     for (int T = 0; T < nT; T++) {
+        pre(T);
         const int i0 = T - nv4 + 1 > 0 ? T - nv4 + 1 : 0, i1 = T < nu4 - 1 ? T : nu4 - 1;
         for (int I = i0; I <= i1; I++) {
             const uint4 a = *reinterpret_cast<const uint4 *>(u + 4 * I);
@@ -541,7 +544,7 @@ __device__ __forceinline__ void sm_mul4(const uint32_t *u, int nu4, const uint32
             asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, %4;\n\taddc.u32 %2, %2, 0;"
                 : "+r"(acc[c][0]), "+r"(acc[c][1]), "+r"(acc[c][2])
                 : "r"(k0), "r"(k1));
-            out(4 * T + c, acc[c][0]);
+            out(T, c, acc[c][0]);
             k0 = acc[c][1];
             k1 = acc[c][2];
         }
@@ -551,6 +554,11 @@ __device__ __forceinline__ void sm_mul4(const uint32_t *u, int nu4, const uint32
             for (int w = 0; w < 3; w++) acc[c][w] = c < 3 ? acc[c + 4][w] : 0u;
         }
     }
+}
+
+template <class Out>
+__device__ __forceinline__ void sm_mul4(const uint32_t *u, int nu4, const uint32_t *v, int nv4, Out out) {
+    sm_mul4_pre(u, nu4, v, nv4, nu4 + nv4, [](int) {}, [&](int T, int c, uint32_t x) { out(4 * T + c, x); });
 }
 
 // Batched basecase product on chip: rp = up * vp (un >= vn), NT operands per CTA.
@@ -831,6 +839,169 @@ __global__ void k_mpz_mulops(MatArgs W, MatArgs U, MatArgs V, int op, int64_t co
         return;
     }
     for (int t = rn < cap ? rn : cap; t < cap; t++) wp[(int64_t)t * ws] = 0u;
+    W.sizes[iw] = top == 0 ? 0 : (neg ? -top : top);
+}
+
+// The same operations with the operands staged on chip (as k_mpn_mul_basecase_sm): a CTA
+// of NT threads takes NT entries, each thread forms its product in 4 x 4 limb blocks
+// from shared memory and merges W's limbs, which are loaded a block ahead of the
+// MACs they meet.  Bound by HBM (U, V and W read once, W written once); the kernel
+// above reads two operand limbs from global memory per MAC.  W += U V of 2^20
+// entries of 16 limbs into 33: 347 us with the kernel above, 130 us with this one
+// (3.3 TB/s; the loads of W and the second pass over negative results keep it from more).
+//
+// Limbs of U and V above their sizes are staged as zeros.  The product runs over
+// the warp's longest operands, so that a warp's loads and stores of W stay whole
+// lines; W's limbs above the result are written as zeros in the same pass.
+template <int NT>
+__device__ __forceinline__ void mpz_stage(uint32_t *dst, int SS, int32_t *ssz, const MatArgs &M, int64_t e0, int64_t count,
+                                          bool vec) {
+    if (e0 + threadIdx.x < count) ssz[threadIdx.x] = M.sizes[ent(M, e0 + threadIdx.x)];
+    else ssz[threadIdx.x] = 0;
+    __syncthreads();
+    constexpr int NQ = NT / 4;
+    const int n4 = (M.nlimbs + 3) >> 2;
+    for (int item = threadIdx.x; item < n4 * NQ; item += NT) {
+        const int q = item % NQ, c = item / NQ;
+        const int64_t eq = e0 + 4 * q;
+        uint32_t L[4][4];  // L[k][j]: limb 4c + k of entry eq + j
+        int sz[4];
+        int64_t off[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            sz[j] = iabs_d(ssz[4 * q + j]);
+            off[j] = vec ? eq + j : (eq + j < count ? ent(M, eq + j) : 0);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int i = 4 * c + k;
+            const uint32_t *row = M.limbs + (int64_t)i * M.ld;
+            if (i < M.nlimbs && vec && eq + 3 < count) {
+                const uint4 w = *reinterpret_cast<const uint4 *>(row + eq);
+                L[k][0] = w.x; L[k][1] = w.y; L[k][2] = w.z; L[k][3] = w.w;
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; j++) L[k][j] = (i < M.nlimbs && eq + j < count) ? row[off[j]] : 0u;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (i >= sz[j]) L[k][j] = 0u;
+        }
+        // entries in an order rotated by q (fewer bank conflicts among the stores), by
+        // selects: an index that depends on q would put L in local memory
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const uint32_t a0 = q & 1 ? L[k][1] : L[k][0], a1 = q & 1 ? L[k][2] : L[k][1],
+                           a2 = q & 1 ? L[k][3] : L[k][2], a3 = q & 1 ? L[k][0] : L[k][3];
+            L[k][0] = q & 2 ? a2 : a0;
+            L[k][1] = q & 2 ? a3 : a1;
+            L[k][2] = q & 2 ? a0 : a2;
+            L[k][3] = q & 2 ? a1 : a3;
+        }
+#pragma unroll
+        for (int jj = 0; jj < 4; jj++)
+            *reinterpret_cast<uint4 *>(dst + (4 * q + ((jj + q) & 3)) * SS + 4 * c) =
+                make_uint4(L[0][jj], L[1][jj], L[2][jj], L[3][jj]);
+    }
+}
+template <int NT>
+__global__ void __launch_bounds__(NT, 896 / NT) k_mpz_mulops_sm(MatArgs W, MatArgs U, MatArgs V, int op, int64_t count, int vec_u,
+                                                      int vec_v, uint32_t *err) {
+    extern __shared__ uint4 sm_raw4[];
+    uint32_t *sm = reinterpret_cast<uint32_t *>(sm_raw4);
+    const int Su = sm_stride(U.nlimbs), Sv = sm_stride(V.nlimbs);
+    uint32_t *su_ = sm, *sv_ = sm + NT * Su;
+    int32_t *szu = reinterpret_cast<int32_t *>(sv_ + NT * Sv), *szv = szu + NT;
+    const int64_t e0 = (int64_t)blockIdx.x * NT;
+    mpz_stage<NT>(su_, Su, szu, U, e0, count, vec_u);
+    mpz_stage<NT>(sv_, Sv, szv, V, e0, count, vec_v);
+    __syncthreads();
+    const int64_t e = e0 + threadIdx.x;
+    const bool live = e < count;
+    const int su = szu[threadIdx.x], sv = szv[threadIdx.x];
+    const int un = min(iabs_d(su), U.nlimbs), vn = min(iabs_d(sv), V.nlimbs);
+    const int64_t iw = live ? ent(W, e) : 0;
+    const int cap = W.nlimbs;
+    const int sw = op == 0 || !live ? 0 : W.sizes[iw];
+    const int wn = min(iabs_d(sw), cap);
+    int pneg = (su < 0) ^ (sv < 0);
+    if (op == 2) pneg ^= 1;
+    const bool prod = un && vn;
+    const bool subtract = wn && prod && ((sw < 0) != (pneg != 0));
+    const int nu4 = __reduce_max_sync(0xFFFFFFFFu, prod ? (un + 3) >> 2 : 0);
+    const int nv4 = __reduce_max_sync(0xFFFFFFFFu, prod ? (vn + 3) >> 2 : 0);
+    if (!live) return;
+    uint32_t *wp = W.limbs + iw;
+    const int64_t ws = W.ld;
+    // a zero operand is staged as zeros, so its product is zero over the warp's length too
+    const int nT = max(nu4 + nv4, (cap + 3) >> 2);
+    // W's limbs of this block and of the next two (in flight)
+    uint32_t wl[4], wx[4], wy[4];
+    auto wload = [&](int T, uint32_t(&x)[4]) {
+#pragma unroll
+        for (int c = 0; c < 4; c++) x[c] = 4 * T + c < wn ? wp[(int64_t)(4 * T + c) * ws] : 0u;
+    };
+    wload(0, wx);
+    wload(1, wy);
+    uint32_t carry = 0;
+    int top = 0;
+    bool hi_nz = false, hi_ones = true;
+    sm_mul4_pre(
+        su_ + threadIdx.x * Su, nu4, sv_ + threadIdx.x * Sv, nv4, nT,
+        [&](int T) {
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                wl[c] = wx[c];
+                wx[c] = wy[c];
+            }
+            wload(T + 2, wy);
+        },
+        [&](int T, int c, uint32_t pl) {
+            const int t = 4 * T + c;
+            const uint32_t w = wl[c];
+            uint32_t r;
+            if (!subtract) {
+                const uint64_t s = (uint64_t)w + pl + carry;
+                r = (uint32_t)s;
+                carry = (uint32_t)(s >> 32);
+            } else {
+                const uint64_t d = (uint64_t)w - pl - carry;
+                r = (uint32_t)d;
+                carry = (uint32_t)(d >> 63);
+            }
+            if (t < cap) {
+                wp[(int64_t)t * ws] = r;
+                if (r) top = t + 1;
+            } else {
+                hi_nz |= r != 0u;
+                hi_ones &= r == 0xFFFFFFFFu;
+            }
+        });
+    int neg = op == 0 ? pneg : (wn ? (sw < 0) : pneg);
+    if (subtract && carry) {
+        // |uv| > |w|: the limbs are the result's two's complement over 4 nT limbs.  The
+        // magnitude fits cap limbs iff the dropped limbs are all ones and the kept part is not zero
+        if (4 * nT > cap && !(hi_ones && top != 0)) { atomicOr(err, DEVERR_CAPACITY); return; }
+        neg = pneg;
+        uint32_t c = 1;
+        top = 0;
+        for (int t0 = 0; t0 < cap; t0 += 8) {
+            uint32_t x[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) x[i] = t0 + i < cap ? wp[(int64_t)(t0 + i) * ws] : 0u;
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                if (t0 + i >= cap) break;
+                const uint64_t s = (uint64_t)(~x[i]) + c;
+                c = (uint32_t)(s >> 32);
+                wp[(int64_t)(t0 + i) * ws] = (uint32_t)s;
+                if ((uint32_t)s) top = t0 + i + 1;
+            }
+        }
+    } else if (hi_nz || (!subtract && carry)) {
+        atomicOr(err, DEVERR_CAPACITY);
+        return;
+    }
     W.sizes[iw] = top == 0 ? 0 : (neg ? -top : top);
 }
 
@@ -1742,8 +1913,26 @@ gbmm_status launch_max_size(const gbmm_mat &a, int32_t *d_out, cudaStream_t s) {
 gbmm_status launch_mpz_mulops(const gbmm_mat &w, const gbmm_mat &u, const gbmm_mat &v, int op, cudaStream_t s) {
     const int64_t n = nentries(w);
     if (n == 0) return GBMM_OK;
+    // staged on chip wherever 32 or more entries' operands fit in shared memory
+    const size_t words = (size_t)sm_stride(u.nlimbs) + sm_stride(v.nlimbs) + 2;
+    const int nt = u.nlimbs > 0 && v.nlimbs > 0 ? sm_threads(words) : 0;
     LaunchScope ls_("k_mpz_mulops", s);
-    k_mpz_mulops<<<grid1(n, 128), 128, 0, s>>>(margs(w), margs(u), margs(v), op, n, device_error_word());
+    if (nt) {
+        const size_t smem = nt * words * 4;
+        const int vu = u.rs == u.cols && vec16(u.limbs, u.ld), vv = v.rs == v.cols && vec16(v.limbs, v.ld);
+#define MULOPS_SM(NT_)                                                                                                \
+    do {                                                                                                              \
+        GBMM_CUDA_TRY(cudaFuncSetAttribute(k_mpz_mulops_sm<NT_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+        k_mpz_mulops_sm<NT_><<<grid1(n, NT_), NT_, smem, s>>>(margs(w), margs(u), margs(v), op, n, vu, vv,            \
+                                                              device_error_word());                                   \
+    } while (0)
+        if (nt == 128) MULOPS_SM(128);
+        else if (nt == 64) MULOPS_SM(64);
+        else MULOPS_SM(32);
+#undef MULOPS_SM
+    } else {
+        k_mpz_mulops<<<grid1(n, 128), 128, 0, s>>>(margs(w), margs(u), margs(v), op, n, device_error_word());
+    }
     GBMM_CUDA_TRY(cudaGetLastError());
     return GBMM_OK;
 }
