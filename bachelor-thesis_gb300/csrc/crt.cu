@@ -65,6 +65,8 @@ constexpr int CTA_THREADS = 192;   // warp 0 TMA, warp 1 MMA, warps 2..5 epilogu
 constexpr int CTA_THREADS8 = 320;  // warp 0 TMA, warp 1 MMA, warps 2..9 epilogue (two per lane quadrant)
 constexpr int RES_EPI_WARPS = 16;   // residue GEMM: four epilogue warps per lane quadrant
 constexpr int RES_THREADS = 32 * (2 + RES_EPI_WARPS);
+constexpr int REC_EPI_WARPS = 16;   // reconstruction: four epilogue warps per lane quadrant
+constexpr int REC_THREADS = 32 * (2 + REC_EPI_WARPS);
 constexpr int RTAB = 256;          // reconstruction table rows are padded to a multiple of this
 }  // namespace
 
@@ -896,9 +898,9 @@ __global__ void __launch_bounds__(CTA_THREADS8, 1)
 // ======================================================================================
 // 4. reconstruction GEMM (persistent over tiles of 128 entries, or 256 entries
 //    for a CTA pair; N tiles of 256 table rows; TMEM double-buffered across N
-//    tiles; 8 epilogue warps per CTA, two per entry splitting the columns.  Base-128 table
-//    digits keep one FP32 accumulation over all 2P rows exact:
-//    2P * 128 * 64 < 2^24.)
+//    tiles; 16 epilogue warps per CTA, four per entry splitting the columns.  Base-128 table
+//    digits keep one FP32 accumulation over all 2P rows exact, 2P * 128 * 64 < 2^24;
+//    base-256 digits do wherever the table's column sums say so.)
 //    Y arrives blocked, [E/64][2Pp][64], so each 64-entry x 64-row A box is one
 //    contiguous 8 KB run.
 //    PAIR: a cluster of two CTAs on two SMs runs one M = 256, N = 256
@@ -915,10 +917,12 @@ struct ReconArgs {
     int32_t ccols;   // columns of C: entries with col >= ccols are padding and not stored
     int32_t nk;      // K steps over 2Pp
     int32_t NT;      // N tiles of 256 table rows
-    int32_t Dout;    // output base-128 digit positions
+    int32_t nlast;   // columns of the last one (a multiple of 32)
+    int32_t Dout;    // output digit positions (base 2^DB)
     int32_t kpad;    // 2Pp: rows of one 64-entry block of Y
     int64_t nmt;     // entry tiles (128 entries, or 256 for a pair)
-    const uint32_t *vtab;  // per 32-digit chunk n: sum_u Mod_(32n+u) 128^u as 7 two's-complement words + sign word
+    const uint32_t *vtab;  // Mod's value per 32-digit chunk, 8 words: DB = 7: sum_u Mod_(32n+u) 128^u as 7
+                           // two's-complement words + sign word; DB = 8: signed base-2^32 digits 8n .. 8n + 7
     uint32_t *climbs;
     int32_t *csizes;
     int64_t cld, crs;
@@ -929,23 +933,34 @@ struct ReconJob {
     CUtensorMap tmY, tmT;
     ReconArgs a;
 };
-// Hand-off between the two epilogue warps of a TMEM lane quadrant (per entry slots).
+// Hand-offs between the four epilogue warps ("parts") of a TMEM lane quadrant, per entry.
+// One token per quadrant goes round the parts, part 0 -> 1 -> 2 -> 3 -> 0 of the next N
+// tile (also on to the next entry tile): the carry, the negation ripple, the highest nonzero
+// limb and the dropped-limb flags so far.  A part writes the next part's slot only while
+// it holds the token, so a slot or a barrier is never a round ahead of its reader.  Part 0's
+// fixed-point results of entry tile i sit in slot and barrier i & 1: those of tile i + 2 are
+// written after the token of tile i's last part came back, and every part reads its q before
+// it passes the token on.
 struct ReconXfer {
-    uint64_t to1[4], to0[4], qready[4];  // mbarriers per quadrant: half 0 -> 1, half 1 -> 0, q ready
-    long long carry1[128], carry0[128];  // carry handed to half 1 / to half 0
-    uint32_t ripple1[128], ripple0[128]; // negation ripple handed on
-    int32_t q[128], sgn[128], amb[128];  // fixed-point results of an entry's tile 0
-    int32_t top0[128];                   // half 0's highest nonzero limb + 1
-    uint32_t drop0[128];                 // half 0's dropped-limb flags (bit 0 nonzero, bit 1 all ones)
+    uint64_t tokbar[4][4], qready[2][4];  // [part][quadrant], [tile parity][quadrant]
+    int4 tok[4][128];                     // (carry, ripple, top, drop) for part p
+    int2 q[2][128];                       // (q, sign and doubt bits)
 };
+
+// a * b + c with 32-bit factors (one wide multiply-add)
+__device__ __forceinline__ long long mad_wide(int a, int b, long long c) {
+    long long d;
+    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+    return d;
+}
 
 // Y's map is 3-D, [Ep/64 blocks][2P rows][64 entries]: the rows 2P .. 2Pp-1 of a
 // block's last K step lie outside it and read as zeros.  GRP: a grouped launch;
 // Mod's chunk values are then read from global memory (each product has its own),
-// and the epilogue's hand-offs take the form that holds for any sequence of N-tile
-// counts (see the half-0 wait at an entry tile's first N tile).
-template <int STAGES, bool PAIR, bool GRP>
-__global__ void __launch_bounds__(CTA_THREADS8, 1)
+// (the epilogue's token order holds for any sequence of N-tile counts).
+// DB: bits of a table digit (see recon_digit_bits): 32 columns are DB limbs.
+template <int STAGES, bool PAIR, bool GRP, int DB>
+__global__ void __launch_bounds__(REC_THREADS, 1)
     k_crt_recon(const __grid_constant__ CUtensorMap tmY, const __grid_constant__ CUtensorMap tmT, ReconArgs a0,
                 Group<ReconJob> grp, uint32_t *err) {
     extern __shared__ uint8_t smem_raw[];
@@ -983,9 +998,8 @@ __global__ void __launch_bounds__(CTA_THREADS8, 1)
     };
     if (threadIdx.x == 0)
         for (int qd = 0; qd < 4; qd++) {
-            tc::mbar_init(&xf->to1[qd], 1);
-            tc::mbar_init(&xf->to0[qd], 1);
-            tc::mbar_init(&xf->qready[qd], 1);
+            for (int pt = 0; pt < 4; pt++) tc::mbar_init(&xf->tokbar[pt][qd], 1);
+            for (int i = 0; i < 2; i++) tc::mbar_init(&xf->qready[i][qd], 1);
         }
     if (PAIR) {
         if (threadIdx.x == 0) {
@@ -995,7 +1009,7 @@ __global__ void __launch_bounds__(CTA_THREADS8, 1)
             }
             for (int b = 0; b < 2; b++) {
                 tc::mbar_init(&bars->tfull[b], 1);
-                tc::mbar_init(&bars->tempty[b], 16);  // the even CTA's: 8 epilogue warps of each CTA
+                tc::mbar_init(&bars->tempty[b], 2 * REC_EPI_WARPS);  // the even CTA's: every epilogue warp of both CTAs
             }
             bars->abort_flag = 0;
             tc::fence_mbar_init();
@@ -1009,13 +1023,13 @@ __global__ void __launch_bounds__(CTA_THREADS8, 1)
         tc::cluster_sync_all();  // both CTAs' barriers exist before any cross-CTA signal
         tc::fence_after_sync();
     } else {
-        cta_setup(bars, STAGES, 512, 1, 8);
+        cta_setup(bars, STAGES, 512, 1, REC_EPI_WARPS);
     }
     tc::grid_dep_wait();  // the planes this launch reads are complete
     const uint32_t tmem = bars->tmem_base;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (tc::elect_one()) {
             if (!GRP) {
                 tc::prefetch_tmap(&tmY);
                 tc::prefetch_tmap(&tmT);
@@ -1041,7 +1055,9 @@ __global__ void __launch_bounds__(CTA_THREADS8, 1)
                             if (rank == 0) tc::mbar_arrive_expect_tx(&bars->full[st], 2 * STAGE);
                             tc::tma_load_3d_pair(sa, mY, full0, 0, s * BK, blk0);
                             tc::tma_load_3d_pair(sa + BOX, mY, full0, 0, s * BK, blk0 + 1);
-                            tc::tma_load_2d_pair(sa + A_BYTES, mT, full0, s * BK, j * RBN + (int)rank * TROWS);
+                            // the even CTA's rows are the tile's first half, also of a narrow last tile
+                            tc::tma_load_2d_pair(sa + A_BYTES, mT, full0, s * BK,
+                                                 j * RBN + (int)rank * (j + 1 < a.NT ? TROWS : a.nlast / 2));
                         } else {
                             tc::mbar_arrive_expect_tx(&bars->full[st], STAGE);
                             tc::tma_load_3d(sa, mY, &bars->full[st], 0, s * BK, blk0);
@@ -1053,8 +1069,7 @@ __global__ void __launch_bounds__(CTA_THREADS8, 1)
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
-            const uint32_t idesc = tc::idesc_bf16_f32(NP * BM, RBN, 1, 0);
+        if (rank == 0 && tc::elect_one()) {
             int it = 0, lt = 0;
             bool ok = true;
             for (int64_t T = tbeg + t0; T < total && ok; T += tstep) {
@@ -1063,6 +1078,8 @@ __global__ void __launch_bounds__(CTA_THREADS8, 1)
                 tile_job(T, a, mY, mT);
                 (void)mY, (void)mT;
                 for (int j = 0; j < a.NT && ok; j++, lt++) {
+                    // the last N tile's MMAs have only the columns it needs
+                    const uint32_t idesc = tc::idesc_bf16_f32(NP * BM, j + 1 < a.NT ? RBN : a.nlast, 1, 0);
                     const int b = lt & 1;
                     if (lt >= 2 && !tc::mbar_wait(&bars->tempty[b], ((lt >> 1) & 1) ^ 1)) {
                         set_abort(bars, err);
@@ -1095,63 +1112,45 @@ __global__ void __launch_bounds__(CTA_THREADS8, 1)
             }
         }
     } else {
-        // 8 epilogue warps.  quad = warp % 4 owns TMEM lanes (entries) quad * 32 .. + 31 and
-        // hf = (warp - 2) / 4 owns accumulator columns hf * 128 .. + 127 of every N tile.  An
-        // entry's digits run through its carry chain in the order (tile 0, half 0), (tile 0,
-        // half 1), (tile 1, half 0), ...  Each half reads its 128 columns at once (so the
-        // TMEM buffer goes back to the MMA immediately), turns them into up to 28 limbs
-        // starting from carry 0, then takes its predecessor's carry and negation ripple from
-        // shared memory, adds them, stores, and hands its own on.  Hand-offs are mbarriers
-        // with bounded waits; the exchange slots are per entry.
-        const int quad = warp & 3, hf = (warp - 2) >> 2, idx = quad * 32 + lane;
-        const uint32_t lb = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(hf * 128);
+        // 16 epilogue warps.  quad = warp % 4 owns TMEM lanes (entries) quad * 32 .. + 31 and
+        // part = (warp - 2) / 4 owns accumulator columns part * 64 .. + 63 of every N tile.  An
+        // entry's digits run through its carry chain part by part, N tile by N tile.  Each part
+        // turns its two 32-column chunks into limbs starting from carry 0, then takes the
+        // token (the carry and negation ripple so far), adds them, stores, and passes it on.
+        // Waits are bounded.
+        // What bounds it: dependent integer chains, not the issue slots (31 % used by two warps per
+        // lane quadrant) and not HBM, hence four warps per quadrant:
+        // 1024 x 1024 entries by 259 moduli 709 -> 518 us, 300 x 300 by 259 85 -> 65 us.  (Base-256 table
+        // digits and one wide multiply-add per digit took the same launches from 921 to 738 us and
+        // the 512 x 512 one by 516 moduli from 439 to 376 us.)
+        const int quad = warp & 3, part = (warp - 2) >> 2, idx = quad * 32 + lane;
+        const uint32_t lb = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(part * 64);
         const uint32_t tempty0 = PAIR ? tc::mapa(tc::smem_u32(&bars->tempty[0]), 0) : 0;
-        int lt = 0, ph1 = 0, ph0 = 0, phq = 0;  // tiles seen; hand-off phases consumed
+        int lt = 0, ntok = 0, et = 0;  // N tiles, tokens taken, entry tiles seen
         bool first = true, ok = true;
-        for (int64_t T = tbeg + t0; T < total && ok; T += tstep) {
+        for (int64_t T = tbeg + t0; T < total && ok; T += tstep, et++) {
             ReconArgs a;
             const CUtensorMap *mY, *mT;
             const int64_t t = tile_job(T, a, mY, mT);
             (void)mY, (void)mT;
-            // UNI: half 1 hands on at the end of an entry tile only after its finalize,
-            // and half 0 takes that hand-off before it writes the next tile's slots (the
-            // only order that is safe when N-tile counts vary from tile to tile); else
-            // the one-N-tile case alone waits for the finalize
-            const bool UNI = GRP || a.NT == 1;
             const int64_t e = t * (NP * BM) + rank * BM + quad * 32 + lane;
             const int64_t er = e / a.ncols, ec = e - er * a.ncols;
             const bool live = e < a.E && ec < a.ccols;
             const int64_t coff = live ? er * a.crs + ec : 0;
-            // C = sum_u (acc_u - q Mod_u) 128^u; the limbs written are |C| (negated on the
+            // C = sum_u (acc_u - q Mod_u) 2^(DB u); the limbs written are |C| (negated on the
             // fly when the fixed-point sum says C < 0)
-            int32_t q = 0, sgn = 1, amb = 0;
-            int top = 0;
-            bool drop_nz = false, drop_ones = true;
-            long long carry_final = 0;
-            uint32_t nc_final = 1;
-            const bool last_t = T + tstep >= total;
+            int q = 0, sgn = 1, amb = 0, top = 0, c = 0;
+            uint32_t nin = 0, drop = 2;  // dropped limbs: bit 0 any nonzero, bit 1 all ones
             for (int j = 0; j < a.NT; j++, lt++) {
                 const int b = lt & 1;
                 if (!tc::mbar_wait(&bars->tfull[b], (lt >> 1) & 1)) { set_abort(bars, err); ok = false; break; }
                 tc::fence_after_sync();
-                // columns 0..63 of this half now, 64..127 after two chunks (then the buffer is released)
-                uint32_t g[64];
-                tc::tmem_ld32(lb + (uint32_t)(256 * b), *reinterpret_cast<uint32_t(*)[32]>(&g[0]));
-                tc::tmem_ld32(lb + (uint32_t)(256 * b + 32), *reinterpret_cast<uint32_t(*)[32]>(&g[32]));
-                tc::tmem_ld_wait();
-                bool took0 = false;  // half 0: the hand-off from half 1 is already taken
+                uint32_t g[32];
+                tc::tmem_ld32(lb + (uint32_t)(256 * b), g);
+                tc::tmem_ld_wait(g);
                 if (j == 0) {
-                    if (hf == 0) {
-                        // the q, top0 and drop0 slots are free only once half 1 is done with
-                        // the previous entry tile (its finalize included).  UNI: take that
-                        // hand-off before writing them, so that the slots and qready never run
-                        // a tile ahead.  Otherwise (the same N tiles, more than one, for every
-                        // entry tile) the hand-off at j = 1 already orders them.
-                        if (!first && UNI) {
-                            if (!tc::mbar_wait(&xf->to0[quad], ph0 & 1)) { set_abort(bars, err); ok = false; break; }
-                            ph0++;
-                            took0 = true;
-                        }
+                    const int qb = et & 1;
+                    if (part == 0) {
                         // fixed-point sum S = sum y_i 2^FIXB / p_i from the first SUSED columns
                         // (base 128): S = (q + C / Mod) 2^FIXB + err, |err| <= 128 P < 2^17, and
                         // |C / Mod| < 2^-18, so q = round(S / 2^FIXB) and the sign of
@@ -1166,33 +1165,29 @@ __global__ void __launch_bounds__(CTA_THREADS8, 1)
                         q = (int32_t)qq;
                         sgn = frac < -tol ? -1 : 1;
                         amb = frac <= tol && frac >= -tol;
-                        xf->q[idx] = q;
-                        xf->sgn[idx] = sgn;
-                        xf->amb[idx] = amb;
+                        xf->q[qb][idx] = make_int2(q, (sgn < 0 ? 1 : 0) | (amb ? 2 : 0));
                         __syncwarp();
-                        if (lane == 0) tc::mbar_arrive(&xf->qready[quad]);
+                        if (lane == 0) tc::mbar_arrive(&xf->qready[qb][quad]);
                     } else {
-                        if (!tc::mbar_wait(&xf->qready[quad], phq & 1)) { set_abort(bars, err); ok = false; break; }
-                        phq++;
-                        q = xf->q[idx];
-                        sgn = xf->sgn[idx];
-                        amb = xf->amb[idx];
+                        if (!tc::mbar_wait(&xf->qready[qb][quad], (et >> 1) & 1)) { set_abort(bars, err); ok = false; break; }
+                        const int2 v = xf->q[qb][idx];
+                        q = v.x;
+                        sgn = v.y & 1 ? -1 : 1;
+                        amb = v.y >> 1;
                     }
                 }
-                // this half's limbs from carry 0: chunks k = 0..3 are digit columns
-                // pos = 256 j + 128 hf + 32 k - SROWS (32 digits = 7 limbs, on limb boundaries)
-                uint32_t L[28];
-                long long c = 0;
-                int nl = 0;
-                const int pos0 = 256 * j + 128 * hf - SROWS;
-                const int k0 = pos0 < 0 ? 1 : 0;  // the fixed-point columns precede digit 0
-                const int li0 = (pos0 + 32 * k0) / 32 * 7;
+                // this part's limbs from carry 0: chunks ch, ch + 1 of 32 digits (DB limbs each, on
+                // limb boundaries; the fixed-point columns are chunk -1)
+                uint32_t L[2 * DB];
+                c = 0;  // |carry| < 2^26
+                const int ch = 8 * j + 2 * part - SROWS / 32;
+                const int nq = -q;
+                bool have[2];
 #pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    if (k == 2) {
-                        tc::tmem_ld32(lb + (uint32_t)(256 * b + 64), *reinterpret_cast<uint32_t(*)[32]>(&g[0]));
-                        tc::tmem_ld32(lb + (uint32_t)(256 * b + 96), *reinterpret_cast<uint32_t(*)[32]>(&g[32]));
-                        tc::tmem_ld_wait();
+                for (int k = 0; k < 2; k++) {
+                    if (k == 1) {
+                        tc::tmem_ld32(lb + (uint32_t)(256 * b + 32), g);
+                        tc::tmem_ld_wait(g);
                         tc::fence_before_sync();
                         __syncwarp();
                         if (lane == 0) {
@@ -1200,114 +1195,87 @@ __global__ void __launch_bounds__(CTA_THREADS8, 1)
                             else tc::mbar_arrive(&bars->tempty[b]);
                         }
                     }
-                    const int pos = pos0 + 32 * k;
-                    if (k < k0 || !live || pos >= a.Dout) continue;
-                    const uint32_t *W = (GRP ? a.vtab : svtab) + (pos >> 5) * 8;
-                    long long A[7];
-                    A[0] = c;
+                    have[k] = live && ch + k >= 0 && (ch + k) * 32 < a.Dout;
+                    if (!have[k]) continue;
+                    const uint32_t *W = (GRP ? a.vtab : svtab) + (ch + k) * 8;
+                    if constexpr (DB == 8) {
+                        // four columns per limb: a0 + 2^8 a1 + 2^16 a2 + 2^24 a3 - q W_l + carry, |.| < 2^49
 #pragma unroll
-                    for (int l = 1; l < 7; l++) A[l] = 0;
+                        for (int l = 0; l < 8; l++) {
+                            long long t = mad_wide(nq, (int)W[l], (long long)tc::acc_int(g[4 * l]));
+                            t = mad_wide(tc::acc_int(g[4 * l + 1]), 1 << 8, t);
+                            t = mad_wide(tc::acc_int(g[4 * l + 2]), 1 << 16, t);
+                            t = mad_wide(tc::acc_int(g[4 * l + 3]), 1 << 24, t) + c;
+                            L[8 * k + l] = (uint32_t)t;
+                            c = (int)(t >> 32);
+                        }
+                    } else {
+                        long long A[7];
+                        A[0] = c;
 #pragma unroll
-                    for (int u = 0; u < 32; u++)
-                        A[(7 * u) >> 5] += (long long)tc::acc_int(g[32 * (k & 1) + u]) * (1LL << ((7 * u) & 31));
+                        for (int l = 1; l < 7; l++) A[l] = 0;
 #pragma unroll
-                    for (int l = 0; l < 7; l++) A[l] -= (long long)q * (long long)W[l];
+                        for (int u = 0; u < 32; u++)
+                            A[(7 * u) >> 5] += (long long)tc::acc_int(g[u]) * (1LL << ((7 * u) & 31));
 #pragma unroll
-                    for (int l = 0; l < 7; l++) {
-                        if (l < 6) A[l + 1] += A[l] >> 32;
-                        L[7 * k + l] = (uint32_t)A[l];
+                        for (int l = 0; l < 7; l++) A[l] += (long long)nq * (long long)W[l];
+#pragma unroll
+                        for (int l = 0; l < 7; l++) {
+                            if (l < 6) A[l + 1] += A[l] >> 32;
+                            L[7 * k + l] = (uint32_t)A[l];
+                        }
+                        // the chunk's Mod value is sum W_l 2^(32 l) - s 2^224 (s = sign word)
+                        c = (int)(A[6] >> 32) + (W[7] ? q : 0);
                     }
-                    // the chunk's Mod value is sum W_l 2^(32 l) - s 2^224 (s = sign word)
-                    c = (A[6] >> 32) + (W[7] ? (long long)q : 0LL);
-                    nl = 7 * (k + 1);
                 }
-                // predecessor's carry and negation ripple: half 1 takes half 0's of the same
-                // tile; half 0 takes half 1's of the previous tile (none at an entry's tile 0)
-                long long cin = 0;
-                uint32_t nin = 1;
-                if (hf == 1) {
-                    if (!tc::mbar_wait(&xf->to1[quad], ph1 & 1)) { set_abort(bars, err); ok = false; break; }
-                    ph1++;
-                    cin = xf->carry1[idx];
-                    nin = xf->ripple1[idx];
-                } else if (!first) {
-                    if (!took0) {
-                        if (!tc::mbar_wait(&xf->to0[quad], ph0 & 1)) { set_abort(bars, err); ok = false; break; }
-                        ph0++;
-                    }
-                    if (j > 0) {
-                        cin = xf->carry0[idx];
-                        nin = xf->ripple0[idx];
+                // the token: nothing to take at an entry's first columns but the turn
+                int cin = 0;
+                nin = sgn < 0;  // a non-negative value passes 0 on
+                if (part > 0 || !first) {
+                    if (!tc::mbar_wait(&xf->tokbar[part][quad], ntok & 1)) { set_abort(bars, err); ok = false; break; }
+                    ntok++;
+                    if (part > 0 || j > 0) {
+                        const int4 v = xf->tok[part][idx];
+                        cin = v.x;
+                        nin = (uint32_t)v.y;
+                        top = v.z;
+                        drop = (uint32_t)v.w;
                     }
                 }
                 first = false;
-                // add the carry in, negate when C < 0, store
+                // add the carry in, negate when C < 0 (~limb + 1, the +1 rippling up), store
+                const uint32_t mask = sgn < 0 ? 0xFFFFFFFFu : 0u;
+                const int li0 = ch * DB, room = a.cnlimbs - li0;  // limbs of this part that C has planes for
+                uint32_t *cp = a.climbs + (int64_t)li0 * a.cld + coff;
 #pragma unroll
-                for (int l = 0; l < 28; l++) {
-                    if (l < k0 * 7 || l >= nl || cin == 0) continue;
-                    const long long s = (long long)L[l] + cin;
-                    L[l] = (uint32_t)s;
-                    cin = s >> 32;
+                for (int l = 0; l < 2 * DB; l++, cp += a.cld) {
+                    if (!have[l / DB]) continue;
+                    const uint32_t sum = L[l] + (uint32_t)cin;
+                    cin = (cin >> 31) + (sum < L[l] ? 1 : 0);
+                    const uint32_t limb = (sum ^ mask) + nin;
+                    nin = limb == 0u ? nin : 0u;
+                    if (l < room) {
+                        *cp = limb;
+                        if (limb) top = li0 + l + 1;
+                    } else {
+                        drop = (drop | (limb != 0u)) & (limb == 0xFFFFFFFFu ? 3u : 1u);
+                    }
                 }
                 c += cin;
-#pragma unroll
-                for (int l = 0; l < 28; l++) {
-                    if (l < k0 * 7 || l >= nl) continue;
-                    uint32_t limb = L[l];
-                    if (sgn < 0) {
-                        const uint32_t nv = ~limb + nin;
-                        nin &= (uint32_t)(limb == 0u);
-                        limb = nv;
-                    }
-                    const int li = li0 + l - k0 * 7;
-                    if (li < a.cnlimbs) {
-                        a.climbs[(int64_t)li * a.cld + coff] = limb;
-                        if (limb) top = li + 1;
-                    } else {
-                        drop_nz |= limb != 0u;
-                        drop_ones &= limb == 0xFFFFFFFFu;
-                    }
-                }
-                // hand on: half 0 -> half 1 of this tile; half 1 -> half 0 of the next tile
-                // (also after an entry's last tile, except the CTA's very last one, so that
-                // half 0 never runs two hand-offs ahead)
-                if (hf == 0) {
-                    xf->carry1[idx] = c;
-                    xf->ripple1[idx] = nin;
-                    if (j == a.NT - 1) {
-                        xf->top0[idx] = top;
-                        xf->drop0[idx] = (drop_nz ? 1u : 0u) | (drop_ones ? 2u : 0u);
-                    }
-                    __syncwarp();
-                    if (lane == 0) tc::mbar_arrive(&xf->to1[quad]);
-                } else {
-                    if (j == a.NT - 1) {
-                        carry_final = c;
-                        nc_final = nin;
-                    } else {
-                        xf->carry0[idx] = c;
-                        xf->ripple0[idx] = nin;
-                    }
-                    // after an entry's last N tile the hand-off waits for the finalize under
-                    // UNI (see half 0's early take at j = 0)
-                    if (j < a.NT - 1 || (!UNI && !last_t)) {
-                        __syncwarp();
-                        if (lane == 0) tc::mbar_arrive(&xf->to0[quad]);
-                    }
-                }
+                // pass the token on (after the CTA's very last column nobody takes it)
+                const int next = (part + 1) & 3;
+                xf->tok[next][idx] = make_int4(c, (int)nin, top, (int)drop);
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(&xf->tokbar[next][quad]);
             }
             if (!ok) break;
-            if (hf == 1 && live) {
-                // finalize: half 0's top limb and dropped-limb flags arrived with its last hand-off
-                top = max(top, xf->top0[idx]);
-                const uint32_t d0 = xf->drop0[idx];
-                drop_nz |= (d0 & 1u) != 0;
-                drop_ones &= (d0 & 2u) != 0;
-                const int nl = (a.Dout + 31) / 32 * 7;  // limbs produced
+            if (part == 3 && live) {
+                const bool drop_nz = drop & 1u, drop_ones = drop & 2u;
+                const int nl = (a.Dout + 31) / 32 * DB;  // limbs produced
                 const int written = nl < a.cnlimbs ? nl : a.cnlimbs;
                 int neg = sgn < 0;
                 // bits above the produced limbs of the written value: C's own, or -C's
-                long long carry = neg ? -carry_final - 1 + (long long)nc_final : carry_final;
+                const long long carry = neg ? -(long long)c - 1 + (long long)nin : (long long)c;
                 if (carry < 0) {
                     // only reachable on the ambiguous path: two's complement -> magnitude
                     if (!amb || carry != -1 || (nl > a.cnlimbs && !(drop_ones && top != 0)))
@@ -1335,11 +1303,6 @@ __global__ void __launch_bounds__(CTA_THREADS8, 1)
                 }
                 for (int li = written; li < a.cnlimbs; li++) a.climbs[(int64_t)li * a.cld + coff] = 0u;
                 a.csizes[coff] = top == 0 ? 0 : (neg ? -top : top);
-            }
-            if (hf == 1 && !last_t && UNI) {
-                // the finalize is done with half 0's slots: hand on to half 0's next entry tile
-                __syncwarp();
-                if (lane == 0) tc::mbar_arrive(&xf->to0[quad]);
             }
         }
     }
@@ -1675,6 +1638,17 @@ static void balanced128(const big &x, int ndig, int *out) {
         }
     }
 }
+// balanced base-256 digits (each in [-128, 127]): digit t takes byte t plus the carry of
+// the digit below
+static void balanced256(const big &x, int ndig, int *out) {
+    int c = 0;
+    for (int t = 0; t < ndig; t++) {
+        const int b = (size_t)(t / 4) < x.size() ? (int)((x[t / 4] >> (8 * (t & 3))) & 255u) : 0;
+        const int v = b + c;
+        c = v >= 128;
+        out[t] = v - (c << 8);
+    }
+}
 static std::vector<int> balanced128(const big &x, int ndig) {
     std::vector<int> out(ndig, 0);
     balanced128(x, ndig, out.data());
@@ -1726,6 +1700,7 @@ struct crt_tables {
     crt_cache *cache = nullptr;  // the cache that holds these tables (and the shared residue table)
     int P = 0, Pp = 0;   // moduli, padded 2P/2 (2Pp multiple of 64)
     int Dout = 0, NT = 0;
+    int db = 7;          // bits of a digit of the reconstruction table
     __nv_bfloat16 *d_recon = nullptr;  // [NT * RTAB][2Pp]
     uint32_t *d_vtab = nullptr;        // [ceil(Dout / 32)][8]: Mod's digits per 32-digit chunk
     std::map<int, __nv_bfloat16 *> residue;  // 2 * dxp + weighted -> [2P rows][dxp]
@@ -1767,20 +1742,34 @@ static int moduli_for_bits(int64_t bits) {
 // chunk values and the constant (p, 1/p) list.
 struct crt_tables_host {
     int P = 0, Pp = 0, Dout = 0, NT = 0;
+    int db = 7;                   // bits of a digit of the reconstruction table
+    double bound = 0;             // largest magnitude an accumulator of its digit columns can reach
     std::vector<ModConst> mods;
     std::vector<uint16_t> recon;  // [NT * RTAB][2Pp] bf16 bits
     std::vector<uint32_t> vtab;   // [ceil(Dout / 32)][8]
     std::vector<float> cmod;      // 4 * CMOD_PAIRS
 };
 
-static void build_tables_host(int P, crt_tables_host &o) {
+// Digits of the reconstruction table: base 128 is exact for every P up to 1023 (2P digits
+// of Y of magnitude 128 against digits of at most 64: 2P * 2^13 < 2^24).  Base 256 digits
+// reach 128, but a column's true bound is 128 times the sum of its digits' magnitudes,
+// half as large on average: below 2^24 up to about 950 moduli (checked on each table as it
+// is built).  They take an eighth fewer columns, and four of them are a limb.
+static constexpr int RECON256_MAX_P = 940;
+
+static void build_tables_host(int P, crt_tables_host &o, int db = 7) {
     const auto &pr = primes_desc();
     o.P = P;
+    o.db = db;
+    auto digits = [db](const big &x, int ndig, int *out) {
+        if (db == 8) balanced256(x, ndig, out);
+        else balanced128(x, ndig, out);
+    };
     o.Pp = (2 * P + 63) / 64 * 32;
     big Mod{1};
     for (int i = 0; i < P; i++) big_mul_small(Mod, pr[i]);
     int modbits = (int)(32 * Mod.size());
-    o.Dout = (modbits + 6) / 7 + 2;  // base-128 output digits
+    o.Dout = (modbits + db - 1) / db + 2;  // output digits
     o.NT = (SROWS + o.Dout + RTAB - 1) / RTAB;  // in units of RTAB rows
     const int rows = o.NT * RTAB, cols = 2 * o.Pp;
     o.recon.assign((size_t)rows * cols, bf16_bits(0.f));
@@ -1793,7 +1782,9 @@ static void build_tables_host(int P, crt_tables_host &o) {
     // row, 2 MB adjacent columns at a time (writing one column at a time would
     // touch a new cache line with every 2-byte store).
     constexpr int MB = 32;
-    auto block = [&](int i0, int i1, std::vector<int8_t> &dig, std::vector<int> &tmp) {
+    std::mutex sum_mu;
+    std::vector<int64_t> colsum(o.Dout, 0);  // sum of the digits' magnitudes per column
+    auto block = [&](int i0, int i1, std::vector<int8_t> &dig, std::vector<int> &tmp, std::vector<int64_t> &cs) {
         const int nb = i1 - i0;
         for (int q = 0; q < nb; q++) {
             const int i = i0 + q;
@@ -1812,9 +1803,9 @@ static void build_tables_host(int P, crt_tables_host &o) {
             mc.w = w;
             o.mods[i] = mc;
             // column 2i multiplies the high digit (x256), column 2i+1 the low digit
-            balanced128(Mi256, o.Dout, tmp.data());
+            digits(Mi256, o.Dout, tmp.data());
             for (int r = 0; r < o.Dout; r++) dig[(size_t)r * (2 * MB) + 2 * q] = (int8_t)tmp[r];
-            balanced128(Mi, o.Dout, tmp.data());
+            digits(Mi, o.Dout, tmp.data());
             for (int r = 0; r < o.Dout; r++) dig[(size_t)r * (2 * MB) + 2 * q + 1] = (int8_t)tmp[r];
             // fixed-point weights: round(2^(FIXB+8) / p) for the high digit, round(2^FIXB / p) for the low digit
             const unsigned __int128 one = 1;
@@ -1834,7 +1825,10 @@ static void build_tables_host(int P, crt_tables_host &o) {
         for (int r = 0; r < o.Dout; r++) {
             uint16_t *row = &tab[(size_t)(SROWS + r) * cols + 2 * i0];
             const int8_t *src = &dig[(size_t)r * (2 * MB)];
-            for (int c = 0; c < 2 * nb; c++) row[c] = bf16_small(src[c]);
+            for (int c = 0; c < 2 * nb; c++) {
+                row[c] = bf16_small(src[c]);
+                cs[r] += std::abs((int)src[c]);
+            }
         }
     };
     const int nblocks = (P + MB - 1) / MB;
@@ -1842,7 +1836,10 @@ static void build_tables_host(int P, crt_tables_host &o) {
     auto range = [&](int th) {
         std::vector<int8_t> dig((size_t)o.Dout * 2 * MB);
         std::vector<int> tmp(o.Dout);
-        for (int bk = th; bk < nblocks; bk += nthr) block(bk * MB, std::min(P, (bk + 1) * MB), dig, tmp);
+        std::vector<int64_t> cs(o.Dout, 0);
+        for (int bk = th; bk < nblocks; bk += nthr) block(bk * MB, std::min(P, (bk + 1) * MB), dig, tmp, cs);
+        std::lock_guard<std::mutex> lk(sum_mu);
+        for (int r = 0; r < o.Dout; r++) colsum[r] += cs[r];
     };
     if (nthr == 1) {
         range(0);
@@ -1852,12 +1849,31 @@ static void build_tables_host(int P, crt_tables_host &o) {
         range(0);
         for (auto &th : pool) th.join();
     }
+    o.bound = 128.0 * (double)*std::max_element(colsum.begin(), colsum.end());
+    const int nch = (o.Dout + 31) / 32;
+    o.vtab.assign((size_t)nch * 8, 0u);
+    // the constant (p, 1/p) list: the same for every table, written with each
+    o.cmod.resize(4 * CMOD_PAIRS);
+    for (int q = 0; q < CMOD_PAIRS; q++) {
+        o.cmod[4 * q] = (float)pr[2 * q];
+        o.cmod[4 * q + 1] = (float)pr[2 * q + 1];
+        o.cmod[4 * q + 2] = 1.0f / (float)pr[2 * q];
+        o.cmod[4 * q + 3] = 1.0f / (float)pr[2 * q + 1];
+    }
+    if (db == 8) {
+        // Mod in signed base-2^32 digits (each in [-2^31, 2^31)); Dout leaves a limb above Mod
+        uint64_t c = 0;
+        for (int l = 0; l < 8 * nch; l++) {
+            const uint64_t v = ((size_t)l < Mod.size() ? (uint64_t)Mod[l] : 0ull) + c;
+            o.vtab[l] = (uint32_t)v;
+            c = (v + 0x80000000ull) >> 32;
+        }
+        return;
+    }
     // Mod's balanced base-128 digits, summed per 32-digit chunk n into the 224-bit
     // value V_n = sum_u Mod_(32n+u) 128^u, kept as 8 words of a 256-bit two's
     // complement number (|V_n| < 2^223, so word 7 is the sign extension)
     std::vector<int> md = balanced128(Mod, o.Dout);
-    const int nch = (o.Dout + 31) / 32;
-    o.vtab.assign((size_t)nch * 8, 0u);
     for (int n = 0; n < nch; n++) {
         uint32_t *w = &o.vtab[(size_t)n * 8];
         for (int u = 0; u < 32; u++) {
@@ -1878,19 +1894,16 @@ static void build_tables_host(int P, crt_tables_host &o) {
             }
         }
     }
-    // the constant (p, 1/p) list: the same for every table, written with each
-    o.cmod.resize(4 * CMOD_PAIRS);
-    for (int q = 0; q < CMOD_PAIRS; q++) {
-        o.cmod[4 * q] = (float)pr[2 * q];
-        o.cmod[4 * q + 1] = (float)pr[2 * q + 1];
-        o.cmod[4 * q + 2] = 1.0f / (float)pr[2 * q];
-        o.cmod[4 * q + 3] = 1.0f / (float)pr[2 * q + 1];
-    }
 }
 
 static gbmm_status build_tables(crt_tables *t, int P) {
     crt_tables_host o;
-    build_tables_host(P, o);
+    if (P <= RECON256_MAX_P) build_tables_host(P, o, 8);
+    if (P > RECON256_MAX_P || o.bound >= 16777216.0) {
+        o = crt_tables_host();
+        build_tables_host(P, o, 7);
+    }
+    t->db = o.db;
     t->P = o.P;
     t->Pp = o.Pp;
     t->Dout = o.Dout;
@@ -2258,6 +2271,7 @@ static gbmm_status make_map_yblocks(CUtensorMap *m, const void *ptr, uint64_t ro
 struct ReconPlan {
     CUtensorMap tmY, tmT;
     ReconArgs ra;
+    int db = 7;
     bool pair = false;
     size_t smem = 0;
 };
@@ -2273,6 +2287,8 @@ static gbmm_status plan_recon(crt_tables *t, __nv_bfloat16 *Y, int m, int n, int
     ReconArgs &ra = rp.ra;
     memset(&ra, 0, sizeof ra);
     ra.E = E; ra.ncols = npad; ra.ccols = n; ra.nk = 2 * t->Pp / BK; ra.NT = (SROWS + t->Dout + 255) / 256;
+    ra.nlast = (SROWS + t->Dout - 256 * (ra.NT - 1) + 31) / 32 * 32;
+    rp.db = t->db;
     ra.Dout = t->Dout; ra.vtab = t->d_vtab; ra.climbs = c.limbs; ra.csizes = c.sizes; ra.cld = c.ld; ra.crs = c.rs;
     ra.cnlimbs = c.nlimbs; ra.kpad = 2 * t->Pp;
     ra.mt0 = 0;
@@ -2415,8 +2431,9 @@ gbmm_status crt_matmul(gbmm_handle h, const gbmm_mat &c, const gbmm_mat &a, cons
         const int64_t nmt = ra.nmt;
         const Group<ReconJob> none{nullptr, nullptr, 0};
         uint32_t *err = device_error_word();
-        if (rp.pair) GBMM_TRY(set_smem((const void *)k_crt_recon<REC_STAGES_PAIR, true, false>, rp.smem));
-        else GBMM_TRY(set_smem((const void *)k_crt_recon<REC_STAGES, false, false>, rp.smem));
+        auto kpair = rp.db == 8 ? k_crt_recon<REC_STAGES_PAIR, true, false, 8> : k_crt_recon<REC_STAGES_PAIR, true, false, 7>;
+        auto kone = rp.db == 8 ? k_crt_recon<REC_STAGES, false, false, 8> : k_crt_recon<REC_STAGES, false, false, 7>;
+        GBMM_TRY(set_smem(rp.pair ? (const void *)kpair : (const void *)kone, rp.smem));
         const int NP = rp.pair ? 2 : 1;
         // one launch, or (stage hooks) entry ranges each followed by an event
         const int parts = hk ? (int)std::max<int64_t>(1, std::min<int64_t>({(int64_t)hk->parts, (int64_t)CRT_MAX_PARTS, nmt})) : 1;
@@ -2425,11 +2442,11 @@ gbmm_status crt_matmul(gbmm_handle h, const gbmm_mat &c, const gbmm_mat &a, cons
             ra.nmt = nmt * (pi + 1) / parts;
             LaunchScope ls_("k_crt_recon", s);
             if (rp.pair) {
-                GBMM_TRY(launch_pairs(k_crt_recon<REC_STAGES_PAIR, true, false>, CTA_THREADS8, ra.nmt - ra.mt0, rp.smem, s,
+                GBMM_TRY(launch_pairs(kpair, REC_THREADS, ra.nmt - ra.mt0, rp.smem, s,
                                       rp.tmY, rp.tmT, ra, none, err));
             } else {
                 dim3 grid((unsigned)std::min<int64_t>(ra.nmt - ra.mt0, num_sms()));
-                GBMM_TRY(launch_one(k_crt_recon<REC_STAGES, false, false>, grid, CTA_THREADS8, rp.smem, s, rp.tmY,
+                GBMM_TRY(launch_one(kone, grid, REC_THREADS, rp.smem, s, rp.tmY,
                                     rp.tmT, ra, none, err));
             }
             GBMM_CUDA_TRY(cudaGetLastError());
@@ -2463,15 +2480,16 @@ struct crt_group {
     // dig by digit form (unsigned, balanced); res by accumulation groups: unsigned
     // digits (one group), balanced with one group (256-column table tiles), balanced
     // with several (table tiles of 128 or 64 columns, a deeper ring of smaller
-    // stages); rec[1]: products with a post step
-    std::vector<Rec> dig[2], res[3], prod, rec[2];
+    // stages); rec[2 f + d]: reconstructions of products with (f = 1) and without a post
+    // step, by table digits (d = 1: base 256)
+    std::vector<Rec> dig[2], res[3], prod, rec[4];
     std::vector<std::function<gbmm_status(cudaStream_t)>> post;
     struct Sect {
         size_t jobs_off = 0, tile0_off = 0;
         int n = 0;
         int64_t total = 0;
     };
-    Sect sdig[2], sres[3], sprod, srec[2];
+    Sect sdig[2], sres[3], sprod, srec[4];
     size_t smem_prod = 0, smem_rec = 0;
     std::vector<char> blob;
 };
@@ -2567,7 +2585,7 @@ gbmm_status crt_group_add(gbmm_handle h, crt_group *g, const gbmm_mat &c, const 
     ReconJob rj;
     memset(&rj, 0, sizeof rj);
     rj.tmY = rp.tmY; rj.tmT = rp.tmT; rj.a = rp.ra;
-    g->rec[halves ? 1 : 0].push_back(make_rec(rj, rp.ra.nmt, (double)rp.ra.NT * rp.ra.nk));
+    g->rec[(halves ? 2 : 0) + (rp.db == 8)].push_back(make_rec(rj, rp.ra.nmt, (double)rp.ra.NT * rp.ra.nk));
     g->smem_rec = std::max(g->smem_rec, rp.smem);
     return GBMM_OK;
 }
@@ -2596,7 +2614,7 @@ const std::vector<char> &crt_group_blob(crt_group *g) {
     for (int f = 0; f < 2; f++) pack_section(g->blob, g->dig[f], g->sdig[f]);
     for (int f = 0; f < 3; f++) pack_section(g->blob, g->res[f], g->sres[f]);
     pack_section(g->blob, g->prod, g->sprod);
-    for (int f = 0; f < 2; f++) pack_section(g->blob, g->rec[f], g->srec[f]);
+    for (int f = 0; f < 4; f++) pack_section(g->blob, g->rec[f], g->srec[f]);
     return g->blob;
 }
 
@@ -2668,14 +2686,15 @@ gbmm_status crt_group_launch(crt_group *g, const char *d_blob, cudaStream_t s, c
     // the products with post steps first: their shifted adds then run on s2 while
     // the other reconstructions do
     for (int f = 1; f >= 0; f--) {
-        const crt_group::Sect &sec = g->srec[f];
-        if (sec.n) {
+        for (int d = 1; d >= 0; d--) {
+            const crt_group::Sect &sec = g->srec[2 * f + d];
+            if (!sec.n) continue;
             ReconArgs none;
             memset(&none, 0, sizeof none);
-            auto kern = k_crt_recon<REC_STAGES_PAIR, true, true>;
+            auto kern = d ? k_crt_recon<REC_STAGES_PAIR, true, true, 8> : k_crt_recon<REC_STAGES_PAIR, true, true, 7>;
             GBMM_TRY(set_smem((const void *)kern, g->smem_rec));
             LaunchScope ls_("k_crt_recon", s);
-            GBMM_TRY(launch_pairs(kern, CTA_THREADS8, sec.total, g->smem_rec, s, zmap, zmap, none,
+            GBMM_TRY(launch_pairs(kern, REC_THREADS, sec.total, g->smem_rec, s, zmap, zmap, none,
                                   group_at<ReconJob>(d_blob, sec), err));
         }
         if (f == 1 && !g->post.empty()) {

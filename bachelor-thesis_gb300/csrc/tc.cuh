@@ -322,9 +322,12 @@ __device__ __forceinline__ void tmem_relinquish_pair() {
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
-// remote arrive on an mbarrier of another CTA of the cluster
+// Arrive on an mbarrier of another CTA of the cluster.  What it hands over is tensor
+// memory, whose reads tcgen05.wait::ld and tcgen05.fence have ordered; a release at cluster
+// scope would also wait for the thread's global stores (the epilogues of pairs spent a
+// fifth of their time in that wait).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster) : "memory");
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster) : "memory");
 }
 
 // Accumulator word -> exact integer (every accumulated value is an integer of
