@@ -400,7 +400,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1)
     };
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (tc::elect_one()) {
             if (!GRP) {
                 tc::prefetch_tmap(&tmD);
                 tc::prefetch_tmap(&tmT);
@@ -444,7 +444,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1)
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && (rank == 0 || MC)) {
+        if ((rank == 0 || MC) && tc::elect_one()) {
             int it = 0, lt = 0;
             bool ok = true;
             for (int64_t T = t0; T < total && ok; T += tstep, lt++) {
@@ -655,6 +655,27 @@ struct ProductJob {
 constexpr int PBX = 64;  // output columns per product tile
 constexpr int YPAD = 16;  // Y's entry rows are padded to a multiple of this (whole 32-byte runs)
 
+// Staging of one epilogue warp's 32 rows x 32 columns of one plane of Y, and its store:
+// four lanes write a row's 64 bytes, so a store instruction covers 8 rows in whole runs
+// (from the rows' own lanes it touched 32 rows with 16 bytes each: every 16 bytes a request
+// of its own to L2, 17 million for 512 x 512 entries by 259 moduli, which bounded
+// products with a short inner dimension).  Rows of Y are padded to whole groups of
+// 16 entries, so a 16-byte chunk of 8 lies inside one 64-entry block.
+constexpr int PROD_STG_BYTES = 32 * 32 * 2;
+__device__ __forceinline__ void store_plane(const ProductArgs &a, const uint4 *stg, int plane, int y0, int xh) {
+    const int lane = threadIdx.x & 31, c = lane & 3;
+    const int x = xh + 8 * c;
+    uint8_t *yp = reinterpret_cast<uint8_t *>(a.Y) + (int64_t)plane * 128;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int row = 8 * i + (lane >> 2), y = y0 + row;
+        const uint4 v = stg[row * 4 + (c ^ ((row >> 1) & 3))];
+        const int64_t e = (int64_t)y * a.npad + x;
+        if (y < a.m && x < a.npad)
+            *reinterpret_cast<uint4 *>(yp + 2 * ((e >> 6) * a.yblk + (e & 63))) = v;
+    }
+}
+
 // PAIR: a cluster of two CTAs shares one M = 256 tcgen05.mma.cta_group::2 per K
 // slice (issued by the even CTA): each CTA stages its own 128 rows of A1 and A0,
 // the even CTA U1's 64 rows and the odd CTA U0's, so per SM a K step moves 40 KB
@@ -670,6 +691,7 @@ __global__ void __launch_bounds__(CTA_THREADS8, 1)
     // together the 128-row B operand [U1; U0]
     constexpr uint32_t A_BYTES = BM * 128, B_BYTES = PBX * 128, STAGE = 2 * A_BYTES + (3 - NP) * B_BYTES;
     Barriers *bars = reinterpret_cast<Barriers *>(base + STAGES * STAGE);
+    uint8_t *stage_out = reinterpret_cast<uint8_t *>(bars) + SMEM_BARS;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = PAIR ? tc::cluster_rank() : 0;
     const int64_t t0 = PAIR ? (blockIdx.x >> 1) : blockIdx.x, tstep = PAIR ? (gridDim.x >> 1) : gridDim.x;
@@ -718,7 +740,7 @@ __global__ void __launch_bounds__(CTA_THREADS8, 1)
     };
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (tc::elect_one()) {
             if (!GRP) {
                 tc::prefetch_tmap(&tmA);
                 tc::prefetch_tmap(&tmB);
@@ -756,7 +778,7 @@ __global__ void __launch_bounds__(CTA_THREADS8, 1)
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0 && tc::elect_one()) {
             const uint32_t idesc = tc::idesc_bf16_f32(NP * BM, 2 * PBX, 0, 0);
             int it = 0, lt = 0;
             bool ok = true;
@@ -806,6 +828,10 @@ __global__ void __launch_bounds__(CTA_THREADS8, 1)
         const int quad = warp & 3, half = (warp - 2) >> 2;
         const uint32_t lb = tmem + ((uint32_t)(quad * 32) << 16);
         const uint32_t tempty0 = PAIR ? tc::mapa(tc::smem_u32(&bars->tempty[0]), 0) : 0;
+        // this warp's staging: 32 rows of 32 entries of one plane, 16-byte chunks at positions
+        // that keep both the row writes and the reads of whole rows conflict-free
+        uint4 *stg = reinterpret_cast<uint4 *>(stage_out + (warp - 2) * PROD_STG_BYTES);
+        const int swz = (lane >> 1) & 3;
         int lt = 0;
         for (int64_t T = t0; T < total; T += tstep, lt++) {
             ProductArgs a;
@@ -815,7 +841,7 @@ __global__ void __launch_bounds__(CTA_THREADS8, 1)
             const int64_t per_mod = (int64_t)a.nyt * a.nxt;
             const int b = lt & 1;
             const int mi = (int)(t / per_mod), r = (int)(t % per_mod);
-            const int y = (r / a.nxt) * (NP * BM) + (int)rank * BM + quad * 32 + lane;
+            const int y0 = (r / a.nxt) * (NP * BM) + (int)rank * BM + quad * 32;  // the warp's first row
             const int xh = (r % a.nxt) * PBX + half * 32;  // this warp's 32 output columns
             if (!tc::mbar_wait(&bars->tfull[b], (lt >> 1) & 1)) { set_abort(bars, err); break; }
             tc::fence_after_sync();
@@ -836,49 +862,36 @@ __global__ void __launch_bounds__(CTA_THREADS8, 1)
             // lanes share mi); the same values as the moduli table's
             const float4 cmp = c_modpair[mi >> 1];
             const float pf = (mi & 1) ? cmp.y : cmp.x, ipf = (mi & 1) ? cmp.w : cmp.z;
-            const int64_t erow = (int64_t)y * a.npad + xh;  // entry index of this warp's first column
-            __nv_bfloat16 *yplane = a.Y + (int64_t)(2 * mi) * 64;  // hi plane; lo plane 64 elements on
+            uint32_t plo[16];
 #pragma unroll
-            for (int c = 0; c < 32; c += 16) {
-                const uint32_t *d11 = D11 + c, *d10 = D10 + c, *d01 = D01 + c, *d00 = D00 + c;
-                uint32_t phi[8], plo[8];
+            for (int c = 0; c < 32; c += 8) {
+                uint32_t phi[4];
 #pragma unroll
-                for (int j = 0; j < 16; j += 2) {
+                for (int j = 0; j < 8; j += 2) {
                     float h2[2], l2[2];
 #pragma unroll
                     for (int u = 0; u < 2; u++) {
                         // |a1 u0 + a0 u1| <= 2^24; each step below stays under 257 * 32772 < 2^24
-                        const float r2 = red(__uint_as_float(d11[j + u]), pf, ipf);
-                        const float r1 = red(__uint_as_float(d10[j + u]) + __uint_as_float(d01[j + u]), pf, ipf);
-                        const float r0 = red(__uint_as_float(d00[j + u]), pf, ipf);
+                        const float r2 = red(__uint_as_float(D11[c + j + u]), pf, ipf);
+                        const float r1 = red(__uint_as_float(D10[c + j + u]) + __uint_as_float(D01[c + j + u]), pf, ipf);
+                        const float r0 = red(__uint_as_float(D00[c + j + u]), pf, ipf);
                         const float tt = red(__fmaf_rn(256.f, r2, r1), pf, ipf);
                         bal_split(red(__fmaf_rn(256.f, tt, r0), pf, ipf), h2[u], l2[u]);
                     }
                     phi[j / 2] = bf16x2_bits(h2[0], h2[1]);
-                    plo[j / 2] = bf16x2_bits(l2[0], l2[1]);
+                    plo[(c + j) / 2] = bf16x2_bits(l2[0], l2[1]);
                 }
-                if (y >= a.m) continue;
-                // rows of Y are padded to whole groups of 16 entries, so every group but a
-                // row's last partial one is two aligned 32-byte runs inside one 64-entry block
-                const int64_t ec = erow + c;
-                if ((ec & 15) == 0 && xh + c < a.n) {
-                    __nv_bfloat16 *dst = yplane + (ec >> 6) * a.yblk + (ec & 63);
-                    uint4 *dsth = reinterpret_cast<uint4 *>(dst), *dstl = reinterpret_cast<uint4 *>(dst + 64);
-                    dsth[0] = make_uint4(phi[0], phi[1], phi[2], phi[3]);
-                    dsth[1] = make_uint4(phi[4], phi[5], phi[6], phi[7]);
-                    dstl[0] = make_uint4(plo[0], plo[1], plo[2], plo[3]);
-                    dstl[1] = make_uint4(plo[4], plo[5], plo[6], plo[7]);
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 16; j++) {
-                        if (xh + c + j >= a.n) break;
-                        const int64_t e = ec + j;
-                        uint16_t *dst = reinterpret_cast<uint16_t *>(yplane + (e >> 6) * a.yblk + (e & 63));
-                        dst[0] = (uint16_t)(phi[j / 2] >> (16 * (j & 1)));
-                        dst[64] = (uint16_t)(plo[j / 2] >> (16 * (j & 1)));
-                    }
-                }
+                stg[lane * 4 + ((c >> 3) ^ swz)] = make_uint4(phi[0], phi[1], phi[2], phi[3]);
             }
+            __syncwarp();
+            store_plane(a, stg, 2 * mi, y0, xh);
+            __syncwarp();
+#pragma unroll
+            for (int c = 0; c < 4; c++)
+                stg[lane * 4 + (c ^ swz)] = make_uint4(plo[4 * c], plo[4 * c + 1], plo[4 * c + 2], plo[4 * c + 3]);
+            __syncwarp();
+            store_plane(a, stg, 2 * mi + 1, y0, xh);
+            __syncwarp();
         }
     }
     tc::grid_dep_launch();
@@ -2227,8 +2240,8 @@ static gbmm_status plan_product(crt_tables *t, __nv_bfloat16 *RA, __nv_bfloat16 
     pa.nyt = (m + NP * BM - 1) / (NP * BM);
     pa.nxt = (n + PBX - 1) / PBX;
     pa.ntiles = (int64_t)P * pa.nyt * pa.nxt;
-    pp.smem = pp.pair ? smem_bytes(PROD_STAGES_PAIR, 2 * BM * 128 + PBX * 128)
-                      : smem_bytes(PROD_STAGES, 2 * BM * 128 + 2 * PBX * 128);
+    pp.smem = (pp.pair ? smem_bytes(PROD_STAGES_PAIR, 2 * BM * 128 + PBX * 128)
+                       : smem_bytes(PROD_STAGES, 2 * BM * 128 + 2 * PBX * 128)) + 8 * PROD_STG_BYTES;
     return GBMM_OK;
 }
 
