@@ -175,8 +175,57 @@ __global__ void __launch_bounds__(256) k_mpn_addsub_n_serial(uint32_t *rp, const
     }
     cy[b] = c;
 }
+// The same for four neighbouring operands per thread, 16-byte loads and stores and four
+// limbs of them in flight: with enough operands to fill the GPU, what counts is the
+// bytes in flight per thread (2^20 operands of 32 limbs: 91 -> 65 us).  Needs 16-byte
+// aligned planes and strides; the last nb % 4 operands take a thread each.
+template <bool SUB>
+__global__ void __launch_bounds__(256) k_mpn_addsub_n_vec(uint4 *rp, const uint4 *up, const uint4 *vp, int n, int64_t ld4,
+                                                          int64_t nb, uint4 *cy) {
+    const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nb4 = nb >> 2;
+    if (b >= nb4) {
+        const int64_t q = 4 * nb4 + (b - nb4);
+        if (q >= nb) return;
+        uint32_t c = 0;
+        for (int i = 0; i < n; i++) {
+            const uint32_t x = reinterpret_cast<const uint32_t *>(up + i * ld4)[q],
+                           y = reinterpret_cast<const uint32_t *>(vp + i * ld4)[q];
+            const uint64_t t = SUB ? (uint64_t)x - y - c : (uint64_t)x + y + c;
+            reinterpret_cast<uint32_t *>(rp + i * ld4)[q] = (uint32_t)t;
+            c = SUB ? (uint32_t)(t >> 63) : (uint32_t)(t >> 32);
+        }
+        reinterpret_cast<uint32_t *>(cy)[q] = c;
+        return;
+    }
+    uint32_t c[4] = {0, 0, 0, 0};
+    for (int i0 = 0; i0 < n; i0 += 4) {
+        uint4 x[4], y[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            if (i0 + i < n) {
+                x[i] = up[(int64_t)(i0 + i) * ld4 + b];
+                y[i] = vp[(int64_t)(i0 + i) * ld4 + b];
+            }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            if (i0 + i >= n) break;
+            const uint32_t xs[4] = {x[i].x, x[i].y, x[i].z, x[i].w}, ys[4] = {y[i].x, y[i].y, y[i].z, y[i].w};
+            uint32_t r[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const uint64_t t = SUB ? (uint64_t)xs[k] - ys[k] - c[k] : (uint64_t)xs[k] + ys[k] + c[k];
+                r[k] = (uint32_t)t;
+                c[k] = SUB ? (uint32_t)(t >> 63) : (uint32_t)(t >> 32);
+            }
+            rp[(int64_t)(i0 + i) * ld4 + b] = make_uint4(r[0], r[1], r[2], r[3]);
+        }
+    }
+    cy[b] = make_uint4(c[0], c[1], c[2], c[3]);
+}
 // batches with at least this many operands take the one-thread-per-operand kernel
 constexpr int64_t ADDSUB_SERIAL_MIN_OPS = 16384;
+// ... and with four per thread when that still leaves eight warps per SM
+constexpr int64_t ADDSUB_VEC_MIN_OPS = 152 * 8 * 32 * 4;
 
 // ---- mul_1 family: one thread per operand, serial over limbs (coalesced) -----------
 template <int OP>  // 0 mul_1, 1 addmul_1, 2 submul_1
@@ -446,13 +495,19 @@ __host__ __device__ __forceinline__ int sm_stride(int n) {
     return (n4 & 7) == 4 ? n4 : n4 + 4;
 }
 
+// the same for strings padded to whole blocks of B limbs
+template <int B>
+__host__ __device__ __forceinline__ int sm_stride_b(int n) {
+    return sm_stride((n + B - 1) / B * B);
+}
+
 // Stages limbs [0, n) of operands b0 .. b0 + NT - 1 (limb i of operand b at
 // g[i * ld + b]) into dst[t * SS + i], zero-filling limbs n .. roundup4(n) and
 // operands past nb.  vec: g and ld allow 16-byte loads (g 16-byte aligned, ld % 4 == 0).
-template <int NT>
+template <int NT, int B = 4>
 __device__ __forceinline__ void sm_stage(uint32_t *dst, int SS, const uint32_t *g, int n, int64_t ld, int64_t b0,
                                          int64_t nb, bool vec) {
-    const int n4 = (n + 3) >> 2;
+    const int n4 = (n + B - 1) / B * (B / 4);  // chunks of four limbs, padded to whole blocks of B
     constexpr int NQ = NT / 4;  // groups of four operands
     for (int item = threadIdx.x; item < n4 * NQ; item += NT) {
         const int q = item % NQ, c = item / NQ;  // consecutive threads: neighbouring operand groups
@@ -513,34 +568,40 @@ __device__ __forceinline__ void sm_stage_map(uint32_t *dst, int SS, int nchunks,
     }
 }
 
-// r = u * v for strings of nu4 and nv4 chunks of four limbs (16-byte aligned,
-// zero-padded), by block product scanning: column block T gathers the 4 x 4
-// blocks (I, T - I); their 7 columns are summed in 96-bit accumulators, the
-// block's four columns absorb the carry from below and go out in ascending
-// order (out(T, c, limb): limb 4 T + c), the upper three seed the next block.
-// pre(T) runs before block T's MACs (loads it issues are in flight during them);
-// blocks nu4 + nv4 .. nT - 1 only pass the carry on.
-template <class Pre, class Out>
-__device__ __forceinline__ void sm_mul4_pre(const uint32_t *u, int nu4, const uint32_t *v, int nv4, int nT, Pre pre,
-                                            Out out) {
-    uint32_t acc[7][3];
+// r = u * v for strings of nu and nv blocks of B limbs (16-byte aligned, zero-padded), by
+// block product scanning: column block T gathers the B x B blocks (I, T - I); their
+// 2 B - 1 columns are summed in 96-bit accumulators, the block's B columns absorb the
+// carry from below and go out in ascending order (out(T, c, limb): limb B T + c), the
+// upper ones seed the next block.  pre(T) runs before block T's MACs (loads it issues are in
+// flight during them); blocks nu + nv .. nT - 1 only pass the carry on.
+// B = 8 halves the shared-memory loads and loop steps per MAC against B = 4 (sm_block
+// says which one a product takes).
+template <int B, class Pre, class Out>
+__device__ __forceinline__ void sm_mul_pre(const uint32_t *u, int nu, const uint32_t *v, int nv, int nT, Pre pre, Out out) {
+    constexpr int NC = 2 * B - 1;
+    uint32_t acc[NC][3];
 #pragma unroll
-    for (int c = 0; c < 7; c++) acc[c][0] = acc[c][1] = acc[c][2] = 0;
+    for (int c = 0; c < NC; c++) acc[c][0] = acc[c][1] = acc[c][2] = 0;
     uint32_t k0 = 0, k1 = 0;  // carry into the next column (64 bits)
     for (int T = 0; T < nT; T++) {
         pre(T);
-        const int i0 = T - nv4 + 1 > 0 ? T - nv4 + 1 : 0, i1 = T < nu4 - 1 ? T : nu4 - 1;
+        const int i0 = T - nv + 1 > 0 ? T - nv + 1 : 0, i1 = T < nu - 1 ? T : nu - 1;
         for (int I = i0; I <= i1; I++) {
-            const uint4 a = *reinterpret_cast<const uint4 *>(u + 4 * I);
-            const uint4 b = *reinterpret_cast<const uint4 *>(v + 4 * (T - I));
-            const uint32_t x[4] = {a.x, a.y, a.z, a.w}, y[4] = {b.x, b.y, b.z, b.w};
+            uint32_t x[B], y[B];
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int w = 0; w < B; w += 4) {
+                const uint4 a = *reinterpret_cast<const uint4 *>(u + B * I + w);
+                const uint4 b = *reinterpret_cast<const uint4 *>(v + B * (T - I) + w);
+                x[w] = a.x; x[w + 1] = a.y; x[w + 2] = a.z; x[w + 3] = a.w;
+                y[w] = b.x; y[w + 1] = b.y; y[w + 2] = b.z; y[w + 3] = b.w;
+            }
 #pragma unroll
-                for (int j = 0; j < 4; j++) MAC96(acc[i + j][0], acc[i + j][1], acc[i + j][2], x[i], y[j]);
+            for (int i = 0; i < B; i++)
+#pragma unroll
+                for (int j = 0; j < B; j++) MAC96(acc[i + j][0], acc[i + j][1], acc[i + j][2], x[i], y[j]);
         }
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
+        for (int c = 0; c < B; c++) {
             asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, %4;\n\taddc.u32 %2, %2, 0;"
                 : "+r"(acc[c][0]), "+r"(acc[c][1]), "+r"(acc[c][2])
                 : "r"(k0), "r"(k1));
@@ -549,38 +610,49 @@ __device__ __forceinline__ void sm_mul4_pre(const uint32_t *u, int nu4, const ui
             k1 = acc[c][2];
         }
 #pragma unroll
-        for (int c = 0; c < 7; c++) {
+        for (int c = 0; c < NC; c++) {
 #pragma unroll
-            for (int w = 0; w < 3; w++) acc[c][w] = c < 3 ? acc[c + 4][w] : 0u;
+            for (int w = 0; w < 3; w++) acc[c][w] = c < B - 1 ? acc[c + B][w] : 0u;
         }
     }
 }
 
 template <class Out>
 __device__ __forceinline__ void sm_mul4(const uint32_t *u, int nu4, const uint32_t *v, int nv4, Out out) {
-    sm_mul4_pre(u, nu4, v, nv4, nu4 + nv4, [](int) {}, [&](int T, int c, uint32_t x) { out(4 * T + c, x); });
+    sm_mul_pre<4>(u, nu4, v, nv4, nu4 + nv4, [](int) {}, [&](int T, int c, uint32_t x) { out(4 * T + c, x); });
+}
+
+// Block edge of an un x vn limb product: 8 where padding both operands to whole blocks
+// costs at most a seventh more MACs than blocks of 4.  Measured, 2^18 products of 32 x 32
+// limbs: 72 us with 4, 68 us with 8; 2^15 of 128 x 100: 144 and 124 us.
+__host__ __device__ __forceinline__ int sm_block(int un, int vn) {
+    const int p4 = ((un + 3) / 4) * ((vn + 3) / 4), p8 = 4 * ((un + 7) / 8) * ((vn + 7) / 8);
+    return un >= 8 && vn >= 8 && 7 * p8 <= 8 * p4 ? 8 : 4;
 }
 
 // Batched basecase product on chip: rp = up * vp (un >= vn), NT operands per CTA.
-template <int NT>
-__global__ void __launch_bounds__(NT) k_mpn_mul_basecase_sm(uint32_t *rp, const uint32_t *up, int un,
+template <int NT, int B>
+__global__ void __launch_bounds__(NT, B == 8 ? 640 / NT : 1) k_mpn_mul_basecase_sm(uint32_t *rp, const uint32_t *up, int un,
                                                             const uint32_t *vp, int vn, int64_t ld, int64_t nb,
                                                             int vec_u, int vec_v) {
     extern __shared__ uint4 sm_raw4[];
     uint32_t *sm = reinterpret_cast<uint32_t *>(sm_raw4);
-    const int Su = sm_stride(un), Sv = sm_stride(vn);
+    const int Su = sm_stride_b<B>(un), Sv = sm_stride_b<B>(vn);
     uint32_t *su = sm, *sv = sm + NT * Su;
     const int64_t b0 = (int64_t)blockIdx.x * NT;
-    sm_stage<NT>(su, Su, up, un, ld, b0, nb, vec_u);
-    sm_stage<NT>(sv, Sv, vp, vn, ld, b0, nb, vec_v);
+    sm_stage<NT, B>(su, Su, up, un, ld, b0, nb, vec_u);
+    sm_stage<NT, B>(sv, Sv, vp, vn, ld, b0, nb, vec_v);
     __syncthreads();
     const int64_t b = b0 + threadIdx.x;
     if (b >= nb) return;
     uint32_t *r = rp + b;
     const int rn = un + vn;
-    sm_mul4(su + threadIdx.x * Su, (un + 3) >> 2, sv + threadIdx.x * Sv, (vn + 3) >> 2, [&](int t, uint32_t x) {
-        if (t < rn) r[(int64_t)t * ld] = x;
-    });
+    const int nu = (un + B - 1) / B, nv = (vn + B - 1) / B;
+    sm_mul_pre<B>(
+        su + threadIdx.x * Su, nu, sv + threadIdx.x * Sv, nv, nu + nv, [](int) {},
+        [&](int T, int c, uint32_t x) {
+            if (B * T + c < rn) r[(int64_t)(B * T + c) * ld] = x;
+        });
 }
 
 // Shared-memory words per thread of the on-chip Toom-2.2 for an x bn limbs: the
@@ -701,6 +773,7 @@ __global__ void __launch_bounds__(NT) k_mpn_toom22_sm(uint32_t *pp, const uint32
 // ======================================================================================
 __device__ __forceinline__ int64_t ent(const MatArgs &m, int64_t e) {
     // elementwise ops treat the view as rows x cols; e is the row-major index
+    if (m.rs == m.cols) return e;  // dense: no 64-bit division
     int64_t r = e / m.cols, c = e - r * m.cols;
     return r * m.rs + c;
 }
@@ -731,28 +804,235 @@ __device__ void addsub_entry(const MatArgs &W, int64_t iw, const MatArgs &U, int
     // last plane (found after the pass) leaves W's limbs undefined
     if (xn > W.nlimbs || yn > W.nlimbs) { atomicOr(err, DEVERR_CAPACITY); W.sizes[iw] = 0; return; }
     // every lane runs over all of W's planes, writing the zero tail in the same pass:
-    // the warp's stores to a plane go out together as whole sectors
+    // the warp's stores to a plane go out together as whole sectors.  Eight limbs at a
+    // time: their loads go out ahead of the carry chain and of the stores (W may be U or V)
     uint32_t c = 0;  // carry or borrow
     int len = 0;
-    for (int i = 0; i < W.nlimbs; i++) {
-        const uint32_t x = i < xn ? xp[(int64_t)i * xs] : 0u, y = i < yn ? yp[(int64_t)i * ys] : 0u;
-        uint32_t r;
-        if (add) {
-            const uint64_t t = (uint64_t)x + y + c;
-            r = (uint32_t)t;
-            c = (uint32_t)(t >> 32);
-        } else {
-            const uint64_t t = (uint64_t)x - y - c;
-            r = (uint32_t)t;
-            c = (uint32_t)(t >> 63);
+    for (int i0 = 0; i0 < W.nlimbs; i0 += 8) {
+        uint32_t x[8], y[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            x[k] = i0 + k < xn ? xp[(int64_t)(i0 + k) * xs] : 0u;
+            y[k] = i0 + k < yn ? yp[(int64_t)(i0 + k) * ys] : 0u;
         }
-        wp[(int64_t)i * W.ld] = r;
-        if (r) len = i + 1;
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            if (i0 + k >= W.nlimbs) break;
+            const uint64_t t = add ? (uint64_t)x[k] + y[k] + c : (uint64_t)x[k] - y[k] - c;
+            c = add ? (uint32_t)(t >> 32) : (uint32_t)(t >> 63);
+            wp[(int64_t)(i0 + k) * W.ld] = (uint32_t)t;
+            if ((uint32_t)t) len = i0 + k + 1;
+        }
     }
     // a carry out of W's last plane: W is too small (its size is set to 0 so a
     // later reader of W stays inside its planes)
     if (add && c) { atomicOr(err, DEVERR_CAPACITY); W.sizes[iw] = 0; return; }
     W.sizes[iw] = len == 0 ? 0 : (neg ? -len : len);
+}
+
+// W = U + sgn V 2^(32 sh), entry by entry, with an entry's limbs split among threads: a block
+// takes 32 entries (threadIdx.x), thread row g the limbs [g SEG, g SEG + SEG).  Every
+// thread forms its limbs of the signed sum from carry 0 (two's complement, in
+// registers, eight limbs' loads of both operands in flight at a time), the carries
+// between segments are resolved through shared memory, then the sign, and each limb is
+// written once.  All operand limbs are read before the first barrier and all of W's written
+// after it, so W may be U or V, shifted or not.  Bound by latency on few entries, where one
+// thread per entry has a carry chain through every load: 128 x 128 entries of 130 limbs
+// 27 -> 12.5 us, the halves of a 181 x 133 product of 595 limbs 194 -> 91 us.
+// strict: an operand longer than W is refused outright (mpz semantics), else only a
+// result that does not fit.
+template <int MS>
+struct Lin2Shared {
+    uint32_t first[MS][32];
+    signed char carry[MS][32];
+    unsigned char rest[MS][32], zero[MS][32];
+    int top[32];
+    signed char fin[32];
+};
+template <int SEG, int MS>
+__global__ void __launch_bounds__(32 * MS) k_mpz_lin2(MatArgs W, MatArgs U, MatArgs V, int sh, int sub, int strict,
+                                                      int64_t count, uint32_t *err) {
+    __shared__ Lin2Shared<MS> s;
+    const int x = threadIdx.x, g = threadIdx.y, ng = blockDim.y, l0 = g * SEG;
+    const int64_t e = (int64_t)blockIdx.x * 32 + x;
+    const bool live = e < count;
+    int64_t iw = 0;
+    int un = 0, vn = 0, bad = 0;  // bad: an error found before the sum
+    bool nu = false, nv = false;
+    const uint32_t *up = U.limbs, *vp = V.limbs;
+    if (live) {
+        iw = ent(W, e);
+        const int64_t iu = ent(U, e), iv = ent(V, e);
+        const int su = U.sizes[iu], sv = sub ? -V.sizes[iv] : V.sizes[iv];
+        un = iabs_d(su);
+        const int vn0 = iabs_d(sv);
+        vn = vn0 ? vn0 + sh : 0;
+        nu = su < 0;
+        nv = sv < 0;
+        up += iu;
+        vp += iv;
+        // a size beyond its operand's planes is malformed input: nothing past the planes is read
+        if (un > U.nlimbs || vn0 > V.nlimbs) bad = DEVERR_BADARG;
+        else if (strict && (un > W.nlimbs || vn > W.nlimbs)) bad = DEVERR_CAPACITY;
+        if (bad) un = vn = 0;
+    }
+    uint32_t r[SEG];
+    {
+        long long c = 0;
+#pragma unroll
+        for (int i0 = 0; i0 < SEG; i0 += 8) {
+            uint32_t a[8], b[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int l = l0 + i0 + i;
+                a[i] = l < un ? up[(int64_t)l * U.ld] : 0u;
+                b[i] = l >= sh && l < vn ? vp[(int64_t)(l - sh) * V.ld] : 0u;
+            }
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                c += nu ? -(long long)a[i] : (long long)a[i];
+                c += nv ? -(long long)b[i] : (long long)b[i];
+                r[i0 + i] = (uint32_t)c;
+                c >>= 32;
+            }
+        }
+        bool ones = true, zeros = true;
+#pragma unroll
+        for (int i = 1; i < SEG; i++) {
+            ones &= r[i] == 0xFFFFFFFFu;
+            zeros &= r[i] == 0u;
+        }
+        s.first[g][x] = r[0];
+        s.carry[g][x] = (signed char)c;
+        s.rest[g][x] = (ones ? 1 : 0) | (zeros ? 2 : 0);
+    }
+    if (g == 0) s.top[x] = 0;
+    __syncthreads();
+    if (g == 0) {
+        int cin = 0;
+        for (int q = 0; q < ng; q++) {
+            const uint32_t f = s.first[q][x];
+            const int rest = s.rest[q][x], c = s.carry[q][x];
+            s.carry[q][x] = (signed char)cin;
+            if (cin > 0) cin = c + ((rest & 1) && f + (uint32_t)cin < f);
+            else if (cin < 0) cin = c - ((rest & 2) && f < (uint32_t)-cin);
+            else cin = c;
+        }
+        s.fin[x] = (signed char)cin;
+    }
+    __syncthreads();
+    {
+        long long c = s.carry[g][x];
+        uint32_t nz = 0;
+#pragma unroll
+        for (int i = 0; i < SEG; i++) {
+            c += r[i];
+            r[i] = (uint32_t)c;
+            c >>= 32;
+            nz |= r[i];
+        }
+        s.zero[g][x] = nz == 0;
+    }
+    __syncthreads();
+    const int fin = s.fin[x];
+    const bool neg = fin < 0;
+    uint32_t one = neg;
+    if (neg)
+        for (int q = 0; q < g; q++) one &= s.zero[q][x];
+    int top = 0;
+#pragma unroll
+    for (int i = 0; i < SEG; i++) {
+        uint32_t v = r[i];
+        if (neg) {
+            v = ~v + one;
+            one &= (uint32_t)(r[i] == 0u);
+        }
+        if (v) top = l0 + i + 1;
+        if (live && !bad && l0 + i < W.nlimbs) W.limbs[(int64_t)(l0 + i) * W.ld + iw] = v;
+    }
+    if (top) atomicMax(&s.top[x], top);
+    __syncthreads();
+    if (g == 0 && live) {
+        const int t = s.top[x];
+        // a carry, or a negative value of 2^(32 limbs): more limbs than W has
+        if (!bad && ((fin != 0 && fin != -1) || t > W.nlimbs || (neg && t == 0))) bad = DEVERR_CAPACITY;
+        if (bad) atomicOr(err, (uint32_t)bad);
+        W.sizes[iw] = bad ? 0 : (neg ? -t : t);
+    }
+}
+
+// The same for four neighbouring entries of dense matrices per thread, with 16-byte loads
+// and stores: streams at HBM speed once there are entries enough (2^20 of 130 limbs: 449 us
+// with a thread per entry, 270 us).  Entries with an error among the four take
+// addsub_entry one by one.
+__global__ void __launch_bounds__(128) k_mpz_addsub_vec(MatArgs W, MatArgs U, MatArgs V, int sub, int64_t count, uint32_t *err) {
+    const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, e = 4 * q;
+    if (e >= count) return;
+    int un[4], vn[4], neg[4];
+    uint32_t add = 0, swap = 0;  // bit k: entry k adds magnitudes; subtracts U's from V's
+    bool ok = e + 3 < count;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        un[k] = vn[k] = neg[k] = 0;
+        if (!ok) continue;
+        const int su = U.sizes[e + k];
+        int sv = V.sizes[e + k];
+        if (sub) sv = -sv;
+        un[k] = iabs_d(su);
+        vn[k] = iabs_d(sv);
+        if (un[k] > min(U.nlimbs, W.nlimbs) || vn[k] > min(V.nlimbs, W.nlimbs)) {
+            ok = false;
+            continue;
+        }
+        const bool a = (su < 0) == (sv < 0) || un[k] == 0 || vn[k] == 0;
+        const bool w = !a && (un[k] != vn[k] ? un[k] < vn[k] : dev_cmp(U.limbs + e + k, U.ld, V.limbs + e + k, V.ld, un[k]) < 0);
+        add |= (uint32_t)a << k;
+        swap |= (uint32_t)w << k;
+        neg[k] = a ? (un[k] ? su < 0 : sv < 0) : (w ? sv < 0 : su < 0);
+    }
+    if (!ok) {
+        for (int k = 0; k < 4 && e + k < count; k++) addsub_entry(W, e + k, U, e + k, V, e + k, sub, err);
+        return;
+    }
+    const uint4 *up = reinterpret_cast<const uint4 *>(U.limbs) + q, *vp = reinterpret_cast<const uint4 *>(V.limbs) + q;
+    uint4 *wp = reinterpret_cast<uint4 *>(W.limbs) + q;
+    const int64_t us = U.ld / 4, vs = V.ld / 4, ws = W.ld / 4;
+    const int mu = max(max(un[0], un[1]), max(un[2], un[3])), mv = max(max(vn[0], vn[1]), max(vn[2], vn[3]));
+    uint32_t c[4] = {0, 0, 0, 0};
+    int len[4] = {0, 0, 0, 0};
+    for (int i0 = 0; i0 < W.nlimbs; i0 += 4) {
+        uint4 x[4], y[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            x[i] = i0 + i < mu ? up[(i0 + i) * us] : make_uint4(0, 0, 0, 0);
+            y[i] = i0 + i < mv ? vp[(i0 + i) * vs] : make_uint4(0, 0, 0, 0);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int l = i0 + i;
+            if (l >= W.nlimbs) break;
+            const uint32_t xs[4] = {x[i].x, x[i].y, x[i].z, x[i].w}, ys[4] = {y[i].x, y[i].y, y[i].z, y[i].w};
+            uint32_t r[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const uint32_t p = l < un[k] ? xs[k] : 0u, t = l < vn[k] ? ys[k] : 0u;
+                const bool sw = swap >> k & 1;
+                const uint32_t a = sw ? t : p, b = sw ? p : t;
+                const uint64_t d = add >> k & 1 ? (uint64_t)a + b + c[k] : (uint64_t)a - b - c[k];
+                c[k] = (uint32_t)(d >> 32) & 1u;  // carry or borrow
+                r[k] = (uint32_t)d;
+                if (r[k]) len[k] = l + 1;
+            }
+            wp[l * ws] = make_uint4(r[0], r[1], r[2], r[3]);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        // a carry out of W's last plane: W is too small
+        const bool bad = (add >> k & 1) && c[k];
+        if (bad) atomicOr(err, DEVERR_CAPACITY);
+        W.sizes[e + k] = bad || len[k] == 0 ? 0 : (neg[k] ? -len[k] : len[k]);
+    }
 }
 
 // w = u + sgn * v, one thread per entry.
@@ -928,13 +1208,13 @@ __global__ void __launch_bounds__(NT, 896 / NT) k_mpz_mulops_sm(MatArgs W, MatAr
     if (op == 2) pneg ^= 1;
     const bool prod = un && vn;
     const bool subtract = wn && prod && ((sw < 0) != (pneg != 0));
-    const int nu4 = __reduce_max_sync(0xFFFFFFFFu, prod ? (un + 3) >> 2 : 0);
-    const int nv4 = __reduce_max_sync(0xFFFFFFFFu, prod ? (vn + 3) >> 2 : 0);
+    const int nu = __reduce_max_sync(0xFFFFFFFFu, prod ? (un + 3) >> 2 : 0);
+    const int nv = __reduce_max_sync(0xFFFFFFFFu, prod ? (vn + 3) >> 2 : 0);
     if (!live) return;
     uint32_t *wp = W.limbs + iw;
     const int64_t ws = W.ld;
     // a zero operand is staged as zeros, so its product is zero over the warp's length too
-    const int nT = max(nu4 + nv4, (cap + 3) >> 2);
+    const int nT = max(nu + nv, (cap + 3) >> 2);
     // W's limbs of this block and of the next two (in flight)
     uint32_t wl[4], wx[4], wy[4];
     auto wload = [&](int T, uint32_t(&x)[4]) {
@@ -946,8 +1226,8 @@ __global__ void __launch_bounds__(NT, 896 / NT) k_mpz_mulops_sm(MatArgs W, MatAr
     uint32_t carry = 0;
     int top = 0;
     bool hi_nz = false, hi_ones = true;
-    sm_mul4_pre(
-        su_ + threadIdx.x * Su, nu4, sv_ + threadIdx.x * Sv, nv4, nT,
+    sm_mul_pre<4>(
+        su_ + threadIdx.x * Su, nu, sv_ + threadIdx.x * Sv, nv, nT,
         [&](int T) {
 #pragma unroll
             for (int c = 0; c < 4; c++) {
@@ -1101,106 +1381,10 @@ __device__ void add_shifted_serial(const MatArgs &W, const MatArgs &U, const Mat
     W.sizes[iw] = len == 0 ? 0 : (neg ? -len : len);
 }
 
-// The same with the limbs of an addition cut into segments: a CTA takes 32 entries
-// (one per lane, loads coalesced across entries) and each of its 8 warps one segment
-// of W's planes.  A segment is summed from carry-in 0, noting its carry-out, whether
-// it came out all ones and its top nonzero limb; warp 0 then resolves each entry's
-// segment carry-ins (carry-select), and a segment that receives a carry adds it from
-// its bottom limb (it stops at the first limb that does not wrap).  Subtractions and
-// results that would not fit W take the one-thread form.
-constexpr int ADDSH_SEGS = 8;
-constexpr int64_t ADDSH_SEG_BELOW = 48 * 1024;  // entries below which the segmented form runs
-
 __global__ void k_add_shifted(MatArgs W, MatArgs U, MatArgs V, int sh, int64_t count, uint32_t *err) {
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= count) return;
     add_shifted_serial(W, U, V, sh, e, err);
-}
-
-__global__ void __launch_bounds__(32 * ADDSH_SEGS) k_add_shifted_seg(MatArgs W, MatArgs U, MatArgs V, int sh,
-                                                                     int64_t count, uint32_t *err) {
-    __shared__ uint32_t s_carry[ADDSH_SEGS][32], s_ones[ADDSH_SEGS][32], s_cin[ADDSH_SEGS][32];
-    __shared__ int s_top[ADDSH_SEGS][32];
-    const int lane = threadIdx.x & 31, j = threadIdx.x >> 5;
-    const int64_t e = (int64_t)blockIdx.x * 32 + lane;
-    bool seg = false;  // this entry takes the segmented addition
-    int64_t iw = 0, iu = 0, iv = 0;
-    int su = 0, sv = 0, un = 0, vn0 = 0, vn = 0;
-    if (e < count) {
-        iw = ent(W, e); iu = ent(U, e); iv = ent(V, e);
-        su = U.sizes[iu]; sv = V.sizes[iv];
-        un = iabs_d(su); vn0 = iabs_d(sv); vn = vn0 ? vn0 + sh : 0;
-        const int mx = un > vn ? un : vn;
-        seg = (vn0 == 0 || un == 0 || (su < 0) == (sv < 0)) && mx <= W.nlimbs && un <= U.nlimbs && vn0 <= V.nlimbs;
-    }
-    const int S = (W.nlimbs + ADDSH_SEGS - 1) / ADDSH_SEGS;
-    const int t0 = min(j * S, W.nlimbs), t1 = min(t0 + S, W.nlimbs);
-    if (seg) {
-        const uint32_t *up = U.limbs + iu, *vp = V.limbs + iv;
-        uint32_t *wp = W.limbs + iw;
-        uint32_t c = 0, ones = 1;  // an empty segment passes a carry through
-        int top = -1;
-        for (int tb = t0; tb < t1; tb += 8) {
-            uint32_t xu[8], xv[8];
-#pragma unroll
-            for (int k = 0; k < 8; k++) {
-                const int t = tb + k;
-                xu[k] = t < un ? up[(int64_t)t * U.ld] : 0u;
-                xv[k] = (t >= sh && t < vn) ? vp[(int64_t)(t - sh) * V.ld] : 0u;
-            }
-#pragma unroll
-            for (int k = 0; k < 8; k++) {
-                const int t = tb + k;
-                if (t >= t1) break;
-                const uint64_t x = (uint64_t)xu[k] + xv[k] + c;
-                const uint32_t w = (uint32_t)x;
-                wp[(int64_t)t * W.ld] = w;
-                c = (uint32_t)(x >> 32);
-                ones &= w == 0xFFFFFFFFu;
-                if (w) top = t;
-            }
-        }
-        s_carry[j][lane] = c;
-        s_ones[j][lane] = ones;
-        s_top[j][lane] = top;
-    }
-    __syncthreads();
-    bool cap = false;  // warp 0: a carry out of W's last plane
-    if (j == 0 && seg) {
-        uint32_t cin = 0;
-        for (int q = 0; q < ADDSH_SEGS; q++) {
-            s_cin[q][lane] = cin;
-            cin = s_carry[q][lane] | (s_ones[q][lane] & cin);
-        }
-        if (cin) {
-            atomicOr(err, DEVERR_CAPACITY);
-            cap = true;
-        }
-    }
-    __syncthreads();
-    if (seg && s_cin[j][lane] && t1 > t0) {
-        uint32_t *wp = W.limbs + iw;
-        int t = t0;
-        for (; t < t1; t++) {
-            const uint32_t w = wp[(int64_t)t * W.ld] + 1u;
-            wp[(int64_t)t * W.ld] = w;
-            if (w) break;
-        }
-        s_top[j][lane] = s_ones[j][lane] ? -1 : max(s_top[j][lane], t);
-    }
-    __syncthreads();
-    if (j == 0 && e < count) {
-        if (seg) {
-            int top = -1;
-            for (int q = 0; q < ADDSH_SEGS; q++) top = max(top, s_top[q][lane]);
-            const int len = top + 1;
-            const int neg = un ? su < 0 : sv < 0;
-            // W too small: its size is set to 0 so a later reader stays inside its planes
-            W.sizes[iw] = (len == 0 || cap) ? 0 : (neg ? -len : len);
-        } else {
-            add_shifted_serial(W, U, V, sh, e, err);
-        }
-    }
 }
 
 // dst = src (entries copied with their sizes; planes beyond the value zeroed)
@@ -2053,11 +2237,39 @@ bool mpn_basecase_on_chip(int un, int vn) { return sm_threads((size_t)sm_stride(
 // whether limb planes at p with stride ld allow 16-byte loads of four operands
 static int vec16(const void *p, int64_t ld) { return ((uintptr_t)p % 16 == 0 && ld % 4 == 0) ? 1 : 0; }
 
+constexpr int64_t LIN2_MAX_ENTRIES = 128 * 1024;
+// four entries per thread from here on (dense operands)
+constexpr int64_t ADDSUB_VEC_MIN_ENTRIES = 48 * 1024;
+// Segments of the widest operand or result; false when they or the entries are too many
+// (the one-thread-per-entry kernels take those).
+static bool launch_lin2(const gbmm_mat &w, const gbmm_mat &u, const gbmm_mat &v, int sh, int sub, int strict, cudaStream_t s) {
+    const int64_t n = nentries(w), blocks = (n + 31) / 32;
+    const int64_t L = std::max<int64_t>({w.nlimbs, u.nlimbs, (int64_t)v.nlimbs + sh, 1});
+    // With many entries the whole GPU walks the limb planes in step, which HBM likes better
+    // than every block reading all planes at once: 2^20 entries of 130 limbs 449 us that way
+    // (270 us four entries per thread), 571 us segmented.
+    if (blocks > 0x7FFFFFFF || L > 1024 || n >= LIN2_MAX_ENTRIES) return false;
+    uint32_t *err = device_error_word();
+#define LIN2(SEG, MS)                                                                                              \
+    k_mpz_lin2<SEG, MS><<<(unsigned)blocks, dim3(32, (unsigned)((L + SEG - 1) / SEG)), 0, s>>>(                   \
+        margs(w), margs(u), margs(v), sh, sub, strict, n, err)
+    if (L <= 128) LIN2(8, 16);
+    else if (L <= 512) LIN2(16, 32);
+    else LIN2(32, 32);
+#undef LIN2
+    return true;
+}
+
 gbmm_status launch_mat_addsub(const gbmm_mat &c, const gbmm_mat &a, const gbmm_mat &b, int sub, cudaStream_t s) {
     const int64_t n = nentries(c);
     if (n == 0) return GBMM_OK;
     LaunchScope ls_("k_mpz_addsub", s);
-    k_mpz_addsub<<<grid1(n, 256), 256, 0, s>>>(margs(c), margs(a), margs(b), sub, n, device_error_word());
+    const bool dense = c.rs == c.cols && a.rs == a.cols && b.rs == b.cols && vec16(c.limbs, c.ld) && vec16(a.limbs, a.ld) &&
+                       vec16(b.limbs, b.ld);
+    if (n >= ADDSUB_VEC_MIN_ENTRIES && dense)
+        k_mpz_addsub_vec<<<grid1((n + 3) / 4, 128), 128, 0, s>>>(margs(c), margs(a), margs(b), sub, n, device_error_word());
+    else if (!launch_lin2(c, a, b, 0, sub, 1, s))
+        k_mpz_addsub<<<grid1(n, 256), 256, 0, s>>>(margs(c), margs(a), margs(b), sub, n, device_error_word());
     GBMM_CUDA_TRY(cudaGetLastError());
     return GBMM_OK;
 }
@@ -2092,17 +2304,9 @@ gbmm_status launch_split_sizes(const gbmm_mat &x, int h, int32_t *lo, int32_t *h
 gbmm_status launch_add_shifted(const gbmm_mat &w, const gbmm_mat &u, const gbmm_mat &v, int sh, cudaStream_t s) {
     const int64_t n = nentries(w);
     if (n == 0) return GBMM_OK;
-    // one thread per entry keeps enough loads in flight once there are many entries
-    // (75k entries of 660 planes: 0.33 ms, against 0.49 ms segmented); fewer entries
-    // take the segmented form (27k entries: 0.22 ms, against 0.29 ms)
-    if (n >= ADDSH_SEG_BELOW) {
-        LaunchScope ls_("k_add_shifted", s);
+    LaunchScope ls_("k_add_shifted", s);
+    if (!launch_lin2(w, u, v, sh, 0, 0, s))
         k_add_shifted<<<grid1(n, 256), 256, 0, s>>>(margs(w), margs(u), margs(v), sh, n, device_error_word());
-    } else {
-        LaunchScope ls_("k_add_shifted_seg", s);
-        k_add_shifted_seg<<<grid1(n, 32), 32 * ADDSH_SEGS, 0, s>>>(margs(w), margs(u), margs(v), sh, n,
-                                                                    device_error_word());
-    }
     GBMM_CUDA_TRY(cudaGetLastError());
     return GBMM_OK;
 }
@@ -2476,35 +2680,33 @@ static gbmm_status check_batch(const void *a, const void *b, int64_t ld, int64_t
     return GBMM_OK;
 }
 
-extern "C" gbmm_status gbmm_mpn_add_n(uint32_t *rp, const uint32_t *up, const uint32_t *vp, int32_t n, int64_t ld,
-                                      int64_t nb, uint32_t *cy, void *stream) {
+template <bool SUB>
+static gbmm_status addsub_n_entry(uint32_t *rp, const uint32_t *up, const uint32_t *vp, int32_t n, int64_t ld, int64_t nb,
+                                  uint32_t *cy, void *stream) {
     GBMM_TRY(check_batch(rp, up, ld, nb, n));
     if (!vp || !cy) return set_error(GBMM_ERR_INVALID, "null pointer");
     if (nb == 0) return GBMM_OK;
-    if (nb >= ADDSUB_SERIAL_MIN_OPS) {
+    if (nb >= ADDSUB_VEC_MIN_OPS && vec16(rp, ld) && vec16(up, ld) && vec16(vp, ld) && vec16(cy, 4)) {
+        LaunchScope ls_("k_mpn_addsub_n_vec", as_stream(stream));
+        k_mpn_addsub_n_vec<SUB><<<grid1(nb / 4 + nb % 4, 256), 256, 0, as_stream(stream)>>>(
+            (uint4 *)rp, (const uint4 *)up, (const uint4 *)vp, n, ld / 4, nb, (uint4 *)cy);
+    } else if (nb >= ADDSUB_SERIAL_MIN_OPS) {
         LaunchScope ls_("k_mpn_addsub_n_serial", as_stream(stream));
-        k_mpn_addsub_n_serial<false><<<grid1(nb, 256), 256, 0, as_stream(stream)>>>(rp, up, vp, n, ld, nb, cy);
+        k_mpn_addsub_n_serial<SUB><<<grid1(nb, 256), 256, 0, as_stream(stream)>>>(rp, up, vp, n, ld, nb, cy);
     } else {
         LaunchScope ls_("k_mpn_addsub_n_cla", as_stream(stream));
-        k_mpn_addsub_n_cla<false><<<grid1(nb, CLA_OPS), 256, 0, as_stream(stream)>>>(rp, up, vp, n, ld, nb, cy);
+        k_mpn_addsub_n_cla<SUB><<<grid1(nb, CLA_OPS), 256, 0, as_stream(stream)>>>(rp, up, vp, n, ld, nb, cy);
     }
     GBMM_CUDA_TRY(cudaGetLastError());
     return GBMM_OK;
 }
+extern "C" gbmm_status gbmm_mpn_add_n(uint32_t *rp, const uint32_t *up, const uint32_t *vp, int32_t n, int64_t ld,
+                                      int64_t nb, uint32_t *cy, void *stream) {
+    return addsub_n_entry<false>(rp, up, vp, n, ld, nb, cy, stream);
+}
 extern "C" gbmm_status gbmm_mpn_sub_n(uint32_t *rp, const uint32_t *up, const uint32_t *vp, int32_t n, int64_t ld,
                                       int64_t nb, uint32_t *cy, void *stream) {
-    GBMM_TRY(check_batch(rp, up, ld, nb, n));
-    if (!vp || !cy) return set_error(GBMM_ERR_INVALID, "null pointer");
-    if (nb == 0) return GBMM_OK;
-    if (nb >= ADDSUB_SERIAL_MIN_OPS) {
-        LaunchScope ls_("k_mpn_addsub_n_serial", as_stream(stream));
-        k_mpn_addsub_n_serial<true><<<grid1(nb, 256), 256, 0, as_stream(stream)>>>(rp, up, vp, n, ld, nb, cy);
-    } else {
-        LaunchScope ls_("k_mpn_addsub_n_cla", as_stream(stream));
-        k_mpn_addsub_n_cla<true><<<grid1(nb, CLA_OPS), 256, 0, as_stream(stream)>>>(rp, up, vp, n, ld, nb, cy);
-    }
-    GBMM_CUDA_TRY(cudaGetLastError());
-    return GBMM_OK;
+    return addsub_n_entry<true>(rp, up, vp, n, ld, nb, cy, stream);
 }
 template <int OP>
 static gbmm_status mul1_entry(uint32_t *rp, const uint32_t *up, int32_t n, const uint32_t *vl, int64_t ld, int64_t nb,
@@ -2636,19 +2838,25 @@ extern "C" gbmm_status gbmm_mpn_mul_basecase(uint32_t *rp, const uint32_t *up, i
         GBMM_CUDA_TRY(cudaGetLastError());
         return GBMM_OK;
     }
-    const size_t smem = (size_t)nt * (sm_stride(un) + sm_stride(vn)) * 4;
     const int vu = vec16(up, ld), vv = vec16(vp, ld);
+    const size_t words8 = (size_t)sm_stride_b<8>(un) + sm_stride_b<8>(vn);
+    const bool by8 = sm_block(un, vn) == 8 && (size_t)nt * words8 * 4 <= MPN_SM_MAX_BYTES;
+    const size_t smem = (size_t)nt * (by8 ? words8 : (size_t)sm_stride(un) + sm_stride(vn)) * 4;
     LaunchScope ls_("k_mpn_mul_basecase_sm", as_stream(stream));
-#define BASECASE_SM(NT_)                                                                                      \
-    do {                                                                                                      \
-        GBMM_CUDA_TRY(cudaFuncSetAttribute(k_mpn_mul_basecase_sm<NT_>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                           (int)smem));                                                       \
-        k_mpn_mul_basecase_sm<NT_><<<grid1(nb, NT_), NT_, smem, as_stream(stream)>>>(rp, up, un, vp, vn, ld, nb, vu, \
-                                                                                     vv);                      \
+#define BASECASE_SM(NT_, B_)                                                                                    \
+    do {                                                                                                        \
+        GBMM_CUDA_TRY(cudaFuncSetAttribute(k_mpn_mul_basecase_sm<NT_, B_>,                                      \
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));            \
+        k_mpn_mul_basecase_sm<NT_, B_><<<grid1(nb, NT_), NT_, smem, as_stream(stream)>>>(rp, up, un, vp, vn, ld, nb, \
+                                                                                         vu, vv);               \
     } while (0)
-    if (nt == 128) BASECASE_SM(128);
-    else if (nt == 64) BASECASE_SM(64);
-    else BASECASE_SM(32);
+    if (by8) {
+        if (nt == 128) BASECASE_SM(128, 8);
+        else if (nt == 64) BASECASE_SM(64, 8);
+        else BASECASE_SM(32, 8);
+    } else if (nt == 128) BASECASE_SM(128, 4);
+    else if (nt == 64) BASECASE_SM(64, 4);
+    else BASECASE_SM(32, 4);
 #undef BASECASE_SM
     GBMM_CUDA_TRY(cudaGetLastError());
     return GBMM_OK;
