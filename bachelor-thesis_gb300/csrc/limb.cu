@@ -2239,7 +2239,7 @@ static int vec16(const void *p, int64_t ld) { return ((uintptr_t)p % 16 == 0 && 
 
 constexpr int64_t LIN2_MAX_ENTRIES = 128 * 1024;
 // four entries per thread from here on (dense operands)
-constexpr int64_t ADDSUB_VEC_MIN_ENTRIES = 48 * 1024;
+constexpr int64_t ADDSUB_VEC_MIN_ENTRIES = 80 * 1024;
 // Segments of the widest operand or result; false when they or the entries are too many
 // (the one-thread-per-entry kernels take those).
 static bool launch_lin2(const gbmm_mat &w, const gbmm_mat &u, const gbmm_mat &v, int sh, int sub, int strict, cudaStream_t s) {
