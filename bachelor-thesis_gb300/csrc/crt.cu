@@ -627,6 +627,364 @@ __global__ void __launch_bounds__(RES_THREADS, 1)
 }
 
 // ======================================================================================
+// 2b. digits and residues of an operand in one kernel, for rows of up to 512 digits
+//
+// A cluster of two CTAs takes 256 entries (8 plane rows x 32 columns k) and keeps
+// their digits in shared memory for all of the table's columns: eight converter warps
+// per CTA turn the limb planes into unsigned byte digits in bf16, straight into the
+// K-major swizzled operand tiles (64 digits a slot), and the table's column tiles stream
+// through a ring.  One M = 256, N = 256 tcgen05.mma.cta_group::2 per K slice.
+// Against the digits kernel followed by the streaming GEMM above, which re-read each
+// digit tile for every 256 table columns, the digit rows are neither written nor read
+// (0.8 GB per operand at 512 x 512 entries of 4096 bits by 516 moduli), and a K step brings 16 KB into
+// an SM instead of 48.  With both operands in one launch, us, digits and residues of both
+// (two kernels each before): 64 x 64 entries of 1024 bits 16.1 (36.6), 256 x 256 of 2048 bits
+// 75 (105), 512 x 512 of 4096 bits 484 (604).  There the issue thread waits for the table's
+// tiles and for the epilogue in turn: shared memory serves the MMA's operand reads, the
+// converters and the epilogue's 2-byte stores, and is what bounds it.
+// ======================================================================================
+constexpr int R2_SLOTS = 8;   // digit tiles of 64 digits x 128 entries
+// Table tiles of 64 digits x 128 rows, and staging buffers per epilogue warp: what is left of
+// shared memory (512 x 512 entries of 4096 bits, us: 5 and 1 515, 4 and 2 527; the epilogue
+// storing residues straight to memory, and 6 tiles, 822)
+constexpr int R2_STAGES = 5, R2_NBUF = 1;
+constexpr int R2_EPI = 8, R2_CONV = 8;  // epilogue and converter warps
+constexpr int R2_THREADS = 32 * (2 + R2_EPI + R2_CONV);
+constexpr uint32_t R2_TILE = 128 * 128;
+
+struct Residue2Args {
+    const uint32_t *limbs;
+    const int32_t *sizes;
+    int64_t ld, srow, sk;  // entry (plane row, k) at srow * row + sk * k
+    int32_t rows, kdim, nlimbs;
+    int32_t hrows, hl;     // a limb-half split read in place (0: none): plane rows from hrows on are
+                           // the high halves (limbs hl ..) of rows 0 .., the others the low hl limbs
+    int32_t nk, ncols, n_ntiles;
+    int32_t nkb, ngr;      // blocks of 32 columns k; column-tile groups a row block is split into
+    int32_t units;         // row blocks x groups
+    int32_t BN;            // table columns per tile (a multiple of 32, at most 256)
+};
+struct Residue2Job {
+    CUtensorMap tmT, tmR;
+    Residue2Args a;
+};
+// unit u: its first plane row, first k and column tiles [j0, j1)
+struct Residue2Unit {
+    int row0, k0, j0, j1;
+};
+__device__ __forceinline__ Residue2Unit residue2_unit(const Residue2Args &a, int u) {
+    Residue2Unit r;
+    const int rb = u / a.ngr, gi = u - rb * a.ngr;
+    const int rg = rb / a.nkb;
+    r.row0 = rg * 8;
+    r.k0 = (rb - rg * a.nkb) * 32;
+    r.j0 = (int)((int64_t)a.n_ntiles * gi / a.ngr);
+    r.j1 = (int)((int64_t)a.n_ntiles * (gi + 1) / a.ngr);
+    return r;
+}
+struct Residue2Bars {
+    uint64_t full[R2_STAGES], empty[R2_STAGES], afull[R2_SLOTS], aempty[R2_SLOTS], tfull[2], tempty[2];
+    uint32_t tmem_base;
+    int abort_flag;
+};
+
+// One or both operands of a product as a kernel parameter (the second with 0 units: none).
+struct Residue2Two {
+    Residue2Job j[2];
+};
+
+template <bool GRP>
+__global__ void __launch_bounds__(R2_THREADS, 1)
+    k_crt_residue2(const __grid_constant__ Residue2Two two, Group<Residue2Job> grp, uint32_t *err) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *base = align1024(smem_raw);
+    uint8_t *tbase = base + R2_SLOTS * R2_TILE, *stage_out = tbase + R2_STAGES * R2_TILE;
+    Residue2Bars *bars = reinterpret_cast<Residue2Bars *>(stage_out + R2_EPI * R2_NBUF * RES_STG_BYTES);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = tc::cluster_rank();
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < R2_STAGES; i++) {
+            tc::mbar_init(&bars->full[i], 1);
+            tc::mbar_init(&bars->empty[i], 1);
+        }
+        for (int i = 0; i < R2_SLOTS; i++) {
+            tc::mbar_init(&bars->afull[i], 2 * R2_CONV);  // the even CTA's: both CTAs' converter warps
+            tc::mbar_init(&bars->aempty[i], 1);
+        }
+        for (int b = 0; b < 2; b++) {
+            tc::mbar_init(&bars->tfull[b], 1);
+            tc::mbar_init(&bars->tempty[b], 2 * R2_EPI);
+        }
+        bars->abort_flag = 0;
+        tc::fence_mbar_init();
+    }
+    if (warp == 1) {
+        tc::tmem_alloc_pair(&bars->tmem_base, 512);
+        tc::tmem_relinquish_pair();
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::cluster_sync_all();  // both CTAs' barriers exist before any cross-CTA signal
+    tc::fence_after_sync();
+    tc::grid_dep_wait();
+    const uint32_t tmem = bars->tmem_base;
+    auto give_up = [&]() {
+        atomicOr(err, DEVERR_TIMEOUT);
+        *(volatile int *)&bars->abort_flag = 1;
+    };
+    const int64_t units0 = two.j[0].a.units;
+    const int64_t total = GRP ? grp.tile0[grp.njobs] : units0 + two.j[1].a.units;
+    const int64_t t0 = blockIdx.x >> 1, tstep = gridDim.x >> 1;
+    GroupCursor cur;
+    auto job = [&](int64_t T, Residue2Args &a, const CUtensorMap *&mT, const CUtensorMap *&mR) -> Residue2Unit {
+        if (GRP) {
+            cur.seek(grp, T);
+            const Residue2Job *J = grp.jobs + cur.j;
+            a = J->a;
+            mT = &J->tmT;
+            mR = &J->tmR;
+            return residue2_unit(a, (int)(T - cur.beg));
+        }
+        const int second = T >= units0;
+        a = two.j[second].a;
+        mT = &two.j[second].tmT;
+        mR = &two.j[second].tmR;
+        return residue2_unit(a, (int)(T - (second ? units0 : 0)));
+    };
+    // the column tiles of a unit in order jj = 0, 1, ..: the narrow last tile first, so that
+    // the digit slots come free one K step at a time during a whole tile
+    auto col_tile = [](const Residue2Args &a, const Residue2Unit &U, int jj, int &n0, int &nn) {
+        const int n = U.j1 - U.j0, j = U.j0 + (jj + n - 1) % n;
+        n0 = j * a.BN;
+        nn = min(a.BN, (a.ncols - n0 + 31) / 32 * 32);
+    };
+
+    if (warp == 0) {
+        if (tc::elect_one()) {
+            int st = 0;
+            uint32_t ph = 1;
+            bool ok = true;
+            for (int64_t T = t0; T < total && ok; T += tstep) {
+                Residue2Args a;
+                const CUtensorMap *mT, *mR;
+                const Residue2Unit U = job(T, a, mT, mR);
+                for (int jj = 0; jj < U.j1 - U.j0 && ok; jj++) {
+                    int n0, nn;
+                    col_tile(a, U, jj, n0, nn);
+                    for (int s = 0; s < a.nk; s++) {
+                        if (!tc::mbar_wait(&bars->empty[st], ph)) {
+                            give_up();
+                            ok = false;
+                            break;
+                        }
+                        const uint32_t full0 = tc::mapa(tc::smem_u32(&bars->full[st]), 0);
+                        if (rank == 0) tc::mbar_arrive_expect_tx(&bars->full[st], 2 * a.BN / 2 * 128);
+                        tc::tma_load_2d_pair(tbase + st * R2_TILE, mT, full0, s * BK, n0 + (int)rank * (nn / 2));
+                        if (++st == R2_STAGES) {
+                            st = 0;
+                            ph ^= 1;
+                        }
+                    }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (rank == 0 && tc::elect_one()) {
+            const uint64_t ad0 = tc::sdesc_kmajor(tc::smem_u32(base)), bd0 = tc::sdesc_kmajor(tc::smem_u32(tbase));
+            int st = 0, lt = 0;
+            uint32_t ph = 0, sc = 0;  // sc: digit slots used before this unit
+            bool ok = true;
+            for (int64_t T = t0; T < total && ok; T += tstep) {
+                Residue2Args a;
+                const CUtensorMap *mT, *mR;
+                const Residue2Unit U = job(T, a, mT, mR);
+                (void)mT, (void)mR;
+                const int nj = U.j1 - U.j0;
+                for (int jj = 0; jj < nj && ok; jj++, lt++) {
+                    int n0, nn;
+                    col_tile(a, U, jj, n0, nn);
+                    const uint32_t idesc = tc::idesc_bf16_f32(2 * BM, (uint32_t)nn, 0, 0);
+                    const int b = lt & 1;
+                    if (lt >= 2 && !tc::mbar_wait(&bars->tempty[b], ((lt >> 1) & 1) ^ 1)) { give_up(); ok = false; break; }
+                    const uint32_t d = tmem + 256u * b;
+                    for (int s = 0; s < a.nk; s++) {
+                        const uint32_t slot = (sc + s) % R2_SLOTS;
+                        if (jj == 0 && !tc::mbar_wait(&bars->afull[slot], ((sc + s) / R2_SLOTS) & 1)) { give_up(); ok = false; break; }
+                        if (!tc::mbar_wait(&bars->full[st], ph)) { give_up(); ok = false; break; }
+                        tc::fence_after_sync();
+                        const uint64_t ad = tc::sdesc_advance(ad0, slot * R2_TILE), bd = tc::sdesc_advance(bd0, st * R2_TILE);
+#pragma unroll
+                        for (int kk = 0; kk < BK / UK; kk++)
+                            tc::mma_bf16_pair(d, tc::sdesc_advance(ad, kk * 32), tc::sdesc_advance(bd, kk * 32), idesc,
+                                              s != 0 || kk != 0);
+                        tc::mma_commit_pair(&bars->empty[st], 0x3);
+                        if (jj + 1 == nj) tc::mma_commit_pair(&bars->aempty[slot], 0x3);
+                        if (++st == R2_STAGES) {
+                            st = 0;
+                            ph ^= 1;
+                        }
+                    }
+                    if (ok) tc::mma_commit_pair(&bars->tfull[b], 0x3);
+                }
+                sc += (uint32_t)a.nk;
+            }
+        }
+    } else if (warp < 2 + R2_EPI) {
+        // epilogue: lane quadrant warp % 4 (one plane row, lane = k), four of a tile's (up to)
+        // eight 32-column chunks
+        const int quad = warp & 3, half = (warp - 2) >> 2;
+        const uint32_t lb = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(half * 128);
+        const uint32_t tempty0 = tc::mapa(tc::smem_u32(&bars->tempty[0]), 0);
+        uint16_t *stg = reinterpret_cast<uint16_t *>(stage_out + (warp - 2) * R2_NBUF * RES_STG_BYTES);
+        int lt = 0, sbuf = 0;
+        bool ok = true;
+        for (int64_t T = t0; T < total && ok; T += tstep) {
+            Residue2Args a;
+            const CUtensorMap *mT, *mR;
+            const Residue2Unit U = job(T, a, mT, mR);
+            (void)mT;
+            const int row = U.row0 + (int)rank * 4 + quad;
+            for (int jj = 0; jj < U.j1 - U.j0; jj++, lt++) {
+                int n0, nn;
+                col_tile(a, U, jj, n0, nn);
+                const int b = lt & 1;
+                if (!tc::mbar_wait(&bars->tfull[b], (lt >> 1) & 1)) { give_up(); ok = false; break; }
+                tc::fence_after_sync();
+                const int mi00 = (n0 + half * 128) >> 1;
+                const int nch = max(0, min(4, (min(nn, a.ncols - n0) - half * 128 + 31) / 32));
+                auto release = [&]() {
+                    tc::fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) tc::mbar_arrive_cluster(tempty0 + 8u * b);
+                };
+                auto chunk = [&](int ch, const uint32_t(&v)[32]) {
+                    const int mi0 = mi00 + 16 * ch;
+                    f32x2 res[8];
+                    residue_fold(v, mi0, true, res);
+                    if (row >= a.rows) return;
+                    if (lane == 0) tc::bulk_wait_read<R2_NBUF - 1>();
+                    __syncwarp();
+                    uint16_t *buf = stg + sbuf * (RES_STG_BYTES / 2);
+#pragma unroll
+                    for (int g = 0; g < 8; g++) {
+                        f32x2 h2, l2;
+                        bal_split2(res[g], h2, l2);
+                        float h0, h1, x0, x1;
+                        upk2(h2, h0, h1);
+                        upk2(l2, x0, x1);
+                        buf[(4 * g) * 32 + lane] = (uint16_t)(__float_as_uint(h0) >> 16);
+                        buf[(4 * g + 1) * 32 + lane] = (uint16_t)(__float_as_uint(x0) >> 16);
+                        buf[(4 * g + 2) * 32 + lane] = (uint16_t)(__float_as_uint(h1) >> 16);
+                        buf[(4 * g + 3) * 32 + lane] = (uint16_t)(__float_as_uint(x1) >> 16);
+                    }
+                    tc::fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0) {
+                        // planes past 2P and columns past kdim are clipped by the map
+                        tc::tma_store_3d(mR, buf, U.k0, row, 2 * mi0);
+                        tc::bulk_commit_group();
+                    }
+                    if (R2_NBUF > 1) sbuf ^= 1;
+                };
+                if (nch == 0) release();
+#pragma unroll 1
+                for (int ch = 0; ch < nch; ch++) {
+                    uint32_t v[32];
+                    tc::tmem_ld32(lb + (uint32_t)(256 * b + 32 * ch), v);
+                    tc::tmem_ld_wait(v);
+                    if (ch == nch - 1) release();
+                    chunk(ch, v);
+                }
+            }
+        }
+        if (lane == 0) tc::bulk_wait_all();  // staging buffers stay live until the stores finish
+        __syncwarp();
+    } else {
+        // converters: two threads per entry, 8 of a slot's 16 limbs each.  A's entries lie
+        // along k (lane = k); B's along the plane row x, so its warps take 8 k by 4 x.
+        const int ct = (warp - 2 - R2_EPI) * 32 + lane, part = ct >> 7;
+        const uint32_t afull0 = tc::mapa(tc::smem_u32(&bars->afull[0]), 0);
+        // All of a unit's limbs are loaded while the unit before it runs: its slots come free
+        // only during that unit's last column tile, and then each has to be filled in a K
+        // step's time (with a slot's loads issued one slot ahead, the GEMM waited for memory
+        // most of the time: 677 us for both operands at 512 x 512 entries of 4096 bits).
+        uint32_t sc = 0;
+        uint32_t v[R2_SLOTS][8];
+        int nk = 0, entry = 0;
+        uint32_t flip = 0;
+        auto fetch = [&](int64_t T) {
+            Residue2Args a;
+            const CUtensorMap *mT, *mR;
+            const Residue2Unit U = job(T, a, mT, mR);
+            (void)mT;
+            int q, kk;
+            if (a.sk == 1) {
+                q = (ct & 127) >> 5;
+                kk = lane;
+            } else {
+                q = lane >> 3;
+                kk = (((ct & 127) >> 5) << 3) + (lane & 7);
+            }
+            entry = q * 32 + kk;
+            int row = U.row0 + (int)rank * 4 + q;
+            const int k = U.k0 + kk;
+            const bool live = row < a.rows && k < a.kdim;
+            int l0 = 0, nl = a.hrows ? a.hl : a.nlimbs;
+            if (a.hrows && row >= a.hrows) {
+                row -= a.hrows;
+                l0 = a.hl;
+                nl = a.nlimbs - a.hl;
+            }
+            const int64_t off = live ? row * a.srow + k * a.sk : 0;
+            if (!live) nl = 0;
+            flip = live && a.sizes[off] < 0 ? 0x80008000u : 0u;  // the digits carry the entry's sign
+            nk = a.nk;
+            const uint32_t *src = a.limbs + off + (int64_t)(l0 + 8 * part) * a.ld;
+            nl -= 8 * part;
+#pragma unroll
+            for (int s = 0; s < R2_SLOTS; s++)
+#pragma unroll
+                for (int i = 0; i < 8; i++) v[s][i] = 16 * s + i < nl ? src[(int64_t)(16 * s + i) * a.ld] : 0u;
+        };
+        bool ok = true;
+        if (t0 < total) fetch(t0);
+        for (int64_t T = t0; T < total && ok; T += tstep) {
+            uint8_t *drow = base + entry * 128;
+#pragma unroll
+            for (int s = 0; s < R2_SLOTS; s++) {
+                if (s >= nk || !ok) continue;
+                const uint32_t slot = sc % R2_SLOTS;
+                if (sc >= R2_SLOTS && !tc::mbar_wait(&bars->aempty[slot], ((sc / R2_SLOTS) & 1) ^ 1)) {
+                    give_up();
+                    ok = false;
+                    continue;
+                }
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    const uint32_t v0 = v[s][2 * c], v1 = v[s][2 * c + 1];
+                    *reinterpret_cast<uint4 *>(drow + slot * R2_TILE + 16 * ((4 * part + c) ^ (entry & 7))) =
+                        make_uint4(byte_pair_bf16(v0, 0) ^ flip, byte_pair_bf16(v0, 2) ^ flip, byte_pair_bf16(v1, 0) ^ flip,
+                                   byte_pair_bf16(v1, 2) ^ flip);
+                }
+                tc::fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive_cluster(afull0 + 8u * slot);
+                sc++;
+            }
+            if (T + tstep < total) fetch(T + tstep);
+        }
+    }
+    tc::grid_dep_launch();
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::cluster_sync_all();  // no CTA leaves while its peer may still signal it or write its TMEM
+    if (warp == 1) {
+        tc::fence_after_sync();
+        tc::tmem_dealloc_pair(tmem, 512);
+    }
+}
+
+// ======================================================================================
 // 3. per-modulus product GEMM (persistent over (modulus, 128 x 64 output tiles);
 //    TMEM double-buffered; 8 epilogue warps)
 //
@@ -2179,12 +2537,33 @@ static gbmm_status plan_operand(crt_tables *t, const gbmm_mat &X, int transpose,
     return GBMM_OK;
 }
 
-static gbmm_status launch_operand(const OperandPlan &op, cudaStream_t s) {
-    {
+// Digits of half hf of an operand given as two stacked limb halves: the stacked operand's
+// digit rows straight from x's planes.  The high half's rows follow the low half's (A:
+// rows m.., B: columns n..); both halves carry x's sign, and digits past a half's limbs
+// read as zeros.
+static DigitArgs half_digits(const OperandPlan &op, const crt_halves &hv, int hf, dim3 &grid) {
+    const gbmm_mat &x = hv.x;
+    DigitArgs a = op.da;
+    a.limbs = x.limbs + (hf ? (int64_t)hv.hl * x.ld : 0);
+    a.sizes = x.sizes;
+    a.ld = x.ld;
+    a.rs = x.rs;
+    a.rows = x.rows;
+    a.cols = x.cols;
+    a.nlimbs = hf ? x.nlimbs - hv.hl : hv.hl;
+    a.out = op.da.out + (hf ? (int64_t)x.rows * x.cols * op.da.dxp : 0);
+    grid = dim3((unsigned)((x.cols + 31) / 32), (unsigned)((x.rows + 3) / 4), op.dgrid.z);
+    return a;
+}
+
+static gbmm_status launch_operand(const OperandPlan &op, const crt_halves *halves, cudaStream_t s) {
+    for (int hf = 0; hf < (halves ? 2 : 1); hf++) {
+        dim3 grid = op.dgrid;
+        const DigitArgs da = halves ? half_digits(op, *halves, hf, grid) : op.da;
         LaunchScope ls_("k_crt_digits", s);
         const Group<DigitJob> none{nullptr, nullptr, 0};
-        if (op.balanced) GBMM_TRY(launch_one(k_crt_digits<true, false>, op.dgrid, 256, 0, s, op.da, none));
-        else GBMM_TRY(launch_one(k_crt_digits<false, false>, op.dgrid, 256, 0, s, op.da, none));
+        if (op.balanced) GBMM_TRY(launch_one(k_crt_digits<true, false>, grid, 256, 0, s, da, none));
+        else GBMM_TRY(launch_one(k_crt_digits<false, false>, grid, 256, 0, s, da, none));
         GBMM_CUDA_TRY(cudaGetLastError());
     }
     const Group<ResidueJob> none{nullptr, nullptr, 0};
@@ -2212,6 +2591,81 @@ static gbmm_status launch_operand(const OperandPlan &op, cudaStream_t s) {
 #undef RESIDUE_LAUNCH
     GBMM_CUDA_TRY(cudaGetLastError());
     return GBMM_OK;
+}
+
+// The one-kernel form of the same (k_crt_residue2).  It takes rows of up to 512 digits,
+// unless an operand is large and most of its 8 x 32 blocks padding.  Measured, digits and
+// residues of both operands: 1024 x 16 x 1024 entries of 2048 bits 47 us, 61 in two kernels;
+// 8192 x 8 x 16 of 4096 bits 228 and 255; 16384 x 6 x 16 of 2048 bits (5.3 times the entries)
+// 222 and 267; 16384 x 4 x 16 of 4096 bits (8 times) 440 and 409; 65536 x 1 x 16 of 1024 bits 505 and
+// 418.  Up to 64 K padded entries are three or four waves, and the second launch costs more.
+static bool residue2_ok(const gbmm_mat &X, int rowsR, int kdim) {
+    if (g_residue_mode >= 0 || operand_dxp(X) / BK > R2_SLOTS) return false;
+    const int64_t padded = (int64_t)((kdim + 31) / 32 * 32) * ((rowsR + 7) / 8 * 8), E = (int64_t)rowsR * kdim;
+    return padded <= 6 * E || padded <= 65536;
+}
+// 256-entry row blocks of an operand
+static int64_t residue2_blocks(int rowsR, int kdim) { return (int64_t)((kdim + 31) / 32) * ((rowsR + 7) / 8); }
+// Into how many CTA pairs the column tiles of a row block are split: few row blocks (of all
+// the launch's operands together) leave pairs idle; each pair then converts the digits itself
+// (about a third of a column tile's time).
+static int residue2_split(int64_t blocks, int ncols) {
+    const int64_t pairs = std::max(1, num_sms() / 2);
+    const int nt = (ncols + 255) / 256;
+    int best_g = 1;
+    double best = 1e30;
+    for (int g = 1; g <= nt; g++) {
+        const double c = (double)((blocks * g + pairs - 1) / pairs) * (0.35 + (double)((nt + g - 1) / g));
+        if (c < best) {
+            best = c;
+            best_g = g;
+        }
+    }
+    return best_g;
+}
+static gbmm_status plan_residue2(crt_tables *t, const gbmm_mat &X, int transpose, int rowsR, int kdim, int kp, int weighted,
+                                 __nv_bfloat16 *R, const crt_halves *halves, int ngr, Residue2Job &rp) {
+    const int dxp = operand_dxp(X);
+    __nv_bfloat16 *T = nullptr;
+    int tpitch = dxp;
+    GBMM_TRY(residue_table(t, dxp, weighted, &T, &tpitch));
+    memset(&rp, 0, sizeof rp);
+    Residue2Args &a = rp.a;
+    const gbmm_mat &x = halves ? halves->x : X;
+    a.limbs = x.limbs; a.sizes = x.sizes; a.ld = x.ld;
+    a.srow = transpose ? 1 : x.rs;
+    a.sk = transpose ? x.rs : 1;
+    a.rows = rowsR; a.kdim = kdim; a.nlimbs = x.nlimbs;
+    if (halves) {
+        a.hrows = rowsR / 2;
+        a.hl = halves->hl;
+    }
+    a.nk = dxp / BK;
+    a.ncols = residue_cols(t->P);
+    a.n_ntiles = (a.ncols + 255) / 256;
+    a.nkb = (kdim + 31) / 32;
+    const int64_t rb = residue2_blocks(rowsR, kdim);
+    a.ngr = ngr;
+    if (rb * a.ngr > INT32_MAX / 2) return set_error(GBMM_ERR_UNSUPPORTED, "crt: too many entries in one operand");
+    a.units = (int32_t)(rb * a.ngr);
+    // One tile per pair: the widest is the launch's time, so they are of about equal width
+    // (both operands at 64 x 64 entries of 1024 bits: 28 us, 30 in tiles of 256).  Otherwise
+    // full tiles and a narrow last one, whose MMAs cost less than the rounding of equal ones
+    // to 32 columns (512 x 512 of 4096 bits: 526 us, 542 in equal tiles).
+    a.BN = a.ngr == a.n_ntiles ? ((a.ncols + a.n_ntiles - 1) / a.n_ntiles + 31) / 32 * 32 : 256;
+    GBMM_TRY(make_map(&rp.tmT, T, dxp, residue_cols(t->P), tpitch, BK, (uint32_t)a.BN / 2));
+    GBMM_TRY(make_map_planes(&rp.tmR, R, kdim, rowsR, 2 * t->P, kp, (uint64_t)rowsR * kp));
+    return GBMM_OK;
+}
+static constexpr size_t R2_SMEM =
+    (size_t)(R2_SLOTS + R2_STAGES) * R2_TILE + (size_t)R2_EPI * R2_NBUF * RES_STG_BYTES + sizeof(Residue2Bars) + 1024 + 64;
+static gbmm_status launch_residue2(const Residue2Two &two, cudaStream_t s) {
+    auto kern = k_crt_residue2<false>;
+    GBMM_TRY(set_smem((const void *)kern, R2_SMEM));
+    LaunchScope ls_("k_crt_residue", s);
+    const Group<Residue2Job> none{nullptr, nullptr, 0};
+    return launch_pairs(kern, R2_THREADS, (int64_t)two.j[0].a.units + two.j[1].a.units, R2_SMEM, s, two, none,
+                        device_error_word());
 }
 
 // Product GEMM over residue planes RA [2P][m][kp] and RB [2P][n][kp].  The maps'
@@ -2357,7 +2811,7 @@ size_t crt_workspace_bytes(int la, int lb, int m, int k, int n, int cn) {
 bool crt_single_pass(int k) { return k <= PROD_MAX_K; }
 
 gbmm_status crt_matmul(gbmm_handle h, const gbmm_mat &c, const gbmm_mat &a, const gbmm_mat &b, int64_t bits_a,
-                       int64_t bits_b, int nprimes, int accumulate, cudaStream_t s) {
+                       int64_t bits_b, int nprimes, int accumulate, cudaStream_t s, const crt_halves *halves) {
     const int m = a.rows, k = a.cols, n = b.cols;
     // stage hooks apply to this product only; any branch but the single-pass one
     // waits for B at once and runs the reconstruction whole
@@ -2369,6 +2823,8 @@ gbmm_status crt_matmul(gbmm_handle h, const gbmm_mat &c, const gbmm_mat &a, cons
     }
     if (m == 0 || n == 0) return GBMM_OK;
     if (k == 0) return accumulate ? GBMM_OK : launch_mat_zero(c, s);
+    if (halves && (accumulate || k > PROD_MAX_K))
+        return set_error(GBMM_ERR_UNSUPPORTED, "crt: stacked halves need a single-pass product");
     if (accumulate) {
         // C += A*B: product into a workspace matrix, then one elementwise add
         size_t mark = arena_mark(h);
@@ -2417,20 +2873,44 @@ gbmm_status crt_matmul(gbmm_handle h, const gbmm_mat &c, const gbmm_mat &a, cons
     // Nothing is cleared: the product reads RA / RB through maps k columns wide and
     // Y through a map 2P rows deep per 64-entry block, and the padding entries
     // E .. Ep-1 of Y only reach accumulator rows that are never stored.
-    {
-        size_t mk = arena_mark(h);
-        OperandPlan op;
-        __nv_bfloat16 *D = (__nv_bfloat16 *)arena_alloc(h, digits_bytes(a));
-        if (!D) return set_error(GBMM_ERR_NOMEM, "crt: workspace for digits");
-        GBMM_TRY(plan_operand(t, a, 0, m, k, kp, 0, RA, D, false, op));
-        GBMM_TRY(launch_operand(op, s));
-        arena_release(h, mk);
-        if (hk && hk->b_ready) GBMM_CUDA_TRY(cudaStreamWaitEvent(s, hk->b_ready, 0));
-        D = (__nv_bfloat16 *)arena_alloc(h, digits_bytes(b));
-        if (!D) return set_error(GBMM_ERR_NOMEM, "crt: workspace for digits");
-        GBMM_TRY(plan_operand(t, b, 1, n, k, kp, 1, RB, D, false, op));
-        GBMM_TRY(launch_operand(op, s));
-        arena_release(h, mk);
+    // Both operands in one launch where they take the one-kernel form, unless B is still on
+    // its way: small operands then fill the chip together and large ones share a last wave.
+    // Two launches and one, us for both operands: 64 x 64 entries of 1024 bits 31.9 and 16.1,
+    // 256 x 256 of 2048 bits 93 and 75, 512 x 512 of 4096 bits 515 and 484.
+    const bool both = residue2_ok(a, m, k) && residue2_ok(b, n, k) && !(hk && hk->b_ready);
+    if (both) {
+        const int split = residue2_split(residue2_blocks(m, k) + residue2_blocks(n, k), residue_cols(P));
+        Residue2Two two;
+        for (int side = 0; side < 2; side++) {
+            // the operand with the longer rows first
+            const int slot = operand_dxp(b) > operand_dxp(a) ? 1 - side : side;
+            GBMM_TRY(plan_residue2(t, side ? b : a, side, side ? n : m, k, kp, side, side ? RB : RA,
+                                   halves && halves->side == side ? halves : nullptr, split, two.j[slot]));
+        }
+        GBMM_TRY(launch_residue2(two, s));
+    } else {
+        for (int side = 0; side < 2; side++) {
+            const gbmm_mat &x = side ? b : a;
+            __nv_bfloat16 *R = side ? RB : RA;
+            const int rows = side ? n : m;
+            const crt_halves *hv = halves && halves->side == side ? halves : nullptr;
+            if (side == 1 && hk && hk->b_ready) GBMM_CUDA_TRY(cudaStreamWaitEvent(s, hk->b_ready, 0));
+            if (residue2_ok(x, rows, k)) {
+                Residue2Two two;
+                memset(&two, 0, sizeof two);
+                const int split = residue2_split(residue2_blocks(rows, k), residue_cols(P));
+                GBMM_TRY(plan_residue2(t, x, side, rows, k, kp, side, R, hv, split, two.j[0]));
+                GBMM_TRY(launch_residue2(two, s));
+                continue;
+            }
+            size_t mk = arena_mark(h);
+            OperandPlan op;
+            __nv_bfloat16 *D = (__nv_bfloat16 *)arena_alloc(h, digits_bytes(x));
+            if (!D) return set_error(GBMM_ERR_NOMEM, "crt: workspace for digits");
+            GBMM_TRY(plan_operand(t, x, side, rows, k, kp, side, R, D, false, op));
+            GBMM_TRY(launch_operand(op, hv, s));
+            arena_release(h, mk);
+        }
     }
     {
         ProductPlan pp;
@@ -2495,14 +2975,14 @@ struct crt_group {
     // with several (table tiles of 128 or 64 columns, a deeper ring of smaller
     // stages); rec[2 f + d]: reconstructions of products with (f = 1) and without a post
     // step, by table digits (d = 1: base 256)
-    std::vector<Rec> dig[2], res[3], prod, rec[4];
+    std::vector<Rec> dig[2], res[3], res2, prod, rec[4];  // res2: operands whose digits and residues are one kernel
     std::vector<std::function<gbmm_status(cudaStream_t)>> post;
     struct Sect {
         size_t jobs_off = 0, tile0_off = 0;
         int n = 0;
         int64_t total = 0;
     };
-    Sect sdig[2], sres[3], sprod, srec[4];
+    Sect sdig[2], sres[3], sres2, sprod, srec[4];
     size_t smem_prod = 0, smem_rec = 0;
     std::vector<char> blob;
 };
@@ -2543,34 +3023,31 @@ gbmm_status crt_group_add(gbmm_handle h, crt_group *g, const gbmm_mat &c, const 
     __nv_bfloat16 *RA = (__nv_bfloat16 *)arena_alloc(h, (size_t)2 * P * m * kp * 2);
     __nv_bfloat16 *RB = (__nv_bfloat16 *)arena_alloc(h, (size_t)2 * P * n * kp * 2);
     __nv_bfloat16 *Y = (__nv_bfloat16 *)arena_alloc(h, (size_t)2 * t->Pp * Ep * 2);
-    __nv_bfloat16 *DA = (__nv_bfloat16 *)arena_alloc(h, digits_bytes(a));
-    __nv_bfloat16 *DB = (__nv_bfloat16 *)arena_alloc(h, digits_bytes(b));
-    if (!RA || !RB || !Y || !DA || !DB) return set_error(GBMM_ERR_NOMEM, "crt group: workspace");
+    if (!RA || !RB || !Y) return set_error(GBMM_ERR_NOMEM, "crt group: workspace");
     for (int side = 0; side < 2; side++) {
+        const gbmm_mat &xs = side ? b : a;
+        __nv_bfloat16 *R = side ? RB : RA;
+        const int rows = side ? n : m;
+        const crt_halves *hv = halves && halves->side == side ? halves : nullptr;
+        if (residue2_ok(xs, rows, k)) {
+            Residue2Job j2;  // not split: the batch's other products fill the chip
+            GBMM_TRY(plan_residue2(t, xs, side, rows, k, kp, side, R, hv, 1, j2));
+            g->res2.push_back(make_rec(j2, j2.a.units, (double)j2.a.nk * j2.a.n_ntiles));
+            continue;
+        }
+        __nv_bfloat16 *D = (__nv_bfloat16 *)arena_alloc(h, digits_bytes(xs));
+        if (!D) return set_error(GBMM_ERR_NOMEM, "crt group: workspace");
         OperandPlan op;
-        if (side == 0) GBMM_TRY(plan_operand(t, a, 0, m, k, kp, 0, RA, DA, true, op));
-        else GBMM_TRY(plan_operand(t, b, 1, n, k, kp, 1, RB, DB, true, op));
-        if (halves && halves->side == side) {
-            // the stacked operand's digit rows straight from x's two limb halves: the
-            // high half's rows follow the low half's (A: rows m.., B: columns n..); both
-            // halves carry x's sign, and digits past a half's limbs read as zeros
-            const gbmm_mat &x = halves->x;
-            const int64_t xe = (int64_t)x.rows * x.cols;
+        GBMM_TRY(plan_operand(t, xs, side, rows, k, kp, side, R, D, true, op));
+        if (hv) {
             for (int hf = 0; hf < 2; hf++) {
                 DigitJob dj;
                 memset(&dj, 0, sizeof dj);
-                dj.a = op.da;
-                dj.a.limbs = x.limbs + (hf ? (int64_t)halves->hl * x.ld : 0);
-                dj.a.sizes = x.sizes;
-                dj.a.ld = x.ld;
-                dj.a.rs = x.rs;
-                dj.a.rows = x.rows;
-                dj.a.cols = x.cols;
-                dj.a.nlimbs = hf ? x.nlimbs - halves->hl : halves->hl;
-                dj.a.out = op.da.out + (hf ? xe * op.da.dxp : 0);
-                dj.nbx = (x.cols + 31) / 32;
-                dj.nby = (x.rows + 3) / 4;
-                g->dig[op.balanced].push_back(make_rec(dj, (int64_t)dj.nbx * dj.nby * op.dgrid.z, 1.0));
+                dim3 grid;
+                dj.a = half_digits(op, *hv, hf, grid);
+                dj.nbx = (int32_t)grid.x;
+                dj.nby = (int32_t)grid.y;
+                g->dig[op.balanced].push_back(make_rec(dj, (int64_t)grid.x * grid.y * grid.z, 1.0));
             }
         } else {
             DigitJob dj;
@@ -2626,6 +3103,7 @@ const std::vector<char> &crt_group_blob(crt_group *g) {
     g->blob.clear();
     for (int f = 0; f < 2; f++) pack_section(g->blob, g->dig[f], g->sdig[f]);
     for (int f = 0; f < 3; f++) pack_section(g->blob, g->res[f], g->sres[f]);
+    pack_section(g->blob, g->res2, g->sres2);
     pack_section(g->blob, g->prod, g->sprod);
     for (int f = 0; f < 4; f++) pack_section(g->blob, g->rec[f], g->srec[f]);
     return g->blob;
@@ -2684,6 +3162,15 @@ gbmm_status crt_group_launch(crt_group *g, const char *d_blob, cudaStream_t s, c
                                 group_at<ResidueJob>(d_blob, sec), err));
         }
         GBMM_CUDA_TRY(cudaGetLastError());
+    }
+    if (g->sres2.n) {
+        Residue2Two none;
+        memset(&none, 0, sizeof none);
+        auto kern = k_crt_residue2<true>;
+        GBMM_TRY(set_smem((const void *)kern, R2_SMEM));
+        LaunchScope ls_("k_crt_residue", s);
+        GBMM_TRY(launch_pairs(kern, R2_THREADS, g->sres2.total, R2_SMEM, s, none,
+                              group_at<Residue2Job>(d_blob, g->sres2), err));
     }
     if (g->sprod.n) {
         ProductArgs none;

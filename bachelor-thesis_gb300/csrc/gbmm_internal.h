@@ -125,8 +125,18 @@ gbmm_status ltc_wino_leaves(gbmm_handle h, const WinoTree &t, int64_t leaves, cu
 struct crt_cache;
 crt_cache *crt_cache_create();
 void crt_cache_destroy(crt_cache *);
+// An operand of a CRT product given as the two limb halves of x (a limb-half
+// split), read in place: side 0, A = [x_lo; x_hi] stacked by rows; side 1, B =
+// [x_lo | x_hi] stacked by columns; x_lo holds x's low hl limbs, x_hi the rest.
+// The stacked operand passed beside it then only gives the shape.
+struct crt_halves {
+    int side;
+    gbmm_mat x;
+    int hl;
+};
 gbmm_status crt_matmul(gbmm_handle h, const gbmm_mat &c, const gbmm_mat &a, const gbmm_mat &b,
-                       int64_t bits_a, int64_t bits_b, int nprimes, int accumulate, cudaStream_t s);
+                       int64_t bits_a, int64_t bits_b, int nprimes, int accumulate, cudaStream_t s,
+                       const crt_halves *halves = nullptr);
 // whether the CRT kernels take la x lb limb entries with inner dimension k directly
 bool crt_feasible(int la, int lb, int k);
 // device workspace one crt_matmul call with these shapes carves from the arena
@@ -142,15 +152,6 @@ struct crt_group;
 crt_group *crt_group_create();
 void crt_group_destroy(crt_group *g);
 bool crt_group_empty(const crt_group *g);
-// An operand of a grouped product given as the two limb halves of x (a limb-half
-// split), read in place: side 0, A = [x_lo; x_hi] stacked by rows; side 1, B =
-// [x_lo | x_hi] stacked by columns; x_lo holds x's low hl limbs, x_hi the rest.
-// The stacked operand passed to crt_group_add then only gives the shape.
-struct crt_halves {
-    int side;
-    gbmm_mat x;
-    int hl;
-};
 gbmm_status crt_group_add(gbmm_handle h, crt_group *g, const gbmm_mat &c, const gbmm_mat &a, const gbmm_mat &b,
                           int64_t bits_a, int64_t bits_b, int nprimes, const crt_halves *halves = nullptr);
 // a step run after the reconstructions of the products added with halves (their

@@ -1396,27 +1396,45 @@ gbmm_status dispatch(gbmm_handle h, const gbmm_mat &c, const gbmm_mat &a, const 
     if (X.nlimbs < 2) return set_error(GBMM_ERR_UNSUPPORTED, "no kernel takes %d x %d limb entries", a.nlimbs, b.nlimbs);
     const int hl = X.nlimbs / 2, hn = X.nlimbs - hl;
     size_t mark = arena_mark(h);
-    const size_t xs = (size_t)(X.rows - 1) * X.rs + X.cols;
-    int32_t *lo = (int32_t *)arena_alloc(h, xs * 4), *hi = (int32_t *)arena_alloc(h, xs * 4);
     // S: the stacked halves (hn limb planes); T: the stacked product
     gbmm_mat S, T;
     const int tn = limbs_needed(sa ? hn : a.nlimbs, sa ? b.nlimbs : hn, k, 0) + 1;
-    if (!lo || !hi || !arena_mat(h, sa ? 2 * m : k, sa ? k : 2 * n, hn, S) ||
-        !arena_mat(h, sa ? 2 * m : m, sa ? n : 2 * n, tn, T))
-        return set_error(GBMM_ERR_NOMEM, "split workspace");
-    GBMM_TRY(launch_split_sizes(X, hl, lo, hi, s));
-    gbmm_mat Xlo = X, Xhi = X;
-    Xlo.nlimbs = hl;
-    Xlo.sizes = lo;
-    Xhi.nlimbs = hn;
-    Xhi.limbs = X.limbs + (int64_t)hl * X.ld;
-    Xhi.sizes = hi;
-    const int xr = X.rows, xc = X.cols;
-    GBMM_TRY(launch_mat_copy(sa ? sub_view(S, 0, 0, xr, xc) : sub_view(S, 0, 0, xr, xc), Xlo, s));
-    GBMM_TRY(launch_mat_copy(sa ? sub_view(S, xr, 0, xr, xc) : sub_view(S, 0, xc, xr, xc), Xhi, s));
+    if (!arena_mat(h, sa ? 2 * m : m, sa ? n : 2 * n, tn, T)) return set_error(GBMM_ERR_NOMEM, "split workspace");
     Plan q = p;
     q.split = std::max(0, p.split - 1);
-    gbmm_status st = dispatch(h, T, sa ? S : a, sa ? b : S, q, 0, s);
+    gbmm_status st;
+    if (q.path == GBMM_PATH_CRT && crt_single_pass(k) && direct_ok(q, sa ? hn : a.nlimbs, sa ? b.nlimbs : hn, k)) {
+        // one single-pass CRT product: its digits come straight from the two limb halves
+        memset(&S, 0, sizeof S);
+        S.rows = sa ? 2 * m : k;
+        S.cols = sa ? k : 2 * n;
+        S.nlimbs = hn;
+        crt_halves hv;
+        hv.side = sa ? 0 : 1;
+        hv.x = X;
+        hv.hl = hl;
+        const int saved = h->crt_tiles;
+        h->crt_tiles = q.tiles;
+        st = crt_matmul(h, T, sa ? S : a, sa ? b : S, 32LL * (sa ? hn : a.nlimbs), 32LL * (sa ? b.nlimbs : hn), q.nprimes, 0,
+                        s, &hv);
+        h->crt_tiles = saved;
+    } else {
+        const size_t xs = (size_t)(X.rows - 1) * X.rs + X.cols;
+        int32_t *lo = (int32_t *)arena_alloc(h, xs * 4), *hi = (int32_t *)arena_alloc(h, xs * 4);
+        if (!lo || !hi || !arena_mat(h, sa ? 2 * m : k, sa ? k : 2 * n, hn, S))
+            return set_error(GBMM_ERR_NOMEM, "split workspace");
+        GBMM_TRY(launch_split_sizes(X, hl, lo, hi, s));
+        gbmm_mat Xlo = X, Xhi = X;
+        Xlo.nlimbs = hl;
+        Xlo.sizes = lo;
+        Xhi.nlimbs = hn;
+        Xhi.limbs = X.limbs + (int64_t)hl * X.ld;
+        Xhi.sizes = hi;
+        const int xr = X.rows, xc = X.cols;
+        GBMM_TRY(launch_mat_copy(sub_view(S, 0, 0, xr, xc), Xlo, s));
+        GBMM_TRY(launch_mat_copy(sa ? sub_view(S, xr, 0, xr, xc) : sub_view(S, 0, xc, xr, xc), Xhi, s));
+        st = dispatch(h, T, sa ? S : a, sa ? b : S, q, 0, s);
+    }
     const gbmm_mat T0 = sub_view(T, 0, 0, m, n), T1 = sa ? sub_view(T, m, 0, m, n) : sub_view(T, 0, n, m, n);
     if (st == GBMM_OK && accumulate) st = launch_add_shifted(c, c, T0, 0, s);
     if (st == GBMM_OK) st = launch_add_shifted(c, accumulate ? c : T0, T1, hl, s);
