@@ -992,6 +992,12 @@ __global__ void __launch_bounds__(R2_THREADS, 1)
 // (residues of B, already multiplied by the CRT weight w = (Mod/p)^-1 mod p),
 // the weighted product is
 //     y = a b w = 65536 a1 u1 + 256 (a1 u0 + a0 u1) + a0 u0   (mod p).
+// The epilogue takes 256 (256 d11 + d10 + d01) + d00 mod p on two columns at a time (packed
+// FP32), three reductions for an entry.  With a short inner dimension it is what bounds the kernel:
+// reads of tensor memory, staging and stores keep the load/store pipe two thirds busy and the warps wait
+// for one another's data.  1024 x 64 x 1024 by 259 moduli 302 us, 380 with five scalar
+// reductions; 512 x 512 x 512 by 516 moduli 350 us, 390 (the MMAs alone: 295).  Sixteen epilogue
+// warps, 16 columns each or on alternate tiles, were no faster (321-350 and 306 us).
 // Each K step issues two N = 128 MMAs against the stacked operand [U1; U0]:
 // A1 into [a1 u1 | a1 u0] and A0 into [a0 u1 | a0 u0].  Each of the four 64-column
 // accumulators sums k products of magnitude <= 2^14: at most 2^23 for k <= 512,
@@ -1220,24 +1226,32 @@ __global__ void __launch_bounds__(CTA_THREADS8, 1)
             // lanes share mi); the same values as the moduli table's
             const float4 cmp = c_modpair[mi >> 1];
             const float pf = (mi & 1) ? cmp.y : cmp.x, ipf = (mi & 1) ? cmp.w : cmp.z;
+            const f32x2 np = pk2(-pf, -pf), ip = pk2(ipf, ipf), np8 = pk2(-pf / 256.f, -pf / 256.f), ip8 = pk2(256.f * ipf, 256.f * ipf);
+            // (256 x mod p) / 256, |256 x / p| < 2^17: the quotient is off by less than 0.01, and the
+            // difference is a multiple of 1/256 below 2^16 / 256, so the FMA gives it exactly
+            auto red8 = [&](f32x2 x) {
+                const f32x2 q = add2(fma2(x, ip8, pk2(RND_MAGIC, RND_MAGIC)), pk2(-RND_MAGIC, -RND_MAGIC));
+                return fma2(q, np8, x);
+            };
+            auto pair = [](const uint32_t(&v)[32], int j) { return pk2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])); };
             uint32_t plo[16];
 #pragma unroll
             for (int c = 0; c < 32; c += 8) {
                 uint32_t phi[4];
 #pragma unroll
-                for (int j = 0; j < 8; j += 2) {
-                    float h2[2], l2[2];
-#pragma unroll
-                    for (int u = 0; u < 2; u++) {
-                        // |a1 u0 + a0 u1| <= 2^24; each step below stays under 257 * 32772 < 2^24
-                        const float r2 = red(__uint_as_float(D11[c + j + u]), pf, ipf);
-                        const float r1 = red(__uint_as_float(D10[c + j + u]) + __uint_as_float(D01[c + j + u]), pf, ipf);
-                        const float r0 = red(__uint_as_float(D00[c + j + u]), pf, ipf);
-                        const float tt = red(__fmaf_rn(256.f, r2, r1), pf, ipf);
-                        bal_split(red(__fmaf_rn(256.f, tt, r0), pf, ipf), h2[u], l2[u]);
-                    }
-                    phi[j / 2] = bf16x2_bits(h2[0], h2[1]);
-                    plo[(c + j) / 2] = bf16x2_bits(l2[0], l2[1]);
+                for (int j = c; j < c + 8; j += 2) {
+                    // y = 256 (256 d11 + d10 + d01) + d00, each 256 x taken mod p.  |d10 + d01| <=
+                    // 2^15 k, so with 256 d11 mod p added it stays below 2^24 up to k = 448
+                    f32x2 mid = add2(pair(D10, j), pair(D01, j));
+                    if (a.nk > 7) mid = red2(mid, np, ip);
+                    const f32x2 w = red8(fma2(red8(pair(D11, j)), pk2(256.f, 256.f), mid));
+                    f32x2 h2, l2;
+                    bal_split2(red2(fma2(w, pk2(256.f, 256.f), pair(D00, j)), np, ip), h2, l2);
+                    float h0, h1, l0, l1;
+                    upk2(h2, h0, h1);
+                    upk2(l2, l0, l1);
+                    phi[(j - c) / 2] = __byte_perm(__float_as_uint(h0), __float_as_uint(h1), 0x7632);
+                    plo[j / 2] = __byte_perm(__float_as_uint(l0), __float_as_uint(l1), 0x7632);
                 }
                 stg[lane * 4 + ((c >> 3) ^ swz)] = make_uint4(phi[0], phi[1], phi[2], phi[3]);
             }
