@@ -115,6 +115,8 @@ gbmm_status launch_wino_combine(const WinoTree &t, int d, cudaStream_t s);
 // whether `leaves` products of these shapes run faster there than on the per-entry
 // kernel, their workspace, and the products; *done = false (nothing launched) when the
 // handle's workspace has no room
+int ltc_wino_levels(int N, int levels, int la, int lb);
+bool ltc_wino_fits(int hh, int la, int lb, int64_t leaves, size_t room);
 bool ltc_pays(int m, int k, int n, int la, int lb, int64_t leaves);
 size_t ltc_ws(int m, int k, int n, int la, int lb, int64_t leaves);
 gbmm_status ltc_matmul(gbmm_handle h, const gbmm_mat &c, const gbmm_mat &a, const gbmm_mat &b, int accumulate,

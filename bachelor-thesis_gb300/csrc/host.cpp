@@ -904,10 +904,23 @@ static bool wino_bf_ok(int method, int N, int levels, int addmul, int capSA, int
     return wino_bf_ws(N, levels, capSA, capSB, capP) <= WINO_BF_MAX_BYTES;
 }
 
+static int64_t pow7_h(int l) {
+    int64_t r = 1;
+    while (l-- > 0) r *= 7;
+    return r;
+}
+
 // Breadth-first Winograd: sums of every level, then all leaf products in one
 // launch, then the combinations of every level bottom up (kernels in limb.cu).
-// Same products and sums as rec_winograd, so the same exact result.
+// Same products and sums as rec_winograd down to its leaves, so the same exact result.
 gbmm_status rec_winograd_bf(RecCtx &c, gbmm_mat C, gbmm_mat A, gbmm_mat B, int N, int levels) {
+    if (c.h->limb_tc) {
+        // fewer levels where that is faster on the tensor cores and the workspace, which was
+        // reserved for all of them, holds the larger leaves' operands
+        const int l = ltc_wino_levels(N, levels, c.capSA, c.capSB);
+        const size_t tree = wino_bf_ws(N, l, c.capSA, c.capSB, c.capP), room = c.h->ws.cap - c.h->ws.top;
+        if (l < levels && room > tree && ltc_wino_fits(N >> l, c.capSA, c.capSB, pow7_h(l), room - tree)) levels = l;
+    }
     WinoTree t;
     t.A = A;
     t.B = B;
@@ -1141,11 +1154,6 @@ static gbmm_mat wt_operand_h(const WinoTree &t, int which, int d, int64_t node) 
     return v;
 }
 
-static int64_t pow7_h(int l) {
-    int64_t r = 1;
-    while (l-- > 0) r *= 7;
-    return r;
-}
 static constexpr int WINO_CRT_MAX_LEVELS = 4;  // 2401 leaf products at most
 
 // Whether a product takes Winograd's tree with CRT leaves: square, at least one
@@ -1330,7 +1338,9 @@ size_t limb_tc_extra(const Plan &p, int la, int lb, int m, int k, int n) {
     size_t x = 0;
     if (ltc_pays(m, k, n, la + up, lb + up, 1)) x = ltc_ws(m, k, n, la + up, lb + up, 1) + 4096;
     if (p.method == GBMM_METHOD_WINOGRAD && m == k && k == n) {
-        const int L = levels_for(m, p.cutoff), hl = m >> L;
+        int L = levels_for(m, p.cutoff);
+        if (L >= 1 && L <= WINO_MAX_LEVELS) L = ltc_wino_levels(m, L, la + 1, lb + 1);
+        const int hl = m >> L;
         if (L >= 1 && L <= WINO_MAX_LEVELS && ltc_pays(hl, hl, hl, la + 1, lb + 1, pow7_h(L))) {
             const size_t per = ltc_ws(hl, hl, hl, la + 1, lb + 1, 1) + 4096;
             x = std::max(x, per * (size_t)std::min<int64_t>(pow7_h(L), std::max<int64_t>(64, (int64_t)(WINO_BYTES / per))));

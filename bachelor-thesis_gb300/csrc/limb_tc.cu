@@ -606,14 +606,11 @@ size_t ltc_ws(int m, int k, int n, int la, int lb, int64_t leaves) {
 // 128^3 64 limbs 1813 / 385, 256^3 8 limbs 575 / 163, 256^3 64 limbs 14002 / 2371,
 // 256 x 256 x 16 32 limbs 341 / 420 (16 columns use 16 of 128 lanes), 200 x 40 x 60 16 limbs 113 / 53.
 static int g_ltc_mode = -1;  // -1 by the estimate, 0 never, 1 wherever the shape allows it
-bool ltc_pays(int m, int k, int n, int la, int lb, int64_t leaves) {
-    if (m < 1 || k < 1 || n < 1 || la < 1 || lb < 1 || g_ltc_mode == 0) return false;
-    LtcArgs a;
-    ltc_shape(a, m, k, n, la, lb, leaves);
-    if (a.went >= ((int64_t)1 << 31) || a.nitems >= ((int64_t)1 << 31)) return false;
-    if (ltc_smem(a) > 227 * 1024) return false;
-    if (leaves * k * n >= ((int64_t)1 << 30)) return false;
-    if (g_ltc_mode == 1) return true;
+static bool ltc_allowed(const LtcArgs &a, int k, int n, int64_t leaves) {
+    return a.went < ((int64_t)1 << 31) && a.nitems < ((int64_t)1 << 31) && ltc_smem(a) <= 227 * 1024 &&
+           leaves * k * n < ((int64_t)1 << 30);
+}
+static double ltc_tensor_us(const LtcArgs &a, int k) {
     // 16-digit blocks a tile reads per k, averaged over the windows
     double nblk = 0;
     for (int w = 0; w < a.nW; w++) {
@@ -626,9 +623,55 @@ bool ltc_pays(int m, int k, int n, int la, int lb, int64_t leaves) {
     }
     nblk /= a.nW;
     const double waves = (double)((a.nitems + ltc_sms() - 1) / ltc_sms());
-    const double tensor = 30.0 + waves * k * (800.0 + 1.1 * nblk * a.W / 2) / 2070.0;
-    const double cores = 10.0 + (double)leaves * m * n * (k + 16.0) * la * lb / (limb_rate(la, lb, leaves * m * n) * 1e6);
-    return tensor < 0.95 * cores;
+    return 30.0 + waves * k * (800.0 + 1.1 * nblk * a.W / 2) / 2070.0;
+}
+static double ltc_cores_us(int m, int k, int n, int la, int lb, int64_t leaves) {
+    return 10.0 + (double)leaves * m * n * (k + 16.0) * la * lb / (limb_rate(la, lb, leaves * m * n) * 1e6);
+}
+bool ltc_pays(int m, int k, int n, int la, int lb, int64_t leaves) {
+    if (m < 1 || k < 1 || n < 1 || la < 1 || lb < 1 || g_ltc_mode == 0) return false;
+    LtcArgs a;
+    ltc_shape(a, m, k, n, la, lb, leaves);
+    if (!ltc_allowed(a, k, n, leaves)) return false;
+    if (g_ltc_mode == 1) return true;
+    return ltc_tensor_us(a, k) < 0.95 * ltc_cores_us(m, k, n, la, lb, leaves);
+}
+
+// Levels of a Winograd tree (1 .. levels, the depth that the cutoff gives) whose sums,
+// leaf products and combinations together are estimated fastest.  Each level has 7/8 of the
+// multiplications, but leaves of fewer than 128 columns leave lanes of the MMAs idle, and
+// the sums and combinations of a level take about 16 us plus their traffic; so on the
+// tensor cores the tree usually stops at blocks of 64 or more, on the CUDA cores at the
+// cutoff.  Products, us (levels, and before at the cutoff's depth): 64^3 16 limbs cutoff 16 98 (1; 151 at 2),
+// 128^3 32 limbs cutoff 32 389 (1; 623 at 2), 256^3 64 limbs cutoff 32 3001 (1; 8560 at 3),
+// 256^3 3 limbs cutoff 32 150 (1; 232 at 3), 512^3 32 limbs cutoff 32 10614 (2; 28664 at 4).
+int ltc_wino_levels(int N, int levels, int la, int lb) {
+    if (g_ltc_mode != -1) return levels;
+    double sums = 0, best = 1e30;
+    int pick = levels;
+    int64_t np = 1;
+    for (int d = 1; d <= levels; d++, np *= 7) {
+        const int hh = N >> d;
+        const double e = (double)hh * hh;
+        sums += 16.0 + np * e * 4.0 * 19.0 * (la + lb) / 4e6;
+        LtcArgs a;
+        ltc_shape(a, hh, hh, hh, la, lb, 7 * np);
+        double t = d == levels ? ltc_cores_us(hh, hh, hh, la, lb, 7 * np) : 1e30;
+        if (hh <= ltc_kmax(la, lb) && ltc_pays(hh, hh, hh, la, lb, 7 * np)) t = std::min(t, ltc_tensor_us(a, hh));
+        if (sums + t < best) {
+            best = sums + t;
+            pick = d;
+        }
+    }
+    return pick;
+}
+// Whether ltc_wino_leaves() would run in `room` bytes of workspace.
+static int64_t ltc_wino_chunk(int hh, int la, int lb, int64_t leaves, size_t room) {
+    const int64_t chunk = std::min<int64_t>(leaves, (int64_t)(room / (ltc_ws(hh, hh, hh, la, lb, 1) + 1)));
+    return chunk < 1 || (chunk < leaves && chunk < 64) ? 0 : chunk;
+}
+bool ltc_wino_fits(int hh, int la, int lb, int64_t leaves, size_t room) {
+    return ltc_wino_chunk(hh, la, lb, leaves, room) > 0;
 }
 
 gbmm_status make_map(CUtensorMap *m, const void *ptr, uint64_t inner, uint64_t outer, uint64_t pitch_elems,
@@ -719,8 +762,8 @@ gbmm_status ltc_wino_leaves(gbmm_handle h, const WinoTree &t, int64_t leaves, cu
     const int hh = t.N >> t.levels;
     if (hh > ltc_kmax(t.capSA, t.capSB)) return GBMM_OK;
     const size_t room = h->ws.cap - h->ws.top;
-    const int64_t chunk = std::min<int64_t>(leaves, (int64_t)(room / (ltc_ws(hh, hh, hh, t.capSA, t.capSB, 1) + 1)));
-    if (chunk < 1 || (chunk < leaves && chunk < 64)) return GBMM_OK;
+    const int64_t chunk = ltc_wino_chunk(hh, t.capSA, t.capSB, leaves, room);
+    if (chunk == 0) return GBMM_OK;
     const size_t mark = arena_mark(h);
     gbmm_status st = GBMM_OK;
     for (int64_t l0 = 0; l0 < leaves && st == GBMM_OK; l0 += chunk) {

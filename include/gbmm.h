@@ -98,7 +98,8 @@ typedef enum gbmm_plan {
 typedef struct gbmm_opts {
     int32_t path;        /* gbmm_path */
     int32_t method;      /* gbmm_method (limb path) */
-    int32_t cutoff;      /* recursion stops at blocks <= cutoff (0 = library default) */
+    int32_t cutoff;      /* recursion stops at blocks <= cutoff (0 = library default); Winograd's tree also
+                          * stops at larger blocks where their tensor-core products are faster */
     int32_t nprimes;     /* CRT: number of moduli (0 = derived from the bit bound) */
     int32_t accumulate;  /* nonzero: C += A*B (mat_addmul) instead of C = A*B */
     int32_t plan;        /* 0: path / method / cutoff as above; 1 + gbmm_plan: run that plan */
