@@ -1929,9 +1929,12 @@ __global__ void __launch_bounds__(NT, NT <= MM_THREADS ? 2 : 1)
 // thread per entry, each limb costs a dependent round trip to memory per addition:
 // the combinations of a two-level tree over 128 x 128 entries of 1024 bits took 233 us that
 // way and its sums 68 us, against 44 and 33 us.
-// (Up to 12 segments leave 168 registers a thread, up to 17 leave 112; entries longer than
-// 136 limbs take one thread per entry: with fewer registers the segments would spill.)
-constexpr int LIN_SHORT = 8, LIN_SHORT_SEGS = 12, LIN_LONG = 8, LIN_LONG_SEGS = 17;
+// Up to 12 segments leave 168 registers a thread; 17 leave 96, with spills.  Longer entries share a
+// block of that size among 16 or 8 entries instead of 32: one level's combinations of 128 x 128
+// entries of 4096 bits 39 us, 327 with one thread per entry (of 8192 bits, two halves of
+// 64 x 64: 44 and 1061).  Blocks of 12 segments without spills but of 16 or 8 entries are no
+// faster (256 x 256 of 2048 bits: 111 us, 74 with 17).  Past 544 limbs one thread takes an entry.
+constexpr int LIN_SEG = 8;
 struct LinIn {
     const uint32_t *p;
     int64_t ld;
@@ -1951,20 +1954,20 @@ __device__ __forceinline__ LinIn lin_in(const MatArgs &m, int64_t i, uint32_t *e
     }
     return x;
 }
-template <int MS>
+template <int MS, int EX>
 struct LinShared {
-    uint32_t first[4][MS][32];  // a segment's first limb
-    signed char carry[4][MS][32];  // its carry out, then its carry in
-    unsigned char rest[4][MS][32]; // bit 0: the other limbs all ones, bit 1: all zeros
-    unsigned char zero[4][MS][32]; // after the carries: the whole segment is zero
-    int top[4][32];
-    signed char fin[4][32];  // carry out of the last segment
+    uint32_t first[4][MS][EX];  // a segment's first limb
+    signed char carry[4][MS][EX];  // its carry out, then its carry in
+    unsigned char rest[4][MS][EX]; // bit 0: the other limbs all ones, bit 1: all zeros
+    unsigned char zero[4][MS][EX]; // after the carries: the whole segment is zero
+    int top[4][EX];
+    signed char fin[4][EX];  // carry out of the last segment
 };
 // Every thread of the block calls it (live: the entry exists).  Outputs o at
 // out[o].limbs[l * ld + io], cap planes each.
-template <class K, int SEG, int MS, int NI>
+template <class K, int SEG, int MS, int EX, int NI>
 __device__ __forceinline__ void lincomb4(const LinIn (&in)[NI], const MatArgs (&out)[4], int64_t io, bool live,
-                                         LinShared<MS> &sh, uint32_t *err) {
+                                         LinShared<MS, EX> &sh, uint32_t *err) {
     const int x = threadIdx.x, g = threadIdx.y, ng = blockDim.y, l0 = g * SEG, cap = out[0].nlimbs;
     uint32_t r[4][SEG];
     {
@@ -2082,15 +2085,15 @@ struct WinoCombine {
     }
 };
 
-// Level d's sums: 32 (operand side, parent, entry of the h x h quadrants) per block.
-template <int SEG, int MS>
-__global__ void __launch_bounds__(32 * MS) k_wino_sums(WinoTree t, int d, int64_t nparents, int h, uint32_t *err) {
-    __shared__ LinShared<MS> sh;
+// Level d's sums: EX (operand side, parent, entry of the h x h quadrants) per block.
+template <int SEG, int MS, int EX>
+__global__ void __launch_bounds__(EX * MS) k_wino_sums(WinoTree t, int d, int64_t nparents, int h, uint32_t *err) {
+    __shared__ LinShared<MS, EX> sh;
     const int64_t hh = (int64_t)h * h;
     // a block stays on one operand side: A's blocks first
-    const int64_t nb = (nparents * hh + 31) / 32;
+    const int64_t nb = (nparents * hh + EX - 1) / EX;
     const int which = blockIdx.x >= nb;
-    int64_t idx = ((int64_t)blockIdx.x - (which ? nb : 0)) * 32 + threadIdx.x;
+    int64_t idx = ((int64_t)blockIdx.x - (which ? nb : 0)) * EX + threadIdx.x;
     const bool live = idx < nparents * hh;
     if (!live) idx = 0;
     const int64_t e = idx % hh, p = idx / hh;
@@ -2103,8 +2106,8 @@ __global__ void __launch_bounds__(32 * MS) k_wino_sums(WinoTree t, int d, int64_
     const int cap = which ? t.capSB : t.capSA;
     const MatArgs o[4] = {wt_dense(L, S, 4 * p + 0, h, cap), wt_dense(L, S, 4 * p + 1, h, cap),
                           wt_dense(L, S, 4 * p + 2, h, cap), wt_dense(L, S, 4 * p + 3, h, cap)};
-    if (which) lincomb4<WinoSumB, SEG, MS>(in, o, e, live, sh, err);
-    else lincomb4<WinoSumA, SEG, MS>(in, o, e, live, sh, err);
+    if (which) lincomb4<WinoSumB, SEG, MS, EX>(in, o, e, live, sh, err);
+    else lincomb4<WinoSumA, SEG, MS, EX>(in, o, e, live, sh, err);
 }
 
 // The same sums for entries longer than the segments cover: one thread per (operand side, parent, entry of the h x h quadrants).
@@ -2151,13 +2154,13 @@ __global__ void __launch_bounds__(NT, NT <= MM_THREADS ? 2 : 1)
     limb_tile<R, THIN>(C, A, B, cfg, rem / nx, rem % nx, smem_raw, err);
 }
 
-// Level d's products combined into their parents' outputs (level d - 1): 32
+// Level d's products combined into their parents' outputs (level d - 1): EX
 // (parent, entry of the h x h quadrants) per block.
-template <int SEG, int MS>
-__global__ void __launch_bounds__(32 * MS) k_wino_combine(WinoTree t, int d, int64_t nparents, int h, uint32_t *err) {
-    __shared__ LinShared<MS> sh;
+template <int SEG, int MS, int EX>
+__global__ void __launch_bounds__(EX * MS) k_wino_combine(WinoTree t, int d, int64_t nparents, int h, uint32_t *err) {
+    __shared__ LinShared<MS, EX> sh;
     const int64_t hh = (int64_t)h * h;
-    int64_t idx = (int64_t)blockIdx.x * 32 + threadIdx.x;
+    int64_t idx = (int64_t)blockIdx.x * EX + threadIdx.x;
     const bool live = idx < nparents * hh;
     if (!live) idx = 0;
     const int64_t e = idx % hh, p = idx / hh;
@@ -2167,7 +2170,7 @@ __global__ void __launch_bounds__(32 * MS) k_wino_combine(WinoTree t, int d, int
 #pragma unroll
     for (int j = 0; j < 7; j++) in[j] = lin_in(wt_dense(t.p_limbs[d], t.p_sizes[d], 7 * p + j, h, t.capP), e, err);
     const MatArgs o[4] = {wt_quad(Cp, 0, 0, h), wt_quad(Cp, 0, 1, h), wt_quad(Cp, 1, 0, h), wt_quad(Cp, 1, 1, h)};
-    lincomb4<WinoCombine, SEG, MS>(in, o, ic, live, sh, err);
+    lincomb4<WinoCombine, SEG, MS, EX>(in, o, ic, live, sh, err);
 }
 
 // The same combinations for entries longer than the segments cover: one
@@ -2598,26 +2601,28 @@ static int64_t pow7(int d) {
     return r;
 }
 
-// segments of an entry of `cap` limbs: LAUNCH(SEG, MS) with ng segments, or 0
-#define LIN_DISPATCH(cap_, LAUNCH, SERIAL)                                                     \
-    do {                                                                                       \
-        if ((cap_) <= LIN_SHORT * LIN_SHORT_SEGS)                                              \
-            LAUNCH(LIN_SHORT, LIN_SHORT_SEGS, std::max(1, ((cap_) + LIN_SHORT - 1) / LIN_SHORT)); \
-        else if ((cap_) <= LIN_LONG * LIN_LONG_SEGS)                                           \
-            LAUNCH(LIN_LONG, LIN_LONG_SEGS, ((cap_) + LIN_LONG - 1) / LIN_LONG);               \
-        else SERIAL;                                                                           \
+// by the limbs of an entry: LAUNCH(segments, entries of a block)
+#define LIN_DISPATCH(cap_, LAUNCH, SERIAL)                  \
+    do {                                                    \
+        if ((cap_) <= LIN_SEG * 12) LAUNCH(12, 32);         \
+        else if ((cap_) <= LIN_SEG * 17) LAUNCH(17, 32);    \
+        else if ((cap_) <= LIN_SEG * 34) LAUNCH(34, 16);    \
+        else if ((cap_) <= LIN_SEG * 68) LAUNCH(68, 8);     \
+        else SERIAL;                                        \
     } while (0)
 
 gbmm_status launch_wino_sums(const WinoTree &t, int d, cudaStream_t s) {
     const int64_t np = pow7(d - 1);
     const int h = t.N >> d;
-    const int64_t n = np * h * h, blocks = 2 * ((n + 31) / 32);
+    const int64_t n = np * h * h, blocks = 2 * ((n + 7) / 8);  // at most
     uint32_t *err = device_error_word();
     LaunchScope ls_("k_wino_sums", s);
     // the sums' planes hold every limb of the quadrants they are formed from
     const int cap = std::max(t.capSA, t.capSB);
     if (blocks > 0x7FFFFFFF) return set_error(GBMM_ERR_UNSUPPORTED, "winograd sums: too many entries");
-#define LAUNCH_S(SEG, MS, ng) k_wino_sums<SEG, MS><<<(unsigned)blocks, dim3(32, (unsigned)(ng)), 0, s>>>(t, d, np, h, err)
+#define LAUNCH_S(MS, EX)                                                                                                       \
+    k_wino_sums<LIN_SEG, MS, EX><<<(unsigned)(2 * ((n + EX - 1) / EX)), dim3(EX, (unsigned)std::max(1, (cap + LIN_SEG - 1) / LIN_SEG)), 0, \
+                                   s>>>(t, d, np, h, err)
     LIN_DISPATCH(cap, LAUNCH_S, (k_wino_sums_serial<<<grid1(2 * n, 128), 128, 0, s>>>(t, d, np, h, err)));
 #undef LAUNCH_S
     GBMM_CUDA_TRY(cudaGetLastError());
@@ -2627,12 +2632,14 @@ gbmm_status launch_wino_sums(const WinoTree &t, int d, cudaStream_t s) {
 gbmm_status launch_wino_combine(const WinoTree &t, int d, cudaStream_t s) {
     const int64_t np = pow7(d - 1);
     const int h = t.N >> d;
-    const int64_t n = np * h * h, blocks = (n + 31) / 32;
+    const int64_t n = np * h * h, blocks = (n + 7) / 8;  // at most
     uint32_t *err = device_error_word();
     LaunchScope ls_("k_wino_combine", s);
     const int cap = std::max(t.capP, d == 1 ? t.C.nlimbs : 0);
     if (blocks > 0x7FFFFFFF) return set_error(GBMM_ERR_UNSUPPORTED, "winograd combinations: too many entries");
-#define LAUNCH_C(SEG, MS, ng) k_wino_combine<SEG, MS><<<(unsigned)blocks, dim3(32, (unsigned)(ng)), 0, s>>>(t, d, np, h, err)
+#define LAUNCH_C(MS, EX)                                                                                                     \
+    k_wino_combine<LIN_SEG, MS, EX><<<(unsigned)((n + EX - 1) / EX), dim3(EX, (unsigned)std::max(1, (cap + LIN_SEG - 1) / LIN_SEG)), 0, \
+                                      s>>>(t, d, np, h, err)
     LIN_DISPATCH(cap, LAUNCH_C, (k_wino_combine_serial<<<grid1(n, 128), 128, 0, s>>>(t, d, np, h, err)));
 #undef LAUNCH_C
     GBMM_CUDA_TRY(cudaGetLastError());

@@ -45,3 +45,20 @@ def test_fewer_levels(g, N, bits, cutoff, extra):
     assert got[0] == got[1]
     for y, x in [(0, 0), (0, N - 1), (N - 1, 0)] + [(rng.randrange(N), rng.randrange(N)) for _ in range(64)]:
         assert got[0][y * N + x] == sum(A[y * N + k] * B[k * N + x] for k in range(N))
+
+
+@pytest.mark.parametrize("limbs", [46, 47, 66, 67, 94, 95, 96, 134, 135, 136, 137, 270, 271, 272, 400])
+def test_sums_and_combinations_by_length(g, limbs):
+    """Sums and combinations with their limbs split among threads: blocks of 32, 16 and 8
+    entries at the edges of their ranges, carries and borrows through whole segments."""
+    N, bits = 6, 32 * limbs
+    rng = random.Random(limbs)
+    top = (1 << bits) - 1
+    kinds = [lambda: rng.getrandbits(bits), lambda: top, lambda: 1 << (32 * rng.randrange(limbs)), lambda: 0,
+             lambda: top - (1 << (32 * rng.randrange(limbs))), lambda: 1]
+    A = [rng.choice(kinds)() * rng.choice((-1, 1)) for _ in range(N * N)]
+    B = [rng.choice(kinds)() * rng.choice((-1, 1)) for _ in range(N * N)]
+    dA, dB = g.DeviceMatrix.from_ints(N, N, A, limbs), g.DeviceMatrix.from_ints(N, N, B, limbs)
+    dC = g.DeviceMatrix(N, N, 2 * limbs + 1)
+    g.default_handle().matmul(dC, dA, dB, path=g.PATH_LIMB, method=g.METHOD_WINOGRAD, cutoff=3)
+    assert dC.to_ints() == [sum(A[y * N + k] * B[k * N + x] for k in range(N)) for y in range(N) for x in range(N)]
