@@ -838,7 +838,7 @@ __device__ void addsub_entry(const MatArgs &W, int64_t iw, const MatArgs &U, int
 // written once.  All operand limbs are read before the first barrier and all of W's written
 // after it, so W may be U or V, shifted or not.  Bound by latency on few entries, where one
 // thread per entry has a carry chain through every load: 128 x 128 entries of 130 limbs
-// 27 -> 12.5 us, the halves of a 181 x 133 product of 595 limbs 194 -> 91 us.
+// 27 -> 12.5 us, the halves of a 181 x 133 product of 595 limbs 194 -> 65 us.
 // strict: an operand longer than W is refused outright (mpz semantics), else only a
 // result that does not fit.
 template <int MS>
@@ -849,8 +849,8 @@ struct Lin2Shared {
     int top[32];
     signed char fin[32];
 };
-template <int SEG, int MS>
-__global__ void __launch_bounds__(32 * MS) k_mpz_lin2(MatArgs W, MatArgs U, MatArgs V, int sh, int sub, int strict,
+template <int SEG, int MS, int NB>
+__global__ void __launch_bounds__(32 * MS, NB) k_mpz_lin2(MatArgs W, MatArgs U, MatArgs V, int sh, int sub, int strict,
                                                       int64_t count, uint32_t *err) {
     __shared__ Lin2Shared<MS> s;
     const int x = threadIdx.x, g = threadIdx.y, ng = blockDim.y, l0 = g * SEG;
@@ -2253,12 +2253,16 @@ static bool launch_lin2(const gbmm_mat &w, const gbmm_mat &u, const gbmm_mat &v,
     // (270 us four entries per thread), 571 us segmented.
     if (blocks > 0x7FFFFFFF || L > 1024 || n >= LIN2_MAX_ENTRIES) return false;
     uint32_t *err = device_error_word();
-#define LIN2(SEG, MS)                                                                                              \
-    k_mpz_lin2<SEG, MS><<<(unsigned)blocks, dim3(32, (unsigned)((L + SEG - 1) / SEG)), 0, s>>>(                   \
+// NB: blocks an SM holds by their registers.  Two, with a few spills, hide one's barriers behind the
+// other's loads (sums of 181 x 133 entries, us, one block and two: 400 limbs 66 and 56, 600 limbs
+// 98 and 74); past 640 limbs the spills cost as much.
+#define LIN2(SEG, MS, NB)                                                                                          \
+    k_mpz_lin2<SEG, MS, NB><<<(unsigned)blocks, dim3(32, (unsigned)((L + SEG - 1) / SEG)), 0, s>>>(               \
         margs(w), margs(u), margs(v), sh, sub, strict, n, err)
-    if (L <= 128) LIN2(8, 16);
-    else if (L <= 512) LIN2(16, 32);
-    else LIN2(32, 32);
+    if (L <= 128) LIN2(8, 16, 1);
+    else if (L <= 512) LIN2(16, 32, 2);
+    else if (L <= 640) LIN2(32, 20, 2);
+    else LIN2(32, 32, 1);
 #undef LIN2
     return true;
 }
