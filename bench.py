@@ -408,7 +408,7 @@ def run_gpu(args, W, world, rank, local):
     roof = kernel_roofline(kname, klaunch, kms, W, args, K, M, N, nl, cn, peaks, prof, macpk)
     limb = None
     if path == gbmm.PATH_CRT and not args.no_limb:
-        limb = measure_limb_path(gbmm, h, dA, dB, dC, K, M, N, nl, args, flush, stream)
+        limb = measure_limb_path(gbmm, h, dA, dB, dC, K, M, N, nl, args, flush, stream, peaks)
 
     if rank != 0:
         return 0
@@ -462,17 +462,17 @@ def crt_params(bits_a, bits_b, k):
         mod *= pr[P]
         P += 1
     modbits = 32 * ((mod.bit_length() + 31) // 32)
-    return P, (modbits + 6) // 7 + 2  # base-128 output digits
+    # output digits, base 256 (base 128 past 940 moduli)
+    return P, ((modbits + 7) // 8 if P <= 940 else (modbits + 6) // 7) + 2
 
 
 # DRAM bytes (read + write) per launch of each CRT GEMM on 512x512x512 at 4096 bits,
 # from a one-pass ncu capture of this workload (dram__bytes_read.sum +
-# dram__bytes_write.sum; profiles/crt_512x512x512_4096b_dram_bytes.md).  The residue
-# figure is the mean of its two launches (A, then B).
+# dram__bytes_write.sum; profiles/crt_512x512x512_4096b_dram_bytes.md).
 NCU_DRAM_BYTES_512_4096 = {
-    "k_crt_residue": (269.558528e6 + 487.749376e6 + 269.553408e6 + 487.559680e6) / 2,
-    "k_crt_product": 1083.140608e6 + 506.246400e6,
-    "k_crt_recon": 583.059200e6 + 241.474048e6,
+    "k_crt_residue": 274.133248e6 + 1026.769664e6,
+    "k_crt_product": 1082.190080e6 + 511.279104e6,
+    "k_crt_recon": 558.553344e6 + 242.209024e6,
 }
 FIXED_POINT_COLUMNS = 14  # reconstruction columns that carry the 2^96 / p_i weights
 
@@ -493,11 +493,18 @@ def kernel_roofline(kname, klaunch, kms, W, args, K, M, N, nl, cn, peaks, prof, 
         flops = 2.0 * K * M * N * 4 * P
         note = f"4 digit-pair GEMMs per modulus, P={P} moduli, {K}x{M}x{N}"
     elif kname == "k_crt_residue":
-        flops = 2.0 * (K * M + M * N) / 2 * dx * 2 * P  # one launch per operand (square: equal halves)
-        note = f"entries x {dx} digits x {2 * P} table columns per operand"
+        per_product = klaunch / max(1, prof.get("k_crt_product", (klaunch, 0.0))[0])  # both operands, or one each
+        flops = 2.0 * (K * M + M * N) / max(1.0, per_product) * dx * 2 * P
+        note = f"entries x {dx} digits x {2 * P} table columns, both operands over {per_product:.0f} launch(es)"
     elif kname == "k_crt_recon":
         flops = 2.0 * K * N * 2 * P * (FIXED_POINT_COLUMNS + Dout)
         note = f"entries x {2 * P} moduli digits x {FIXED_POINT_COLUMNS + Dout} output columns"
+    elif kname == "k_ltc_gemm":
+        steps = max(1, args.profile_steps)
+        levels = prof.get("k_wino_sums", (0, 0.0))[0] // steps
+        macs = winograd_leaf_macs(K, levels, nl, nl) if levels else K * M * N * nl * nl
+        flops = 32.0 * macs * steps / max(1, klaunch)
+        note = "16 byte-digit MACs per 32-bit limb MAC of the products, no padding counted"
     if flops is not None:
         ach = flops / (per_ms * 1e-3) / 1e12
         traffic = None
@@ -570,7 +577,7 @@ def winograd_leaf_macs(N, levels, la, lb):
     return macs * h ** 3
 
 
-def measure_limb_path(gbmm, h, dA, dB, dC_crt, K, M, N, nl, args, flush, stream):
+def measure_limb_path(gbmm, h, dA, dB, dC_crt, K, M, N, nl, args, flush, stream, peaks):
     """The plain limb form on the same inputs (the >= 10x comparison of the CRT form is
     against it): the per-entry kernel alone and Winograd's breadth-first tree down to
     --limb-cutoff, each timed over --limb-steps steps; the faster is the comparison
@@ -611,25 +618,26 @@ def measure_limb_path(gbmm, h, dA, dB, dC_crt, K, M, N, nl, args, flush, stream)
         prof = gbmm.profile_read()
         gbmm.profile(False)
         del dL
-        levels = 0
-        if method == gbmm.METHOD_WINOGRAD and K == M == N and K > cutoff:
-            # the recursion depth the library uses: floor(log2(N / cutoff)), lowered until 2^levels divides N
-            levels = (K // cutoff).bit_length() - 1
-            while levels > 0 and K % (1 << levels):
-                levels -= 1
-        lk = "k_wino_leaves" if "k_wino_leaves" in prof else "k_limb_matmul"
-        lms = prof.get(lk, (1, 0.0))[1]
-        macs = winograd_leaf_macs(K, levels, nl, nl) if lk == "k_wino_leaves" else K * M * N * nl * nl
-        ach = macs / (lms * 1e-3)
+        # the recursion depth the library chose: one launch of the sums per level
+        levels = prof.get("k_wino_sums", (0, 0.0))[0] if method == gbmm.METHOD_WINOGRAD else 0
+        lk = next(k for k in ("k_ltc_gemm", "k_wino_leaves", "k_limb_matmul") if k in prof)
+        lms = prof[lk][1]
+        macs = winograd_leaf_macs(K, levels, nl, nl) if levels else K * M * N * nl * nl
+        if lk == "k_ltc_gemm":
+            # on the tensor cores: 16 byte-digit MACs of 2 FLOPs per 32-bit limb MAC
+            ach, pk, bound, unit = 32 * macs / (lms * 1e-3) / 1e12, peaks.get("bf16_tflops", 1900.0), "tensor", "TFLOP/s"
+            note = "byte-digit FLOPs of the products (no padding) / the kernel's time; peak: bf16 dense, burst"
+        else:
+            ach, pk, bound, unit = macs / (lms * 1e-3), peak, "int-mul", "MAC/s"
+            note = ("32x32-bit limb MACs of the kernel's products / its time; peak: measured rate "
+                    "of the same 96-bit column MAC step on register operands (k_mac_peak)")
         forms[form] = {
             "ms_per_step": statistics.median(times), "steps": args.limb_steps,
             "cutoff": cutoff if method == gbmm.METHOD_WINOGRAD else None, "levels": levels,
             "launches_per_step": int(launches), "equals_crt_result": same,
             "kernels": {k: {"launches": v[0], "ms_total": round(v[1], 3)} for k, v in sorted(prof.items())},
-            "roofline": {"kernel": lk, "bound": "int-mul", "achieved": ach, "peak": peak, "unit": "MAC/s",
-                         "frac": ach / peak,
-                         "note": "32x32-bit limb MACs of the kernel's products / its time; peak: measured rate "
-                                 "of the same 96-bit column MAC step on register operands (k_mac_peak)"}}
+            "roofline": {"kernel": lk, "bound": bound, "achieved": ach, "peak": pk, "unit": unit, "frac": ach / pk,
+                         "note": note}}
     best = min(forms, key=lambda f: forms[f]["ms_per_step"])
     return {"ms_per_step": forms[best]["ms_per_step"], "form": best, "forms": forms,
             "roofline": forms[best]["roofline"]}
@@ -904,9 +912,9 @@ def run_limb_kernels(args, W, world, rank, local):
         out[name] = r
 
     L4 = 4 * n * nb                           # bytes of one operand batch
-    rec("mpn_add_n", "k_mpn_addsub_n_serial", timed(lambda: gbmm.mpn_add_n(rp, up, vp, n, nb, nb, cy)),
+    rec("mpn_add_n", "k_mpn_addsub_n_vec", timed(lambda: gbmm.mpn_add_n(rp, up, vp, n, nb, nb, cy)),
         3 * L4 + 4 * nb)
-    rec("mpn_sub_n", "k_mpn_addsub_n_serial", timed(lambda: gbmm.mpn_sub_n(rp, up, vp, n, nb, nb, cy)),
+    rec("mpn_sub_n", "k_mpn_addsub_n_vec", timed(lambda: gbmm.mpn_sub_n(rp, up, vp, n, nb, nb, cy)),
         3 * L4 + 4 * nb)
     rec("mpn_mul_1", "k_mpn_mul1ops", timed(lambda: gbmm.mpn_mul_1(rp, up, n, vl, nb, nb, cy)),
         2 * L4 + 8 * nb, n * nb)
