@@ -15,6 +15,8 @@
 //                 applies the entry's sign and stores the residue as two
 //                 balanced digits in per-modulus planes.  B's table carries the
 //                 CRT weight w_i = (Mod/p_i)^-1 mod p_i.
+//                 Rows of up to 512 digits take both steps in one kernel, for both
+//                 operands at once (2b below).
 //  3. product   : for each modulus, A's two digit planes against B's two
 //                 (pre-weighted) digit planes in four accumulators;
 //                 y_i = 65536 a1 u1 + 256 (a1 u0 + a0 u1) + a0 u0 mod p_i, stored

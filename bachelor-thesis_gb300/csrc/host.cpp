@@ -1503,7 +1503,7 @@ gbmm_status crt_collect(gbmm_handle h, crt_group *g, const gbmm_mat &c, const gb
         return set_error(GBMM_ERR_UNSUPPORTED, "crt group: no single-pass form for %d x %d limb entries", a.nlimbs,
                          b.nlimbs);
     // as dispatch(): one product T against the halves stacked (read in place by the
-    // digits stage), then C = T_0 + T_1 2^(32 hl); T stays carved until the group has run
+    // digit and residue stages), then C = T_0 + T_1 2^(32 hl); T stays carved until the group has run
     const bool sa = a.nlimbs >= b.nlimbs;
     const gbmm_mat &X = sa ? a : b;
     gbmm_mat S, T;
