@@ -2331,9 +2331,11 @@ gbmm_status launch_max_size(const gbmm_mat &a, int32_t *d_out, cudaStream_t s) {
 gbmm_status launch_mpz_mulops(const gbmm_mat &w, const gbmm_mat &u, const gbmm_mat &v, int op, cudaStream_t s) {
     const int64_t n = nentries(w);
     if (n == 0) return GBMM_OK;
-    // staged on chip wherever 32 or more entries' operands fit in shared memory
+    // staged on chip wherever 32 or more entries' operands fit in shared memory, but for the
+    // shortest products, whose limbs are read once anyway (10^6 addmul, us, staged and not: 1 x 1
+    // limbs 35 and 22, 2 x 2 36 and 31, 2 x 4 39 and 39, 4 x 4 47 and 51, 16 x 16 127 and 337)
     const size_t words = (size_t)sm_stride(u.nlimbs) + sm_stride(v.nlimbs) + 2;
-    const int nt = u.nlimbs > 0 && v.nlimbs > 0 ? sm_threads(words) : 0;
+    const int nt = (int64_t)u.nlimbs * v.nlimbs > 8 ? sm_threads(words) : 0;
     LaunchScope ls_("k_mpz_mulops", s);
     if (nt) {
         const size_t smem = nt * words * 4;

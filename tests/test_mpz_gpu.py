@@ -21,7 +21,7 @@ def _vals(rng, n, limbs):
             for _ in range(n)]
 
 
-@pytest.mark.parametrize("ul,vl,rows,cols", [(1, 1, 1, 1), (3, 5, 7, 19), (4, 4, 16, 16), (16, 16, 5, 129),
+@pytest.mark.parametrize("ul,vl,rows,cols", [(1, 1, 1, 1), (2, 4, 9, 31), (1, 9, 5, 33), (3, 3, 4, 40), (3, 5, 7, 19), (4, 4, 16, 16), (16, 16, 5, 129),
                                              (17, 2, 9, 67), (40, 33, 3, 50), (700, 3, 2, 33), (1200, 1200, 1, 3)])
 @pytest.mark.parametrize("op", ["mul", "addmul", "submul"])
 @pytest.mark.parametrize("view", [False, True])
