@@ -2438,6 +2438,21 @@ static void finish_cfg(MMCfg &cfg, int M, int accumulate) {
     cfg.accumulate = accumulate;
 }
 
+// The same for a product of so many entries: operands of 3 to 8 limbs otherwise take one thread
+// per entry, which leaves most of the GPU idle on few entries; blocks of 2 x 2 limbs put 4 to 16
+// threads on each.  One thread and blocks of 2, us: 16 x 64 x 16 entries of 4 limbs 37 and 17, of
+// 8 limbs 86 and 17; 64 x 64 x 64 of 4 limbs 38 and 37, of 8 limbs 87 and 38; 100 x 64 x 100 of
+// 4 limbs 38 and 66, of 5 limbs 87 and 114, of 8 limbs 87 and 69.
+constexpr int64_t MM_FEW_ENTRIES = 4096;
+static bool choose_mm_for(int la, int lb, int64_t entries, MMCfg &cfg) {
+    if (!choose_mm(la, lb, cfg)) return false;
+    MMCfg few;
+    if (cfg.G == 1 && std::max(la, lb) > 2 && la > 0 && lb > 0 && entries <= MM_FEW_ENTRIES &&
+        try_block(la, lb, 2, 2, MM_THREADS, few))
+        cfg = few;
+    return true;
+}
+
 bool limb_kernel_fits(int la, int lb) {
     MMCfg cfg;
     return choose_mm(la, lb, cfg);
@@ -2445,7 +2460,7 @@ bool limb_kernel_fits(int la, int lb) {
 
 double limb_rate(int la, int lb, int64_t entries) {
     MMCfg cfg;
-    if (!choose_mm(la, lb, cfg)) return 1.0;
+    if (!choose_mm_for(la, lb, entries, cfg)) return 1.0;
     // one thread per entry: it takes about 40 thousand entries to fill the GPU
     if (cfg.G == 1) return 1.9 * std::min(1.0, entries / 41000.0);
     const bool thin = cfg.thinA || cfg.thinB;
@@ -2470,7 +2485,7 @@ gbmm_status launch_limb_matmul(const gbmm_mat &c, const gbmm_mat &a, const gbmm_
         return launch_mat_zero(c, s);
     }
     MMCfg cfg;
-    if (!choose_mm(a.nlimbs, b.nlimbs, cfg))
+    if (!choose_mm_for(a.nlimbs, b.nlimbs, (int64_t)c.rows * c.cols, cfg))
         return set_error(GBMM_ERR_UNSUPPORTED, "limb matmul: %d x %d limb entries exceed the per-entry kernel", a.nlimbs,
                          b.nlimbs);
     finish_cfg(cfg, a.cols, accumulate);
@@ -2655,7 +2670,7 @@ gbmm_status launch_wino_combine(const WinoTree &t, int d, cudaStream_t s) {
 gbmm_status launch_wino_leaves(const WinoTree &t, cudaStream_t s) {
     const int h = t.N >> t.levels;
     MMCfg cfg;
-    if (!choose_mm(t.capSA, t.capSB, cfg))
+    if (!choose_mm_for(t.capSA, t.capSB, pow7(t.levels) * h * h, cfg))
         return set_error(GBMM_ERR_UNSUPPORTED, "winograd leaves: %d x %d limb operands exceed the per-entry kernel",
                          t.capSA, t.capSB);
     finish_cfg(cfg, h, 0);
