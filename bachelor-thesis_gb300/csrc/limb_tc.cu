@@ -530,8 +530,10 @@ __global__ void __launch_bounds__(256)
     a.out = out + leaf * v.rows * v.cols * (int64_t)dx;
     digits_block<true>(a, b % nbx, b / nbx, blockIdx.y);
 }
-__global__ void __launch_bounds__(256) k_ltc_digits(DigitArgs a) {
-    digits_block<true>(a, blockIdx.x, blockIdx.y, blockIdx.z);
+// One operand's digit rows; blockIdx.x = tile of 4 rows x 32 columns (rows alone pass a
+// grid's 65535 blocks in y from 262141 on).
+__global__ void __launch_bounds__(256) k_ltc_digits(DigitArgs a, int nbx) {
+    digits_block<true>(a, blockIdx.x % nbx, blockIdx.x / nbx, blockIdx.y);
 }
 
 // ---- host side ----------------------------------------------------------------------------
@@ -740,9 +742,10 @@ gbmm_status ltc_matmul(gbmm_handle h, const gbmm_mat &c, const gbmm_mat &a, cons
             d.transpose = 0;
             d.dxp = side ? q.dxb : q.dxa;
             d.out = side ? w.db : w.da;
-            const dim3 grid((unsigned)((x.cols + 31) / 32), (unsigned)((x.rows + 3) / 4), (unsigned)((d.dxp / 4 + 63) / 64));
+            const int nbx = (x.cols + 31) / 32;
+            const dim3 grid((unsigned)(nbx * ((x.rows + 3) / 4)), (unsigned)((d.dxp / 4 + 63) / 64));
             LaunchScope ls_("k_ltc_digits", s);
-            k_ltc_digits<<<grid, 256, 0, s>>>(d);
+            k_ltc_digits<<<grid, 256, 0, s>>>(d, nbx);
             if (cudaError_t e = cudaGetLastError(); e != cudaSuccess) st = cuda_error(e, "k_ltc_digits");
         }
         LtcOut o;
