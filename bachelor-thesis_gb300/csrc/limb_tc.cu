@@ -18,7 +18,10 @@
 //
 // After the last K step a tile turns its columns into limbs from carry 0 (two's
 // complement, carry out kept per segment); k_ltc_finish resolves the carries between
-// segments, adds the old C for C += A B, and writes sign and magnitude.
+// segments, adds the old C for C += A B, and writes sign and magnitude.  A longer inner
+// dimension runs in chunks: a later chunk's tiles add the earlier ones' limbs and carries
+// to theirs, and C, whose planes only the exact result has to fit, is read and written
+// once at the end.
 //
 // Replaces the launcher_mul / launcher_addmul kernels (mat-gpu/mat-core.h:7-137)
 // wherever ltc_pays() says so; the CUDA-core kernel (limb.cu) takes the rest.
@@ -61,7 +64,9 @@ struct LtcArgs {
     int32_t nxt;       // tiles of 128 columns x
     int64_t nitems;
     uint32_t *wl;      // [T / 4][entries] limbs, two's complement per segment
-    int32_t *wq;       // [T / seg][entries] carry out of each segment
+    void *wq;          // [T / seg][entries] carry out of each segment: int32_t, int64_t with `chunks`
+    int32_t chunks;    // one of several chunks of the inner dimension
+    int32_t later;     // ... and not the first
     int64_t went;      // entries = leaves m n
     int32_t esize, rsize;  // bytes of a Hankel ring entry and of a builder's digit row buffer
 };
@@ -124,6 +129,8 @@ __device__ __forceinline__ uint64_t sdesc_hankel(uint32_t saddr) {
 // reach halves the multiplications, but every change of the column range drains the
 // pipe (measured at 256^3, 2048 bits: 4.5 ms with exact ranges, 3.7 ms with one range
 // per K step, 2.8 ms without, before the operands had rings of their own).
+// CHUNKS: a.chunks, kept out of the common launches' epilogue.
+template <bool CHUNKS>
 __global__ void __launch_bounds__(LT_THREADS, 1)
     k_ltc_gemm(const __grid_constant__ CUtensorMap tmP, LtcArgs a, uint32_t *err) {
     extern __shared__ uint8_t smem_raw[];
@@ -389,8 +396,9 @@ __global__ void __launch_bounds__(LT_THREADS, 1)
                 if (4 * g >= hc) continue;
                 // one group at a time: the columns leave no registers for groups formed ahead
                 asm volatile("" : "+r"(acc[4 * g]), "+r"(acc[4 * g + 1]), "+r"(acc[4 * g + 2]), "+r"(acc[4 * g + 3]));
-                const long long v = (long long)acc[4 * g + 3] + (long long)acc[4 * g + 2] * 256 +
-                                    (long long)acc[4 * g + 1] * 65536 + (long long)acc[4 * g] * 16777216 + cy;
+                long long v = (long long)acc[4 * g + 3] + (long long)acc[4 * g + 2] * 256 +
+                              (long long)acc[4 * g + 1] * 65536 + (long long)acc[4 * g] * 16777216 + cy;
+                if (CHUNKS && a.later && live) v += *wp;
                 if (live) *wp = (uint32_t)v;
                 cy = v >> 32;
                 tcol += 4;
@@ -398,7 +406,13 @@ __global__ void __launch_bounds__(LT_THREADS, 1)
                 wp += a.went;
                 if (sleft == 0) {
                     // tcol is one past the segment's last column
-                    if (live) a.wq[(int64_t)(tcol / a.seg - 1) * a.went + ent] = (int32_t)cy;
+                    const int64_t qi = (int64_t)(tcol / a.seg - 1) * a.went + ent;
+                    if (CHUNKS) {
+                        long long *wq = static_cast<long long *>(a.wq) + qi;
+                        if (live) *wq = cy + (a.later ? *wq : 0ll);
+                    } else if (live) {
+                        static_cast<int32_t *>(a.wq)[qi] = (int32_t)cy;
+                    }
                     cy = 0;
                     sleft = a.seg;
                     if (a.nY > 1) {
@@ -470,7 +484,10 @@ __global__ void __launch_bounds__(128) k_ltc_finish(LtcArgs a, LtcOut o, uint32_
                 u[i] = l0 + i < cn ? C.limbs[(int64_t)(l0 + i) * C.ld + ic] : 0u;
             }
             // the carry out of segment s enters segment s + 1 (also past the last one)
-            if (l0 > 0 && l0 <= TL && l0 % SL == 0) c += a.wq[(int64_t)(l0 / SL - 1) * a.went + e];
+            if (l0 > 0 && l0 <= TL && l0 % SL == 0) {
+                const int64_t qi = (int64_t)(l0 / SL - 1) * a.went + e;
+                c += a.chunks ? static_cast<const long long *>(a.wq)[qi] : static_cast<const int32_t *>(a.wq)[qi];
+            }
 #pragma unroll
             for (int i = 0; i < 4; i++) {
                 const long long v = (long long)w[i] + c + (sc < 0 ? -(long long)u[i] : (long long)u[i]);
@@ -596,7 +613,7 @@ size_t ltc_ws(int m, int k, int n, int la, int lb, int64_t leaves) {
     const int kc = std::min(k, ltc_kmax(la, lb));
     ltc_shape(a, m, kc, n, la, lb, leaves);
     return ltc_align((size_t)leaves * m * kc * a.dxa * 2) + ltc_align((size_t)leaves * kc * n * a.dxb * 2) +
-           ltc_align((size_t)(a.T / 4) * a.went * 4) + ltc_align((size_t)(a.T / a.seg) * a.went * 4) + 2048;
+           ltc_align((size_t)(a.T / 4) * a.went * 4) + ltc_align((size_t)(a.T / a.seg) * a.went * (k > kc ? 8 : 4)) + 2048;
 }
 
 // Estimated time of both forms in microseconds; the tensor form is taken when it is
@@ -687,20 +704,22 @@ static bool ltc_carve(gbmm_handle h, LtcArgs &a, LtcBufs &w, int64_t leaves) {
     w.da = (__nv_bfloat16 *)arena_alloc(h, (size_t)leaves * a.m * a.k * a.dxa * 2);
     w.db = (__nv_bfloat16 *)arena_alloc(h, (size_t)leaves * a.k * a.n * a.dxb * 2);
     a.wl = (uint32_t *)arena_alloc(h, (size_t)(a.T / 4) * a.went * 4);
-    a.wq = (int32_t *)arena_alloc(h, (size_t)(a.T / a.seg) * a.went * 4);
+    a.wq = arena_alloc(h, (size_t)(a.T / a.seg) * a.went * (a.chunks ? 8 : 4));
     a.ad = w.da;
     return w.da && w.db && a.wl && a.wq;
 }
-static gbmm_status ltc_gemm(const LtcArgs &a, const LtcBufs &w, int64_t leaves, const LtcOut &o, cudaStream_t s) {
+static gbmm_status ltc_gemm(const LtcArgs &a, const LtcBufs &w, int64_t leaves, cudaStream_t s) {
     CUtensorMap tmP;
     GBMM_TRY(make_map(&tmP, w.db, a.dxb, (uint64_t)leaves * a.k * a.n, a.dxb, 64, (uint32_t)a.prow));
     const size_t smem = ltc_smem(a);
-    GBMM_CUDA_TRY(cudaFuncSetAttribute(k_ltc_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    {
-        LaunchScope ls_("k_ltc_gemm", s);
-        k_ltc_gemm<<<(unsigned)std::min<int64_t>(a.nitems, ltc_sms()), LT_THREADS, smem, s>>>(tmP, a, device_error_word());
-        GBMM_CUDA_TRY(cudaGetLastError());
-    }
+    auto kern = a.chunks ? k_ltc_gemm<true> : k_ltc_gemm<false>;
+    GBMM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    LaunchScope ls_("k_ltc_gemm", s);
+    kern<<<(unsigned)std::min<int64_t>(a.nitems, ltc_sms()), LT_THREADS, smem, s>>>(tmP, a, device_error_word());
+    GBMM_CUDA_TRY(cudaGetLastError());
+    return GBMM_OK;
+}
+static gbmm_status ltc_finish(const LtcArgs &a, const LtcOut &o, cudaStream_t s) {
     LaunchScope ls_("k_ltc_finish", s);
     k_ltc_finish<<<(unsigned)((a.went + 127) / 128), 128, 0, s>>>(a, o, device_error_word());
     GBMM_CUDA_TRY(cudaGetLastError());
@@ -717,6 +736,7 @@ gbmm_status ltc_matmul(gbmm_handle h, const gbmm_mat &c, const gbmm_mat &a, cons
     const size_t mark = arena_mark(h);
     LtcArgs full;
     ltc_shape(full, a.rows, kc, b.cols, a.nlimbs, b.nlimbs, 1);
+    full.chunks = K > kc;
     LtcBufs w;
     if (!ltc_carve(h, full, w, 1)) {
         arena_release(h, mark);
@@ -728,6 +748,7 @@ gbmm_status ltc_matmul(gbmm_handle h, const gbmm_mat &c, const gbmm_mat &a, cons
         const int kn = std::min(kc, K - k0);
         LtcArgs q = full;
         q.k = kn;
+        q.later = k0 > 0;
         const gbmm_mat ac = sub_view(a, 0, k0, a.rows, kn), bc = sub_view(b, k0, 0, kn, b.cols);
         for (int side = 0; side < 2; side++) {
             const gbmm_mat &x = side ? bc : ac;
@@ -748,12 +769,13 @@ gbmm_status ltc_matmul(gbmm_handle h, const gbmm_mat &c, const gbmm_mat &a, cons
             k_ltc_digits<<<grid, 256, 0, s>>>(d, nbx);
             if (cudaError_t e = cudaGetLastError(); e != cudaSuccess) st = cuda_error(e, "k_ltc_digits");
         }
-        LtcOut o;
-        memset(&o, 0, sizeof o);
-        o.C = c;
-        o.accumulate = accumulate || k0 > 0;
-        if (st == GBMM_OK) st = ltc_gemm(q, w, 1, o, s);
+        if (st == GBMM_OK) st = ltc_gemm(q, w, 1, s);
     }
+    LtcOut o;
+    memset(&o, 0, sizeof o);
+    o.C = c;
+    o.accumulate = accumulate;
+    if (st == GBMM_OK) st = ltc_finish(full, o, s);
     arena_release(h, mark);
     return st;
 }
@@ -792,7 +814,8 @@ gbmm_status ltc_wino_leaves(gbmm_handle h, const WinoTree &t, int64_t leaves, cu
         o.pl = t.p_limbs[t.levels] + l0 * (int64_t)hh * hh * t.capP;
         o.ps = t.p_sizes[t.levels] + l0 * (int64_t)hh * hh;
         o.pcap = t.capP;
-        if (st == GBMM_OK) st = ltc_gemm(q, w, nl, o, s);
+        if (st == GBMM_OK) st = ltc_gemm(q, w, nl, s);
+        if (st == GBMM_OK) st = ltc_finish(q, o, s);
         arena_release(h, mark);
     }
     return st;
