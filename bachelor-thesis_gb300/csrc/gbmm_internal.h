@@ -238,7 +238,7 @@ gbmm_status crt_collect(gbmm_handle h, crt_group *g, const gbmm_mat &c, const gb
                         const Plan &p);
 // extra workspace with which dispatch() runs its limb products on the tensor cores
 size_t limb_tc_extra(const Plan &p, int la, int lb, int m, int k, int n);
-// Reserves `ws` bytes, with `extra` more when they can be had; *got says whether
+// Reserves `ws` bytes, with `extra` more when they can be had without giving anything up; *got says whether
 gbmm_status arena_reserve_extra(gbmm_handle h, size_t ws, size_t extra, bool *got);
 gbmm_status resolve_plan(gbmm_handle h, const gbmm_mat &a, const gbmm_mat &b, const gbmm_opts &o, Plan &p);
 void invalidate_graphs(gbmm_handle h);
@@ -255,6 +255,7 @@ struct arena {
     char *base = nullptr;
     size_t cap = 0;
     size_t top = 0;
+    size_t plain = 0;  // the part of it that calls needed; the rest was optional (arena_reserve_extra)
 };
 
 }  // namespace gbmm

@@ -146,21 +146,75 @@ gbmm_status validate_mat(const gbmm_mat &m, const char *name) {
 }
 
 // ---- arena ------------------------------------------------------------------------------
-gbmm_status arena_reserve(gbmm_handle h, size_t bytes) {
-    if (h->ws.top + bytes <= h->ws.cap) return GBMM_OK;
-    if (h->ws.top != 0) return set_error(GBMM_ERR_INVALID, "workspace grow while in use");
-    size_t want = std::max(bytes, h->ws.cap * 2);
-    want = (want + 0xFFFFF) & ~(size_t)0xFFFFF;
+static size_t round_mib(size_t bytes) { return (bytes + 0xFFFFF) & ~(size_t)0xFFFFF; }
+
+// Ends the current block: work in it has run, captured graphs that point into it go.
+static gbmm_status arena_drop(gbmm_handle h) {
     GBMM_CUDA_TRY(cudaStreamSynchronize(h->stream));
-    invalidate_graphs(h);  // captured graphs point into the old block
+    invalidate_graphs(h);
     if (h->ws.base) GBMM_CUDA_TRY(cudaFree(h->ws.base));
     h->ws.base = nullptr;
     h->ws.cap = 0;
+    return GBMM_OK;
+}
+
+gbmm_status arena_reserve(gbmm_handle h, size_t bytes) {
+    if (h->ws.top + bytes <= h->ws.cap) {
+        h->ws.plain = std::max(h->ws.plain, h->ws.top + bytes);
+        return GBMM_OK;
+    }
+    if (h->ws.top != 0) return set_error(GBMM_ERR_INVALID, "workspace grow while in use");
+    // twice what calls needed so far (an optional part is not doubled)
+    const size_t want = round_mib(std::max(bytes, h->ws.plain * 2));
+    GBMM_TRY(arena_drop(h));
     void *p = nullptr;
     GBMM_CUDA_TRY(cudaMalloc(&p, want));
     h->ws.base = (char *)p;
     h->ws.cap = want;
+    h->ws.plain = want;
     return GBMM_OK;
+}
+
+// Bytes an optional workspace may take: half of what the device has free (a test may
+// set another figure for its thread).
+static thread_local int64_t t_extra_room = -1;
+static size_t extra_room() {
+    if (t_extra_room >= 0) return (size_t)t_extra_room;
+    size_t fr = 0, tot = 0;
+    if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return fr / 2;
+}
+
+// The extra part is had when the block holds it or can grow to it: the new block is
+// allocated beside the old one, so that a refusal costs neither the old block nor the graphs
+// captured in it, and never while the stream is being captured.
+gbmm_status arena_reserve_extra(gbmm_handle h, size_t ws, size_t extra, bool *got) {
+    *got = false;
+    if (extra && h->ws.top + ws + extra <= h->ws.cap) {
+        *got = true;
+    } else if (extra && h->ws.top == 0) {
+        const size_t plain = ws > h->ws.cap ? std::max(ws, h->ws.plain * 2) : ws, want = round_mib(plain + extra);
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        void *p = nullptr;
+        if (cudaStreamIsCapturing(h->stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone &&
+            want <= extra_room() && cudaMalloc(&p, want) == cudaSuccess) {
+            const gbmm_status st = arena_drop(h);
+            if (st != GBMM_OK) {
+                cudaFree(p);
+                return st;
+            }
+            h->ws.base = (char *)p;
+            h->ws.cap = want;
+            h->ws.plain = std::max(h->ws.plain, plain);
+            *got = true;
+        } else {
+            cudaGetLastError();  // refused: run without the extra part
+        }
+    }
+    return arena_reserve(h, ws);
 }
 
 void *arena_alloc(gbmm_handle h, size_t bytes) {
@@ -1349,18 +1403,6 @@ size_t limb_tc_extra(const Plan &p, int la, int lb, int m, int k, int n) {
     return x <= MAX_BYTES ? x : 0;
 }
 
-gbmm_status arena_reserve_extra(gbmm_handle h, size_t ws, size_t extra, bool *got) {
-    *got = false;
-    if (extra) {
-        if (arena_reserve(h, ws + extra) == GBMM_OK) {
-            *got = true;
-            return GBMM_OK;
-        }
-        cudaGetLastError();  // a failed allocation: run without the extra
-    }
-    return arena_reserve(h, ws);
-}
-
 // C (+)= A*B with the planned path.  An operand too long for the chosen kernels
 // is split into low and high limb halves, X = X_hi 2^(32h) + X_lo (the
 // Karatsuba-style split of Knuth 4.3.3 without the middle-product trick), and
@@ -1548,6 +1590,14 @@ gbmm_status resolve_plan(gbmm_handle h, const gbmm_mat &a, const gbmm_mat &b, co
 }
 
 }  // namespace gbmm
+
+// Internal hook: bytes that an optional workspace may take in this thread's calls (-1, the
+// default: by the device's free memory); returns the old value.
+extern "C" int64_t gbmmx_extra_room(int64_t bytes) {
+    const int64_t old = t_extra_room;
+    t_extra_room = bytes < 0 ? -1 : bytes;
+    return old;
+}
 
 // Internal hook: schoolbook work (m k n la lb) from which the heuristic takes the CRT
 // form for entries of fewer than 16 limbs together (0: never); returns the old value.

@@ -154,7 +154,7 @@ size_t device_budget(gbmm_handle h) {
     if (h->dev_budget) return h->dev_budget;
     size_t fr = 0, tot = 0;
     if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return (size_t)-1;
-    return fr / 10 * 9 + h->ws.cap;  // the arena can be reused
+    return fr / 10 * 9 + h->ws.plain;  // the arena can be reused (an optional part of it is not counted on)
 }
 
 // One product too large for the device, in blocks (see the file comment).
