@@ -284,6 +284,7 @@ struct gbmm_handle_s {
     void *pipe = nullptr;
     // device bytes a host-buffer product may use before it runs out of core (0: free memory)
     size_t dev_budget = 0;
+    bool in_budget = false;  // a call is running its blocks under dev_budget
     // stage hooks for the next CRT product (pipeline.cpp sets them, crt_matmul clears them)
     gbmm::crt_stage_hooks *stage = nullptr;
 };

@@ -1622,8 +1622,11 @@ extern "C" gbmm_status gbmm_matmul(gbmm_handle h, gbmm_mat c, gbmm_mat a, gbmm_m
     Plan p;
     GBMM_TRY(resolve_plan(h, a, b, o, p));
     bool tc = false;
+    // a block of a product that runs out of core under a device budget takes no optional part:
+    // the block sizes were chosen by the plain workspace
+    const size_t extra = h->in_budget ? 0 : limb_tc_extra(p, a.nlimbs, b.nlimbs, a.rows, a.cols, b.cols);
     GBMM_TRY(arena_reserve_extra(h, dispatch_ws(p, a.nlimbs, b.nlimbs, a.rows, a.cols, b.cols, c.nlimbs, o.accumulate) + 65536,
-                                 limb_tc_extra(p, a.nlimbs, b.nlimbs, a.rows, a.cols, b.cols), &tc));
+                                 extra, &tc));
     h->limb_tc = tc;
     const gbmm_status st = dispatch(h, c, a, b, p, o.accumulate, h->stream);
     h->limb_tc = 0;

@@ -224,8 +224,10 @@ gbmm_status run_blocked(gbmm_handle h, PipeState &ps, gbmm_host_job &q, size_t b
                 if (st != GBMM_OK) break;
                 gbmm_opts o = o0;
                 o.accumulate = t0 > 0;
+                h->in_budget = h->dev_budget != 0;
                 st = gbmm_matmul(h, view(kr, nc, lc, bf.c[cs], bf.cs[cs]), view(kr, mk, la, bf.a[s], bf.as[s]),
                                  view(mk, nc, lb, bf.b[s], bf.bs[s]), &o);
+                h->in_budget = false;
                 if (st == GBMM_OK) st = ck(cudaEventRecord(bf.comp[s], h->stream), "cudaEventRecord");
                 if (q.M == 0) break;
             }

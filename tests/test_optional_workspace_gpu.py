@@ -1,6 +1,7 @@
 """The workspace with which limb products run on the tensor cores is optional: a call
 that the plain workspace serves is not refused, does not end a stream capture, does not
-grow the workspace past what later calls need and gives nothing up for a refused part."""
+grow the workspace past what later calls need, gives nothing up for a refused part and
+stays inside a device budget."""
 import random
 
 import pytest
@@ -107,3 +108,30 @@ def test_graphs_survive_a_refused_request(g):
         assert replayed()
         _check(A, B, n, dC)
         h.close()
+
+
+def test_device_budget_covers_blocked_limb_products(g):
+    """A product that runs out of core under a device budget takes no optional workspace
+    beside its blocks (its footprint counts the plain workspace)."""
+    import numpy as np
+    import torch
+    n, limbs = 96, 32
+    rng = random.Random(8)
+    A, B = ([rng.getrandbits(32 * limbs) * rng.choice((-1, 1)) for _ in range(n * n)] for _ in range(2))
+    (Al, As), (Bl, Bs) = g.ints_to_planes(A, limbs), g.ints_to_planes(B, limbs)
+    Cl, Cs = np.zeros((2 * limbs + 1, n * n), dtype=np.uint32), np.zeros(n * n, dtype=np.int32)
+    h = g.Handle()
+    spec = [(n, n, n, (Al, As), (Bl, Bs), (Cl, Cs))]
+    for budget in (0, 12 << 20):
+        h.set_device_budget(budget)
+        g.profile(1)
+        h.matmul_host(h.host_jobs(spec, path=g.PATH_LIMB, method=g.METHOD_NAIVE))
+        ran = g.profile_read()
+        g.profile(0)
+        assert ("k_ltc_gemm" in ran) == (budget == 0)
+        got = g.planes_to_ints(Cl, Cs)
+        for _ in range(40):
+            y, x = rng.randrange(n), rng.randrange(n)
+            assert got[y * n + x] == sum(A[y * n + k] * B[k * n + x] for k in range(n))
+        Cl[:], Cs[:] = 0, 0
+    h.close()
