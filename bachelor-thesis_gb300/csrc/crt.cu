@@ -306,52 +306,25 @@ __device__ __forceinline__ void residue_fold(const uint32_t (&v)[32], int mi0, b
 // PAIR: a cluster of two CTAs shares one M = 256 tcgen05.mma.cta_group::2 per K
 // slice (issued by the even CTA); each CTA stages its own 128 entries and half of
 // the tile's table columns, and keeps its own 128 rows of D in its TMEM.
-// MC: a cluster of two CTAs with an M = 128 MMA each, on neighbouring 128-entry
-// row blocks and the same table columns: each CTA loads half of the table box and
-// multicasts it to both, so the table is read from L2 once per pair of row blocks,
-// and each CTA's MMA commit frees the stage in both CTAs.
 // GRP: a grouped launch (single CTAs only); every stage is sized for GBN table
 // columns (the launch's operands have table tiles of at most GBN columns).
-template <int STAGES, bool PAIR, bool MC, int GS, bool GRP, int GBN = 256>
+template <int STAGES, bool PAIR, int GS, bool GRP, int GBN = 256>
 __global__ void __launch_bounds__(RES_THREADS, 1)
     k_crt_residue(const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmT,
                   const __grid_constant__ CUtensorMap tmR, ResidueArgs a0, Group<ResidueJob> grp, uint32_t *err) {
-    static_assert(!GRP || (!PAIR && !MC), "grouped residue launches use single CTAs");
+    static_assert(!GRP || !PAIR, "grouped residue launches use single CTAs");
     extern __shared__ uint8_t smem_raw[];
     uint8_t *base = align1024(smem_raw);
-    constexpr bool CL = PAIR || MC;     // launched as clusters of two CTAs
-    constexpr int NP = CL ? 2 : 1;      // row blocks per tile (per cluster)
+    constexpr int NP = PAIR ? 2 : 1;    // row blocks per tile (per cluster)
     constexpr int NBUF = PAIR ? 2 : 1;  // staging buffers per epilogue warp
     const uint32_t A_BYTES = BM * 128, B_BYTES = GRP ? (uint32_t)GBN * 128 : (uint32_t)(PAIR ? a0.BN / 2 : a0.BN) * 128,
                    STAGE = A_BYTES + B_BYTES;
     Barriers *bars = reinterpret_cast<Barriers *>(base + STAGES * STAGE);
     uint8_t *stage_out = reinterpret_cast<uint8_t *>(bars) + SMEM_BARS;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t rank = CL ? tc::cluster_rank() : 0;
-    const int64_t t0 = CL ? (blockIdx.x >> 1) : blockIdx.x, tstep = CL ? (gridDim.x >> 1) : gridDim.x;
-    if (MC) {
-        // per CTA as below, but every stage is freed by both CTAs' MMA commits
-        if (threadIdx.x == 0) {
-            for (int s = 0; s < STAGES; s++) {
-                tc::mbar_init(&bars->full[s], 1);
-                tc::mbar_init(&bars->empty[s], 2);
-            }
-            for (int b = 0; b < 2; b++) {
-                tc::mbar_init(&bars->tfull[b], 1);
-                tc::mbar_init(&bars->tempty[b], RES_EPI_WARPS);
-            }
-            bars->abort_flag = 0;
-            tc::fence_mbar_init();
-        }
-        if (warp == 1) {
-            tc::tmem_alloc(&bars->tmem_base, 512);
-            tc::tmem_relinquish();
-        }
-        tc::fence_before_sync();
-        __syncthreads();
-        tc::cluster_sync_all();  // both CTAs' barriers exist before any multicast lands
-        tc::fence_after_sync();
-    } else if (PAIR) {
+    const uint32_t rank = PAIR ? tc::cluster_rank() : 0;
+    const int64_t t0 = PAIR ? (blockIdx.x >> 1) : blockIdx.x, tstep = PAIR ? (gridDim.x >> 1) : gridDim.x;
+    if (PAIR) {
         if (threadIdx.x == 0) {
             for (int s = 0; s < STAGES; s++) {
                 tc::mbar_init(&bars->full[s], 1);
@@ -379,7 +352,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1)
     const uint32_t tmem = bars->tmem_base;
     // the last table tile may be narrow: its MMA has only the columns it needs
     // (a multiple of 16, of 32 for a pair so that each CTA stages whole 8-row groups)
-    const int ngran = CL ? 32 : 16;
+    const int ngran = PAIR ? 32 : 16;
     const int64_t total = GRP ? grp.tile0[grp.njobs] : (int64_t)a0.ntiles;
     // global tile T -> its operand's arguments and maps, and the tile within it
     GroupCursor cur;
@@ -430,12 +403,6 @@ __global__ void __launch_bounds__(RES_THREADS, 1)
                         if (rank == 0) tc::mbar_arrive_expect_tx(&bars->full[st], 2 * STAGE);
                         tc::tma_load_2d_pair(sa, mD, full0, s * BK, (int)e0);
                         tc::tma_load_2d_pair(sa + A_BYTES, mT, full0, s * BK, n0 + (int)rank * (nn / 2));
-                    } else if (MC) {
-                        // own digit rows; this CTA's half of the table box to both CTAs
-                        tc::mbar_arrive_expect_tx(&bars->full[st], STAGE);
-                        tc::tma_load_2d(sa, mD, &bars->full[st], s * BK, (int)e0);
-                        tc::tma_load_2d_mc(sa + A_BYTES + rank * (B_BYTES / 2), mT, &bars->full[st], s * BK,
-                                           n0 + (int)rank * (a.BN / 2), 0x3);
                     } else {
                         // a grouped stage holds this operand's BN table rows of its 256
                         tc::mbar_arrive_expect_tx(&bars->full[st], GRP ? A_BYTES + (uint32_t)a.BN * 128 : STAGE);
@@ -446,7 +413,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1)
             }
         }
     } else if (warp == 1) {
-        if ((rank == 0 || MC) && tc::elect_one()) {
+        if (rank == 0 && tc::elect_one()) {
             int it = 0, lt = 0;
             bool ok = true;
             for (int64_t T = t0; T < total && ok; T += tstep, lt++) {
@@ -477,7 +444,6 @@ __global__ void __launch_bounds__(RES_THREADS, 1)
                         else tc::mma_bf16(d, adesc, bdesc, idesc, acc);
                     }
                     if (PAIR) tc::mma_commit_pair(&bars->empty[st], 0x3);
-                    else if (MC) tc::mma_commit_mc(&bars->empty[st], 0x3);
                     else tc::mma_commit(&bars->empty[st]);
                 }
                 if (ok) {
@@ -614,14 +580,6 @@ __global__ void __launch_bounds__(RES_THREADS, 1)
         if (warp == 1) {
             tc::fence_after_sync();
             tc::tmem_dealloc_pair(tmem, 512);
-        }
-    } else if (MC) {
-        tc::fence_before_sync();
-        __syncthreads();
-        tc::cluster_sync_all();  // no CTA leaves while its peer may still multicast into it or arrive on it
-        if (warp == 1) {
-            tc::fence_after_sync();
-            tc::tmem_dealloc(tmem, 512);
         }
     } else {
         cta_teardown(bars, 512);
@@ -2405,11 +2363,9 @@ static constexpr int REC_STAGES_PAIR = 6;  // a pair CTA stages 32 KB per K step
 static constexpr int RES_STAGES_PAIR = 5;  // a pair CTA stages 32 KB per K step
 static constexpr int PROD_STAGES_PAIR = 5;  // a pair CTA stages 40 KB per K step
 static constexpr int PROD_PAIR_MIN_NK = 8;  // K steps (of 64) from which the product runs on CTA pairs
-// residue GEMM form: -1 by the K loop's length, 0 single CTAs, 1 CTA pairs
-static int g_residue_mode = -1;  // -1 by size, 0 one CTA, 1 CTA pairs, 2 multicast clusters
+static int g_residue_mode = -1;  // residue GEMM form: -1 by the K loop's length, 0 one CTA, 1 CTA pairs
 static constexpr int RES_PAIR_MIN_NK = 1 << 30;  // the pair form of the residue GEMM measured slower at every size
 static bool residue_pair(int nk) { return g_residue_mode < 0 ? nk >= RES_PAIR_MIN_NK : g_residue_mode == 1; }
-static bool residue_mc(int nk) { (void)nk; return g_residue_mode == 2; }
 
 static int num_sms() {
     static int n = 0;
@@ -2503,7 +2459,7 @@ struct OperandPlan {
     DigitArgs da;
     dim3 dgrid;
     int balanced = 0, gsteps = 0;
-    bool pair = false, mc = false;
+    bool pair = false;
     CUtensorMap tmD, tmT, tmR;
     ResidueArgs ra;
     size_t smem = 0;
@@ -2531,8 +2487,7 @@ static gbmm_status plan_operand(crt_tables *t, const gbmm_mat &X, int transpose,
     while (BN * G > 256) BN /= 2;
     if (BN < 64) return set_error(GBMM_ERR_UNSUPPORTED, "crt: entries longer than 30720 bits");
     op.pair = !grouped && residue_pair(nk);
-    op.mc = !grouped && !op.pair && residue_mc(nk);
-    const int NP = op.pair || op.mc ? 2 : 1;
+    const int NP = op.pair ? 2 : 1;
     GBMM_TRY(make_map(&op.tmD, D, dxp, E, dxp, BK, BM));
     GBMM_TRY(make_map(&op.tmT, T, dxp, residue_cols(t->P), tpitch, BK, BN / NP));
     ResidueArgs &r = op.ra;
@@ -2587,18 +2542,14 @@ static gbmm_status launch_operand(const OperandPlan &op, const crt_halves *halve
     LaunchScope ls_("k_crt_residue", s);
 #define RESIDUE_LAUNCH(GS_)                                                                                          \
     do {                                                                                                             \
-        if (op.mc) {                                                                                                 \
-            GBMM_TRY(set_smem((const void *)k_crt_residue<RES_STAGES, false, true, GS_, false>, sm));                \
-            GBMM_TRY(launch_pairs(k_crt_residue<RES_STAGES, false, true, GS_, false>, RES_THREADS, op.ra.ntiles, sm, \
-                                  s, op.tmD, op.tmT, op.tmR, op.ra, none, device_error_word()));                     \
-        } else if (op.pair) {                                                                                        \
-            GBMM_TRY(set_smem((const void *)k_crt_residue<RES_STAGES_PAIR, true, false, GS_, false>, sm));           \
-            GBMM_TRY(launch_pairs(k_crt_residue<RES_STAGES_PAIR, true, false, GS_, false>, RES_THREADS,            \
+        if (op.pair) {                                                                                       \
+            GBMM_TRY(set_smem((const void *)k_crt_residue<RES_STAGES_PAIR, true, GS_, false>, sm));           \
+            GBMM_TRY(launch_pairs(k_crt_residue<RES_STAGES_PAIR, true, GS_, false>, RES_THREADS,            \
                                   op.ra.ntiles, sm, s, op.tmD, op.tmT, op.tmR, op.ra, none, device_error_word()));   \
         } else {                                                                                                     \
-            GBMM_TRY(set_smem((const void *)k_crt_residue<RES_STAGES, false, false, GS_, false>, sm));               \
+            GBMM_TRY(set_smem((const void *)k_crt_residue<RES_STAGES, false, GS_, false>, sm));               \
             dim3 grid((unsigned)std::min<int64_t>(op.ra.ntiles, num_sms()));                                         \
-            GBMM_TRY(launch_one(k_crt_residue<RES_STAGES, false, false, GS_, false>, grid, RES_THREADS, sm, s,      \
+            GBMM_TRY(launch_one(k_crt_residue<RES_STAGES, false, GS_, false>, grid, RES_THREADS, sm, s,      \
                                 op.tmD, op.tmT, op.tmR, op.ra, none, device_error_word()));                          \
         }                                                                                                            \
     } while (0)
@@ -3159,19 +3110,19 @@ gbmm_status crt_group_launch(crt_group *g, const char *d_blob, cudaStream_t s, c
         const size_t stg = (size_t)RES_EPI_WARPS * RES_STG_BYTES;
         LaunchScope ls_("k_crt_residue", s);
         if (f == 0) {
-            auto kern = k_crt_residue<RES_STAGES, false, false, RES_GROUP_STEPS_U, true, 256>;
+            auto kern = k_crt_residue<RES_STAGES, false, RES_GROUP_STEPS_U, true, 256>;
             const size_t sm = smem_bytes(RES_STAGES, BM * 128 + 256 * 128) + stg;
             GBMM_TRY(set_smem((const void *)kern, sm));
             GBMM_TRY(launch_one(kern, grid, RES_THREADS, sm, s, zmap, zmap, zmap, none,
                                 group_at<ResidueJob>(d_blob, sec), err));
         } else if (f == 1) {
-            auto kern = k_crt_residue<RES_STAGES, false, false, RES_GROUP_STEPS_B, true, 256>;
+            auto kern = k_crt_residue<RES_STAGES, false, RES_GROUP_STEPS_B, true, 256>;
             const size_t sm = smem_bytes(RES_STAGES, BM * 128 + 256 * 128) + stg;
             GBMM_TRY(set_smem((const void *)kern, sm));
             GBMM_TRY(launch_one(kern, grid, RES_THREADS, sm, s, zmap, zmap, zmap, none,
                                 group_at<ResidueJob>(d_blob, sec), err));
         } else {
-            auto kern = k_crt_residue<RES_STAGES_NARROW, false, false, RES_GROUP_STEPS_B, true, 128>;
+            auto kern = k_crt_residue<RES_STAGES_NARROW, false, RES_GROUP_STEPS_B, true, 128>;
             const size_t sm = smem_bytes(RES_STAGES_NARROW, BM * 128 + 128 * 128) + stg;
             GBMM_TRY(set_smem((const void *)kern, sm));
             GBMM_TRY(launch_one(kern, grid, RES_THREADS, sm, s, zmap, zmap, zmap, none,
@@ -3339,9 +3290,9 @@ extern "C" int32_t gbmmx_launch_pdl(int32_t enable) {
 }
 
 // Test hook: the residue GEMM's form (-1 by the K loop's length, 0 single CTAs,
-// 1 CTA pairs); returns the previous setting.
+// 1 or more CTA pairs); returns the previous setting.
 extern "C" int32_t gbmmx_residue_mode(int32_t mode) {
     const int32_t old = g_residue_mode;
-    g_residue_mode = mode < 0 ? -1 : (mode > 2 ? 2 : mode);
+    g_residue_mode = mode < 0 ? -1 : (mode > 1 ? 1 : mode);
     return old;
 }

@@ -74,17 +74,6 @@ __device__ __forceinline__ void tma_load_2d(void *smem_dst, const CUtensorMap *m
         "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y)
         : "memory");
 }
-// TMA load multicast to the CTAs of `mask` in the cluster: the box lands at the
-// same shared-memory offset in each of them and completes on the mbarrier at the
-// same offset in each
-__device__ __forceinline__ void tma_load_2d_mc(void *smem_dst, const CUtensorMap *map, uint64_t *bar, int x, int y,
-                                               uint16_t mask) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.multicast::cluster [%0], [%1, {%3, "
-        "%4}], [%2], %5;" ::"r"(smem_u32(smem_dst)),
-        "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y), "h"(mask)
-        : "memory");
-}
 __device__ __forceinline__ void tma_load_3d(void *smem_dst, const CUtensorMap *map, uint64_t *bar, int x, int y, int z) {
     asm volatile(
         "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(
@@ -295,15 +284,6 @@ __device__ __forceinline__ void mma_bf16_pair(uint32_t d_tmem, uint64_t adesc, u
         : "memory");
 }
 // arrive on the mbarrier at this offset in every CTA of `mask` once the pair's prior MMAs complete
-// arrive (once per CTA of `mask`) on the mbarrier at this offset in each of those
-// CTAs when this CTA's MMAs issued so far have completed
-__device__ __forceinline__ void mma_commit_mc(uint64_t *bar, uint16_t mask) {
-    asm volatile(
-        "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
-            smem_u32(bar)),
-        "h"(mask)
-        : "memory");
-}
 __device__ __forceinline__ void mma_commit_pair(uint64_t *bar, uint16_t mask) {
     asm volatile(
         "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
