@@ -1047,16 +1047,13 @@ __global__ void k_mpz_addsub(MatArgs W, MatArgs U, MatArgs V, int sub, int64_t c
 // in the same pass.  When w and the product have opposite signs the merge is a
 // two's complement subtraction; a final borrow means |uv| > |w| and the
 // written limbs are negated in place.
-__global__ void k_mpz_mulops(MatArgs W, MatArgs U, MatArgs V, int op, int64_t count, uint32_t *err) {
-    int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= count) return;
-    const int64_t iw = ent(W, e), iu = ent(U, e), iv = ent(V, e);
-    const int su = U.sizes[iu], sv = V.sizes[iv];
-    const int un = iabs_d(su), vn = iabs_d(sv);
-    const uint32_t *up = U.limbs + iu, *vp = V.limbs + iv;
+__device__ __forceinline__ void mulops_entry(const MatArgs &W, const MatArgs &U, const MatArgs &V, int op, int64_t e, int su,
+                                             int sv, int sw, uint32_t *err) {
+    const int64_t iw = ent(W, e);
+    const int un = min(iabs_d(su), U.nlimbs), vn = min(iabs_d(sv), V.nlimbs);
+    const uint32_t *up = U.limbs + ent(U, e), *vp = V.limbs + ent(V, e);
     uint32_t *wp = W.limbs + iw;
     const int64_t ws = W.ld;
-    int sw = op == 0 ? 0 : W.sizes[iw];
     const int wn = iabs_d(sw);
     int pneg = (su < 0) ^ (sv < 0);
     if (op == 2) pneg ^= 1;
@@ -1122,6 +1119,12 @@ __global__ void k_mpz_mulops(MatArgs W, MatArgs U, MatArgs V, int op, int64_t co
     W.sizes[iw] = top == 0 ? 0 : (neg ? -top : top);
 }
 
+__global__ void k_mpz_mulops(MatArgs W, MatArgs U, MatArgs V, int op, int64_t count, uint32_t *err) {
+    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= count) return;
+    mulops_entry(W, U, V, op, e, U.sizes[ent(U, e)], V.sizes[ent(V, e)], op == 0 ? 0 : W.sizes[ent(W, e)], err);
+}
+
 // The same operations with the operands staged on chip (as k_mpn_mul_basecase_sm): a CTA
 // of NT threads takes NT entries, each thread forms its product in 4 x 4 limb blocks
 // from shared memory and merges W's limbs, which are loaded a block ahead of the
@@ -1130,38 +1133,54 @@ __global__ void k_mpz_mulops(MatArgs W, MatArgs U, MatArgs V, int op, int64_t co
 // entries of 16 limbs into 33: 347 us with the kernel above, 130 us with this one
 // (3.3 TB/s; the loads of W and the second pass over negative results keep it from more).
 //
+// Entries may be much shorter than their planes (sums, accumulators with room to grow): the
+// limbs read and the blocks multiplied go by the CTA's longest entries, a CTA whose
+// products have at most MPZ_DIRECT limb products takes the kernel above's way, and the
+// shared memory (with it the threads an SM holds) goes by the planes of U, V and W: a
+// factor of a product that fits W has at most one limb more than W.  An entry past `room`
+// words (a result that does not fit) takes the kernel above's way too.
+// 2^20 entries, us (the kernel above; every plane read and multiplied; this): 4 limbs of 64 planes
+// into 10 49, 306, 48; 4 of 16 into 33 60, 94, 66; 4 of 64 into 129 103, 503, 165 (three CTAs an SM).
+//
 // Limbs of U and V above their sizes are staged as zeros.  The product runs over
 // the warp's longest operands, so that a warp's loads and stores of W stay whole
-// lines; W's limbs above the result are written as zeros in the same pass.
+// lines; W's limbs above the result are written as zeros.
+constexpr int MPZ_DIRECT = 8;
+// out of line: its registers would cost the staged product's loop 4 % (700 x 700 limbs)
+__device__ __noinline__ void mulops_short(MatArgs W, MatArgs U, MatArgs V, int op, int64_t e, int su, int sv, int sw,
+                                          uint32_t *err) {
+    mulops_entry(W, U, V, op, e, su, sv, sw, err);
+}
+
+// Limbs [0, n) of entries e0 .. e0 + NT - 1 into dst[t * SS + i], zeros above an entry's size
+// up to whole blocks of four; ssz: the entries' lengths in shared memory (zeros past the last entry).
 template <int NT>
-__device__ __forceinline__ void mpz_stage(uint32_t *dst, int SS, int32_t *ssz, const MatArgs &M, int64_t e0, int64_t count,
-                                          bool vec) {
-    if (e0 + threadIdx.x < count) ssz[threadIdx.x] = M.sizes[ent(M, e0 + threadIdx.x)];
-    else ssz[threadIdx.x] = 0;
-    __syncthreads();
+__device__ __forceinline__ void mpz_stage(uint32_t *dst, int SS, const int32_t *ssz, const MatArgs &M, int n, int64_t e0,
+                                          int64_t count, bool vec) {
     constexpr int NQ = NT / 4;
-    const int n4 = (M.nlimbs + 3) >> 2;
+    const int n4 = (n + 3) >> 2;
     for (int item = threadIdx.x; item < n4 * NQ; item += NT) {
         const int q = item % NQ, c = item / NQ;
         const int64_t eq = e0 + 4 * q;
         uint32_t L[4][4];  // L[k][j]: limb 4c + k of entry eq + j
-        int sz[4];
+        int sz[4], longest = 0;
         int64_t off[4];
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            sz[j] = iabs_d(ssz[4 * q + j]);
+            sz[j] = ssz[4 * q + j];
+            longest = max(longest, sz[j]);
             off[j] = vec ? eq + j : (eq + j < count ? ent(M, eq + j) : 0);
         }
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             const int i = 4 * c + k;
             const uint32_t *row = M.limbs + (int64_t)i * M.ld;
-            if (i < M.nlimbs && vec && eq + 3 < count) {
-                const uint4 w = *reinterpret_cast<const uint4 *>(row + eq);
+            if (vec && eq + 3 < count) {
+                const uint4 w = i < longest ? *reinterpret_cast<const uint4 *>(row + eq) : make_uint4(0u, 0u, 0u, 0u);
                 L[k][0] = w.x; L[k][1] = w.y; L[k][2] = w.z; L[k][3] = w.w;
             } else {
 #pragma unroll
-                for (int j = 0; j < 4; j++) L[k][j] = (i < M.nlimbs && eq + j < count) ? row[off[j]] : 0u;
+                for (int j = 0; j < 4; j++) L[k][j] = i < sz[j] ? row[off[j]] : 0u;
             }
 #pragma unroll
             for (int j = 0; j < 4; j++)
@@ -1184,37 +1203,55 @@ __device__ __forceinline__ void mpz_stage(uint32_t *dst, int SS, int32_t *ssz, c
                 make_uint4(L[0][jj], L[1][jj], L[2][jj], L[3][jj]);
     }
 }
+
+// Registers: seven CTAs of 128 threads an SM; CTAs of 64 and 32 threads take 100 KB and more
+// of shared memory, so two.
 template <int NT>
-__global__ void __launch_bounds__(NT, 896 / NT) k_mpz_mulops_sm(MatArgs W, MatArgs U, MatArgs V, int op, int64_t count, int vec_u,
-                                                      int vec_v, uint32_t *err) {
+__global__ void __launch_bounds__(NT, NT == 128 ? 7 : 2) k_mpz_mulops_sm(MatArgs W, MatArgs U, MatArgs V, int op, int64_t count, int vec_u,
+                                                                int vec_v, int room, uint32_t *err) {
     extern __shared__ uint4 sm_raw4[];
     uint32_t *sm = reinterpret_cast<uint32_t *>(sm_raw4);
-    const int Su = sm_stride(U.nlimbs), Sv = sm_stride(V.nlimbs);
-    uint32_t *su_ = sm, *sv_ = sm + NT * Su;
-    int32_t *szu = reinterpret_cast<int32_t *>(sv_ + NT * Sv), *szv = szu + NT;
-    const int64_t e0 = (int64_t)blockIdx.x * NT;
-    mpz_stage<NT>(su_, Su, szu, U, e0, count, vec_u);
-    mpz_stage<NT>(sv_, Sv, szv, V, e0, count, vec_v);
-    __syncthreads();
-    const int64_t e = e0 + threadIdx.x;
+    __shared__ int32_t ssz[2][NT];
+    const int64_t e0 = (int64_t)blockIdx.x * NT, e = e0 + threadIdx.x;
     const bool live = e < count;
-    const int su = szu[threadIdx.x], sv = szv[threadIdx.x];
-    const int un = min(iabs_d(su), U.nlimbs), vn = min(iabs_d(sv), V.nlimbs);
+    const int su = live ? U.sizes[ent(U, e)] : 0, sv = live ? V.sizes[ent(V, e)] : 0;
     const int64_t iw = live ? ent(W, e) : 0;
-    const int cap = W.nlimbs;
     const int sw = op == 0 || !live ? 0 : W.sizes[iw];
+    const bool prod = su && sv;
+    const int un = prod ? min(iabs_d(su), U.nlimbs) : 0, vn = prod ? min(iabs_d(sv), V.nlimbs) : 0;
+    ssz[0][threadIdx.x] = un;
+    ssz[1][threadIdx.x] = vn;
+    __syncthreads();
+    int bu = 0, bv = 0;  // the CTA's longest
+#pragma unroll
+    for (int w = 0; w < NT; w += 32) {
+        bu = max(bu, ssz[0][w + (threadIdx.x & 31)]);
+        bv = max(bv, ssz[1][w + (threadIdx.x & 31)]);
+    }
+    bu = __reduce_max_sync(0xFFFFFFFFu, bu);
+    bv = __reduce_max_sync(0xFFFFFFFFu, bv);
+    const int Su = sm_stride(bu), Sv = sm_stride(bv);
+    if (bu * bv <= MPZ_DIRECT || NT * (Su + Sv) > room) {
+        if (live) mulops_short(W, U, V, op, e, su, sv, sw, err);
+        return;
+    }
+    uint32_t *su_ = sm, *sv_ = sm + NT * Su;
+    mpz_stage<NT>(su_, Su, ssz[0], U, bu, e0, count, vec_u);
+    mpz_stage<NT>(sv_, Sv, ssz[1], V, bv, e0, count, vec_v);
+    __syncthreads();
+    const int cap = W.nlimbs;
     const int wn = min(iabs_d(sw), cap);
     int pneg = (su < 0) ^ (sv < 0);
     if (op == 2) pneg ^= 1;
-    const bool prod = un && vn;
     const bool subtract = wn && prod && ((sw < 0) != (pneg != 0));
-    const int nu = __reduce_max_sync(0xFFFFFFFFu, prod ? (un + 3) >> 2 : 0);
-    const int nv = __reduce_max_sync(0xFFFFFFFFu, prod ? (vn + 3) >> 2 : 0);
+    const int nu = (__reduce_max_sync(0xFFFFFFFFu, un) + 3) >> 2, nv = (__reduce_max_sync(0xFFFFFFFFu, vn) + 3) >> 2;
+    // blocks up to the warp's longest product and W, one more for the carry; a zero operand is
+    // staged as zeros, so its product is zero over the warp's length too
+    const int ww = __reduce_max_sync(0xFFFFFFFFu, wn);
+    const int nT = max(nu + nv, min(max(nu + nv, (ww + 3) >> 2) + 1, (cap + 3) >> 2));
     if (!live) return;
     uint32_t *wp = W.limbs + iw;
     const int64_t ws = W.ld;
-    // a zero operand is staged as zeros, so its product is zero over the warp's length too
-    const int nT = max(nu + nv, (cap + 3) >> 2);
     // W's limbs of this block and of the next two (in flight)
     uint32_t wl[4], wx[4], wy[4];
     auto wload = [&](int T, uint32_t(&x)[4]) {
@@ -1265,13 +1302,14 @@ __global__ void __launch_bounds__(NT, 896 / NT) k_mpz_mulops_sm(MatArgs W, MatAr
         neg = pneg;
         uint32_t c = 1;
         top = 0;
-        for (int t0 = 0; t0 < cap; t0 += 8) {
+        const int kept = min(4 * nT, cap);
+        for (int t0 = 0; t0 < kept; t0 += 8) {
             uint32_t x[8];
 #pragma unroll
-            for (int i = 0; i < 8; i++) x[i] = t0 + i < cap ? wp[(int64_t)(t0 + i) * ws] : 0u;
+            for (int i = 0; i < 8; i++) x[i] = t0 + i < kept ? wp[(int64_t)(t0 + i) * ws] : 0u;
 #pragma unroll
             for (int i = 0; i < 8; i++) {
-                if (t0 + i >= cap) break;
+                if (t0 + i >= kept) break;
                 const uint64_t s = (uint64_t)(~x[i]) + c;
                 c = (uint32_t)(s >> 32);
                 wp[(int64_t)(t0 + i) * ws] = (uint32_t)s;
@@ -1282,6 +1320,9 @@ __global__ void __launch_bounds__(NT, 896 / NT) k_mpz_mulops_sm(MatArgs W, MatAr
         atomicOr(err, DEVERR_CAPACITY);
         return;
     }
+    uint32_t *zp = wp + (int64_t)(4 * nT) * ws;
+#pragma unroll 4
+    for (int t = 4 * nT; t < cap; t++, zp += ws) *zp = 0u;
     W.sizes[iw] = top == 0 ? 0 : (neg ? -top : top);
 }
 
@@ -2334,8 +2375,9 @@ gbmm_status launch_mpz_mulops(const gbmm_mat &w, const gbmm_mat &u, const gbmm_m
     // staged on chip wherever 32 or more entries' operands fit in shared memory, but for the
     // shortest products, whose limbs are read once anyway (10^6 addmul, us, staged and not: 1 x 1
     // limbs 35 and 22, 2 x 2 36 and 31, 2 x 4 39 and 39, 4 x 4 47 and 51, 16 x 16 127 and 337)
-    const size_t words = (size_t)sm_stride(u.nlimbs) + sm_stride(v.nlimbs) + 2;
-    const int nt = (int64_t)u.nlimbs * v.nlimbs > 8 ? sm_threads(words) : 0;
+    const int64_t ul = std::min<int64_t>(u.nlimbs, (int64_t)w.nlimbs + 1), vl = std::min<int64_t>(v.nlimbs, (int64_t)w.nlimbs + 1);
+    const size_t words = (size_t)sm_stride((int)ul) + sm_stride((int)vl);
+    const int nt = ul * vl > MPZ_DIRECT ? sm_threads(words + 2) : 0;  // two words an entry of static shared memory
     LaunchScope ls_("k_mpz_mulops", s);
     if (nt) {
         const size_t smem = nt * words * 4;
@@ -2344,7 +2386,7 @@ gbmm_status launch_mpz_mulops(const gbmm_mat &w, const gbmm_mat &u, const gbmm_m
     do {                                                                                                              \
         GBMM_CUDA_TRY(cudaFuncSetAttribute(k_mpz_mulops_sm<NT_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
         k_mpz_mulops_sm<NT_><<<grid1(n, NT_), NT_, smem, s>>>(margs(w), margs(u), margs(v), op, n, vu, vv,            \
-                                                              device_error_word());                                   \
+                                                              (int)(smem / 4), device_error_word());                                   \
     } while (0)
         if (nt == 128) MULOPS_SM(128);
         else if (nt == 64) MULOPS_SM(64);
