@@ -240,7 +240,7 @@ extern "C" gbmm_status gbmm_matmul_batched(gbmm_handle h, gbmm_job *jobs, int32_
         oj.path = q.path ? q.path : o.path;
         if (q.cutoff) oj.cutoff = q.cutoff;
         if (q.nprimes) oj.nprimes = q.nprimes;
-        GBMM_TRY(resolve_plan(h, q.a, q.b, oj, plans[j]));
+        GBMM_TRY(resolve_plan(h, q.a, q.b, oj, plans[j], true));
         jobs[j].chosen_path = plans[j].path;
         jobs[j].chosen_plan = plans[j].id;
     }

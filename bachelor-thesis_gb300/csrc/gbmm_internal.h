@@ -240,7 +240,8 @@ gbmm_status crt_collect(gbmm_handle h, crt_group *g, const gbmm_mat &c, const gb
 size_t limb_tc_extra(const Plan &p, int la, int lb, int m, int k, int n);
 // Reserves `ws` bytes, with `extra` more when they can be had without giving anything up; *got says whether
 gbmm_status arena_reserve_extra(gbmm_handle h, size_t ws, size_t extra, bool *got);
-gbmm_status resolve_plan(gbmm_handle h, const gbmm_mat &a, const gbmm_mat &b, const gbmm_opts &o, Plan &p);
+// batch: the product runs in a batch, where limb products stay on the CUDA cores
+gbmm_status resolve_plan(gbmm_handle h, const gbmm_mat &a, const gbmm_mat &b, const gbmm_opts &o, Plan &p, bool batch = false);
 void invalidate_graphs(gbmm_handle h);
 void batch_state_destroy(gbmm_handle h);
 // learned cost model (mlp.cu): the gbmm_plan it picks, or -1 when no model applies

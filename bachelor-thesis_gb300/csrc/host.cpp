@@ -1566,7 +1566,7 @@ gbmm_status crt_collect(gbmm_handle h, crt_group *g, const gbmm_mat &c, const gb
     return GBMM_OK;
 }
 
-gbmm_status resolve_plan(gbmm_handle h, const gbmm_mat &a, const gbmm_mat &b, const gbmm_opts &o, Plan &p) {
+gbmm_status resolve_plan(gbmm_handle h, const gbmm_mat &a, const gbmm_mat &b, const gbmm_opts &o, Plan &p, bool batch) {
     if (o.plan) {
         if (o.plan < 1 || o.plan > GBMM_NPLANS) return set_error(GBMM_ERR_INVALID, "unknown plan %d", o.plan - 1);
         p = plan_of(o.plan - 1);
@@ -1574,7 +1574,13 @@ gbmm_status resolve_plan(gbmm_handle h, const gbmm_mat &a, const gbmm_mat &b, co
         return GBMM_OK;
     }
     if (o.path == GBMM_PATH_AUTO) {
-        p = plan_of(choose_plan(h, a.rows, a.cols, b.cols, a.nlimbs, b.nlimbs));
+        int id = choose_plan(h, a.rows, a.cols, b.cols, a.nlimbs, b.nlimbs);
+        // the table's and the model's times are those of products run alone, where limb products
+        // may run on the tensor cores; a batch runs them on the CUDA cores (up to five times
+        // slower), so there such a time counts for nothing
+        if (batch && limb_tc_extra(plan_of(id), a.nlimbs, b.nlimbs, a.rows, a.cols, b.cols))
+            id = heuristic_plan(a.rows, a.cols, b.cols, a.nlimbs, b.nlimbs);
+        p = plan_of(id);
         if (o.cutoff > 0) p.cutoff = o.cutoff;
         p.nprimes = o.nprimes;
         return GBMM_OK;

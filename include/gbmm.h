@@ -280,6 +280,8 @@ gbmm_status gbmm_set_graphs(gbmm_handle h, int32_t enable);
  * log_path (may be NULL): the timing record the learned cost model trains on.
  * Limb candidates predicted far slower than any plan needs (m k n la lb > 2e11)
  * and Winograd cutoffs that give no recursion at this size are skipped.
+ * The times are those of products run alone; a batch takes a limb plan from the
+ * table only where it runs on the CUDA cores alone too.
  * replaces: the fixed BASE_SIZE / TRANSFER_SIZE / GPU_BLK_* tuning constants
  * (mat-gpu/mat-params.h:4-14). */
 gbmm_status gbmm_autotune(gbmm_handle h, const gbmm_job *jobs, int32_t njobs, int32_t repeats,
