@@ -230,6 +230,9 @@ bool crt_groupable(const Plan &p, int la, int lb, int m, int k, int n);
 // Winograd's breadth-first tree with CRT leaf products (GBMM_METHOD_WINOGRAD_CRT):
 // whether it takes this product, its workspace, and the product itself
 bool wino_crt_ok(int la, int lb, int m, int k, int n, int cutoff);
+// whether dispatch() hands the product itself to crt_matmul (no limb-half split, whose halves
+// are another product, and no tree, which reads B first): only then stage hooks apply
+bool dispatch_crt_whole(const Plan &p, int la, int lb, int m, int k, int n);
 size_t wino_crt_ws(int la, int lb, int N, int cn, int cutoff);
 gbmm_status wino_crt(gbmm_handle h, const gbmm_mat &c, const gbmm_mat &a, const gbmm_mat &b, int cutoff,
                      cudaStream_t s);

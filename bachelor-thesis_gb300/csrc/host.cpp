@@ -1344,6 +1344,11 @@ static bool direct_ok(const Plan &p, int la, int lb, int k) {
     return limb_kernel_fits(la, lb);
 }
 
+bool dispatch_crt_whole(const Plan &p, int la, int lb, int m, int k, int n) {
+    if (p.path != GBMM_PATH_CRT || !direct_ok(p, la, lb, k)) return false;
+    return p.method != GBMM_METHOD_WINOGRAD_CRT || !wino_crt_ok(la, lb, m, k, n, p.cutoff);
+}
+
 // Upper bound of the device workspace dispatch() carves from the arena.
 size_t dispatch_ws(const Plan &p, int la, int lb, int m, int k, int n, int cn, int accumulate) {
     if (m == 0 || n == 0 || k == 0) return 0;

@@ -350,8 +350,8 @@ extern "C" gbmm_status gbmm_matmul_host(gbmm_handle h, gbmm_host_job *jobs, int3
         q.chosen_path = p.path;
         // a single-pass CRT product starts on A while B is still uploading, and the call's
         // last product returns C in entry ranges as its reconstruction finishes them
-        const bool staged = p.path == GBMM_PATH_CRT && crt_feasible(q.a_nlimbs, q.b_nlimbs, q.M) &&
-                            crt_single_pass(q.M) && ec > 0 && q.M > 0;
+        const bool staged = ec > 0 && q.M > 0 && dispatch_crt_whole(p, q.a_nlimbs, q.b_nlimbs, q.K, q.M, q.N) &&
+                            crt_single_pass(q.M);
         bool last = true;
         for (int j2 = j + 1; j2 < njobs; j2++) last = last && blocked[j2];
         // uploads: the slot's operands are free once the compute two jobs back has run
