@@ -36,6 +36,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <utility>
 #include <cmath>
@@ -2367,15 +2368,16 @@ static int g_residue_mode = -1;  // residue GEMM form: -1 by the K loop's length
 static constexpr int RES_PAIR_MIN_NK = 1 << 30;  // the pair form of the residue GEMM measured slower at every size
 static bool residue_pair(int nk) { return g_residue_mode < 0 ? nk >= RES_PAIR_MIN_NK : g_residue_mode == 1; }
 
-static int num_sms() {
-    static int n = 0;
-    if (!n) {
+int num_sms() {
+    static std::atomic<int> n{0};
+    int v = n.load(std::memory_order_relaxed);
+    if (v <= 0) {
         int dev = 0;
         cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        if (n <= 0) n = 148;
+        if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) return 148;
+        n.store(v, std::memory_order_relaxed);
     }
-    return n;
+    return v;
 }
 static size_t smem_bytes(int stages, size_t stage_bytes) { return stages * stage_bytes + SMEM_BARS + 1024 + 64; }
 

@@ -123,6 +123,9 @@ gbmm_status ltc_matmul(gbmm_handle h, const gbmm_mat &c, const gbmm_mat &a, cons
                        cudaStream_t s, bool *done);
 gbmm_status ltc_wino_leaves(gbmm_handle h, const WinoTree &t, int64_t leaves, cudaStream_t s, bool *done);
 
+// the device's SM count (crt.cu)
+int num_sms();
+
 // ---- CRT path (crt.cu) --------------------------------------------------------------
 struct crt_cache;
 crt_cache *crt_cache_create();

@@ -555,18 +555,6 @@ __global__ void __launch_bounds__(256) k_ltc_digits(DigitArgs a, int nbx) {
 
 // ---- host side ----------------------------------------------------------------------------
 static int ltc_dx(int nl) { return (4 * std::max(nl, 1) + 15) / 16 * 16; }
-static int ltc_sms() {
-    static int n = 0;
-    if (!n) {
-        int dev = 0, v = 0;
-        if (cudaGetDevice(&dev) == cudaSuccess &&
-            cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && v > 0)
-            n = v;
-        else
-            return 148;
-    }
-    return n;
-}
 
 // Tiles of a product of la x lb limb entries: columns and their split.
 static void ltc_shape(LtcArgs &a, int m, int k, int n, int la, int lb, int64_t leaves) {
@@ -624,7 +612,8 @@ size_t ltc_ws(int m, int k, int n, int la, int lb, int64_t leaves) {
 // 32^3 32 limbs 24 / 63, 64^3 16 limbs 59 / 61, 64^3 33 limbs 141 / 95, 128^3 16 limbs 330 / 90,
 // 128^3 64 limbs 1813 / 385, 256^3 8 limbs 575 / 163, 256^3 64 limbs 14002 / 2371,
 // 256 x 256 x 16 32 limbs 341 / 420 (16 columns use 16 of 128 lanes), 200 x 40 x 60 16 limbs 113 / 53.
-static int g_ltc_mode = -1;  // -1 by the estimate, 0 never, 1 wherever the shape allows it
+// -1 by the estimate, 0 never, 1 wherever the shape allows it: of this thread's calls
+static thread_local int t_ltc_mode = -1;
 static bool ltc_allowed(const LtcArgs &a, int k, int n, int64_t leaves) {
     return a.went < ((int64_t)1 << 31) && a.nitems < ((int64_t)1 << 31) && ltc_smem(a) <= 227 * 1024 &&
            leaves * k * n < ((int64_t)1 << 30);
@@ -641,18 +630,18 @@ static double ltc_tensor_us(const LtcArgs &a, int k) {
         nblk += std::min(a.dxb / 16, 4 * (jhi / 64 + 1)) - 4 * (jlo / 64);
     }
     nblk /= a.nW;
-    const double waves = (double)((a.nitems + ltc_sms() - 1) / ltc_sms());
+    const double waves = (double)((a.nitems + num_sms() - 1) / num_sms());
     return 30.0 + waves * k * (800.0 + 1.1 * nblk * a.W / 2) / 2070.0;
 }
 static double ltc_cores_us(int m, int k, int n, int la, int lb, int64_t leaves) {
     return 10.0 + (double)leaves * m * n * (k + 16.0) * la * lb / (limb_rate(la, lb, leaves * m * n) * 1e6);
 }
 bool ltc_pays(int m, int k, int n, int la, int lb, int64_t leaves) {
-    if (m < 1 || k < 1 || n < 1 || la < 1 || lb < 1 || g_ltc_mode == 0) return false;
+    if (m < 1 || k < 1 || n < 1 || la < 1 || lb < 1 || t_ltc_mode == 0) return false;
     LtcArgs a;
     ltc_shape(a, m, k, n, la, lb, leaves);
     if (!ltc_allowed(a, k, n, leaves)) return false;
-    if (g_ltc_mode == 1) return true;
+    if (t_ltc_mode == 1) return true;
     return ltc_tensor_us(a, k) < 0.95 * ltc_cores_us(m, k, n, la, lb, leaves);
 }
 
@@ -665,7 +654,7 @@ bool ltc_pays(int m, int k, int n, int la, int lb, int64_t leaves) {
 // 128^3 32 limbs cutoff 32 389 (1; 623 at 2), 256^3 64 limbs cutoff 32 3001 (1; 8560 at 3),
 // 256^3 3 limbs cutoff 32 150 (1; 232 at 3), 512^3 32 limbs cutoff 32 10614 (2; 28664 at 4).
 int ltc_wino_levels(int N, int levels, int la, int lb) {
-    if (g_ltc_mode != -1) return levels;
+    if (t_ltc_mode != -1) return levels;
     double sums = 0, best = 1e30;
     int pick = levels;
     int64_t np = 1;
@@ -715,7 +704,7 @@ static gbmm_status ltc_gemm(const LtcArgs &a, const LtcBufs &w, int64_t leaves, 
     auto kern = a.chunks ? k_ltc_gemm<true> : k_ltc_gemm<false>;
     GBMM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     LaunchScope ls_("k_ltc_gemm", s);
-    kern<<<(unsigned)std::min<int64_t>(a.nitems, ltc_sms()), LT_THREADS, smem, s>>>(tmP, a, device_error_word());
+    kern<<<(unsigned)std::min<int64_t>(a.nitems, num_sms()), LT_THREADS, smem, s>>>(tmP, a, device_error_word());
     GBMM_CUDA_TRY(cudaGetLastError());
     return GBMM_OK;
 }
@@ -824,9 +813,10 @@ gbmm_status ltc_wino_leaves(gbmm_handle h, const WinoTree &t, int64_t leaves, cu
 }  // namespace gbmm
 
 // Test hook: the limb form's products on the tensor cores by the estimate (-1, the
-// default), never (0) or wherever the shape allows it (1); returns the previous setting.
+// default), never (0) or wherever the shape allows it (1), in the calls of this thread;
+// returns its previous setting.
 extern "C" int32_t gbmmx_limb_tc(int32_t mode) {
-    const int32_t old = gbmm::g_ltc_mode;
-    gbmm::g_ltc_mode = mode < 0 ? -1 : (mode ? 1 : 0);
+    const int32_t old = gbmm::t_ltc_mode;
+    gbmm::t_ltc_mode = mode < 0 ? -1 : (mode ? 1 : 0);
     return old;
 }
