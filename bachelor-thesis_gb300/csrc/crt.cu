@@ -1304,7 +1304,7 @@ __device__ __forceinline__ long long mad_wide(int a, int b, long long c) {
 // block's last K step lie outside it and read as zeros.  GRP: a grouped launch;
 // Mod's chunk values are then read from global memory (each product has its own),
 // (the epilogue's token order holds for any sequence of N-tile counts).
-// DB: bits of a table digit (see recon_digit_bits): 32 columns are DB limbs.
+// DB: bits of a table digit (build_tables chooses): 32 columns are DB limbs.
 template <int STAGES, bool PAIR, bool GRP, int DB>
 __global__ void __launch_bounds__(REC_THREADS, 1)
     k_crt_recon(const __grid_constant__ CUtensorMap tmY, const __grid_constant__ CUtensorMap tmT, ReconArgs a0,
@@ -2631,7 +2631,7 @@ static constexpr size_t R2_SMEM =
 static gbmm_status launch_residue2(const Residue2Two &two, cudaStream_t s) {
     auto kern = k_crt_residue2<false>;
     GBMM_TRY(set_smem((const void *)kern, R2_SMEM));
-    LaunchScope ls_("k_crt_residue", s);
+    LaunchScope ls_("k_crt_residue2", s);
     const Group<Residue2Job> none{nullptr, nullptr, 0};
     return launch_pairs(kern, R2_THREADS, (int64_t)two.j[0].a.units + two.j[1].a.units, R2_SMEM, s, two, none,
                         device_error_word());
@@ -3137,7 +3137,7 @@ gbmm_status crt_group_launch(crt_group *g, const char *d_blob, cudaStream_t s, c
         memset(&none, 0, sizeof none);
         auto kern = k_crt_residue2<true>;
         GBMM_TRY(set_smem((const void *)kern, R2_SMEM));
-        LaunchScope ls_("k_crt_residue", s);
+        LaunchScope ls_("k_crt_residue2", s);
         GBMM_TRY(launch_pairs(kern, R2_THREADS, g->sres2.total, R2_SMEM, s, none,
                               group_at<Residue2Job>(d_blob, g->sres2), err));
     }

@@ -2294,6 +2294,7 @@ static bool launch_lin2(const gbmm_mat &w, const gbmm_mat &u, const gbmm_mat &v,
     // (270 us four entries per thread), 571 us segmented.
     if (blocks > 0x7FFFFFFF || L > 1024 || n >= LIN2_MAX_ENTRIES) return false;
     uint32_t *err = device_error_word();
+    LaunchScope ls_("k_mpz_lin2", s);
 // NB: blocks an SM holds by their registers.  Two, with a few spills, hide one's barriers behind the
 // other's loads (sums of 181 x 133 entries, us, one block and two: 400 limbs 66 and 56, 600 limbs
 // 98 and 74); past 640 limbs the spills cost as much.
@@ -2311,13 +2312,15 @@ static bool launch_lin2(const gbmm_mat &w, const gbmm_mat &u, const gbmm_mat &v,
 gbmm_status launch_mat_addsub(const gbmm_mat &c, const gbmm_mat &a, const gbmm_mat &b, int sub, cudaStream_t s) {
     const int64_t n = nentries(c);
     if (n == 0) return GBMM_OK;
-    LaunchScope ls_("k_mpz_addsub", s);
     const bool dense = c.rs == c.cols && a.rs == a.cols && b.rs == b.cols && vec16(c.limbs, c.ld) && vec16(a.limbs, a.ld) &&
                        vec16(b.limbs, b.ld);
-    if (n >= ADDSUB_VEC_MIN_ENTRIES && dense)
+    if (n >= ADDSUB_VEC_MIN_ENTRIES && dense) {
+        LaunchScope ls_("k_mpz_addsub_vec", s);
         k_mpz_addsub_vec<<<grid1((n + 3) / 4, 128), 128, 0, s>>>(margs(c), margs(a), margs(b), sub, n, device_error_word());
-    else if (!launch_lin2(c, a, b, 0, sub, 1, s))
+    } else if (!launch_lin2(c, a, b, 0, sub, 1, s)) {
+        LaunchScope ls_("k_mpz_addsub", s);
         k_mpz_addsub<<<grid1(n, 256), 256, 0, s>>>(margs(c), margs(a), margs(b), sub, n, device_error_word());
+    }
     GBMM_CUDA_TRY(cudaGetLastError());
     return GBMM_OK;
 }
@@ -2352,9 +2355,10 @@ gbmm_status launch_split_sizes(const gbmm_mat &x, int h, int32_t *lo, int32_t *h
 gbmm_status launch_add_shifted(const gbmm_mat &w, const gbmm_mat &u, const gbmm_mat &v, int sh, cudaStream_t s) {
     const int64_t n = nentries(w);
     if (n == 0) return GBMM_OK;
-    LaunchScope ls_("k_add_shifted", s);
-    if (!launch_lin2(w, u, v, sh, 0, 0, s))
+    if (!launch_lin2(w, u, v, sh, 0, 0, s)) {
+        LaunchScope ls_("k_add_shifted", s);
         k_add_shifted<<<grid1(n, 256), 256, 0, s>>>(margs(w), margs(u), margs(v), sh, n, device_error_word());
+    }
     GBMM_CUDA_TRY(cudaGetLastError());
     return GBMM_OK;
 }
@@ -2378,7 +2382,7 @@ gbmm_status launch_mpz_mulops(const gbmm_mat &w, const gbmm_mat &u, const gbmm_m
     const int64_t ul = std::min<int64_t>(u.nlimbs, (int64_t)w.nlimbs + 1), vl = std::min<int64_t>(v.nlimbs, (int64_t)w.nlimbs + 1);
     const size_t words = (size_t)sm_stride((int)ul) + sm_stride((int)vl);
     const int nt = ul * vl > MPZ_DIRECT ? sm_threads(words + 2) : 0;  // two words an entry of static shared memory
-    LaunchScope ls_("k_mpz_mulops", s);
+    LaunchScope ls_(nt ? "k_mpz_mulops_sm" : "k_mpz_mulops", s);
     if (nt) {
         const size_t smem = nt * words * 4;
         const int vu = u.rs == u.cols && vec16(u.limbs, u.ld), vv = v.rs == v.cols && vec16(v.limbs, v.ld);
@@ -2665,12 +2669,13 @@ static int64_t pow7(int d) {
 }
 
 // by the limbs of an entry: LAUNCH(segments, entries of a block)
+constexpr int LIN_MAX_LIMBS = LIN_SEG * 68;
 #define LIN_DISPATCH(cap_, LAUNCH, SERIAL)                  \
     do {                                                    \
         if ((cap_) <= LIN_SEG * 12) LAUNCH(12, 32);         \
         else if ((cap_) <= LIN_SEG * 17) LAUNCH(17, 32);    \
         else if ((cap_) <= LIN_SEG * 34) LAUNCH(34, 16);    \
-        else if ((cap_) <= LIN_SEG * 68) LAUNCH(68, 8);     \
+        else if ((cap_) <= LIN_MAX_LIMBS) LAUNCH(68, 8);    \
         else SERIAL;                                        \
     } while (0)
 
@@ -2679,9 +2684,9 @@ gbmm_status launch_wino_sums(const WinoTree &t, int d, cudaStream_t s) {
     const int h = t.N >> d;
     const int64_t n = np * h * h, blocks = 2 * ((n + 7) / 8);  // at most
     uint32_t *err = device_error_word();
-    LaunchScope ls_("k_wino_sums", s);
     // the sums' planes hold every limb of the quadrants they are formed from
     const int cap = std::max(t.capSA, t.capSB);
+    LaunchScope ls_(cap <= LIN_MAX_LIMBS ? "k_wino_sums" : "k_wino_sums_serial", s);
     if (blocks > 0x7FFFFFFF) return set_error(GBMM_ERR_UNSUPPORTED, "winograd sums: too many entries");
 #define LAUNCH_S(MS, EX)                                                                                                       \
     k_wino_sums<LIN_SEG, MS, EX><<<(unsigned)(2 * ((n + EX - 1) / EX)), dim3(EX, (unsigned)std::max(1, (cap + LIN_SEG - 1) / LIN_SEG)), 0, \
@@ -2697,8 +2702,8 @@ gbmm_status launch_wino_combine(const WinoTree &t, int d, cudaStream_t s) {
     const int h = t.N >> d;
     const int64_t n = np * h * h, blocks = (n + 7) / 8;  // at most
     uint32_t *err = device_error_word();
-    LaunchScope ls_("k_wino_combine", s);
     const int cap = std::max(t.capP, d == 1 ? t.C.nlimbs : 0);
+    LaunchScope ls_(cap <= LIN_MAX_LIMBS ? "k_wino_combine" : "k_wino_combine_serial", s);
     if (blocks > 0x7FFFFFFF) return set_error(GBMM_ERR_UNSUPPORTED, "winograd combinations: too many entries");
 #define LAUNCH_C(MS, EX)                                                                                                     \
     k_wino_combine<LIN_SEG, MS, EX><<<(unsigned)((n + EX - 1) / EX), dim3(EX, (unsigned)std::max(1, (cap + LIN_SEG - 1) / LIN_SEG)), 0, \

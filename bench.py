@@ -470,11 +470,16 @@ def crt_params(bits_a, bits_b, k):
 # from a one-pass ncu capture of this workload (dram__bytes_read.sum +
 # dram__bytes_write.sum; profiles/crt_512x512x512_4096b_dram_bytes.md).
 NCU_DRAM_BYTES_512_4096 = {
-    "k_crt_residue": 274.133248e6 + 1026.769664e6,
+    "k_crt_residue2": 274.133248e6 + 1026.769664e6,
     "k_crt_product": 1082.190080e6 + 511.279104e6,
     "k_crt_recon": 558.553344e6 + 242.209024e6,
 }
 FIXED_POINT_COLUMNS = 14  # reconstruction columns that carry the 2^96 / p_i weights
+
+
+def wino_levels_run(prof):
+    """Levels of Winograd's tree: one launch of the sums each, by either kernel."""
+    return sum(prof.get(k, (0, 0.0))[0] for k in ("k_wino_sums", "k_wino_sums_serial"))
 
 
 def kernel_roofline(kname, klaunch, kms, W, args, K, M, N, nl, cn, peaks, prof, macpk=None):
@@ -492,7 +497,7 @@ def kernel_roofline(kname, klaunch, kms, W, args, K, M, N, nl, cn, peaks, prof, 
     if kname == "k_crt_product":
         flops = 2.0 * K * M * N * 4 * P
         note = f"4 digit-pair GEMMs per modulus, P={P} moduli, {K}x{M}x{N}"
-    elif kname == "k_crt_residue":
+    elif kname in ("k_crt_residue", "k_crt_residue2"):
         per_product = klaunch / max(1, prof.get("k_crt_product", (klaunch, 0.0))[0])  # both operands, or one each
         flops = 2.0 * (K * M + M * N) / max(1.0, per_product) * dx * 2 * P
         note = f"entries x {dx} digits x {2 * P} table columns, both operands over {per_product:.0f} launch(es)"
@@ -501,7 +506,7 @@ def kernel_roofline(kname, klaunch, kms, W, args, K, M, N, nl, cn, peaks, prof, 
         note = f"entries x {2 * P} moduli digits x {FIXED_POINT_COLUMNS + Dout} output columns"
     elif kname == "k_ltc_gemm":
         steps = max(1, args.profile_steps)
-        levels = prof.get("k_wino_sums", (0, 0.0))[0] // steps
+        levels = wino_levels_run(prof) // steps
         macs = winograd_leaf_macs(K, levels, nl, nl) if levels else K * M * N * nl * nl
         flops = 32.0 * macs * steps / max(1, klaunch)
         note = "16 byte-digit MACs per 32-bit limb MAC of the products, no padding counted"
@@ -619,7 +624,7 @@ def measure_limb_path(gbmm, h, dA, dB, dC_crt, K, M, N, nl, args, flush, stream,
         gbmm.profile(False)
         del dL
         # the recursion depth the library chose: one launch of the sums per level
-        levels = prof.get("k_wino_sums", (0, 0.0))[0] if method == gbmm.METHOD_WINOGRAD else 0
+        levels = wino_levels_run(prof) if method == gbmm.METHOD_WINOGRAD else 0
         lk = next(k for k in ("k_ltc_gemm", "k_wino_leaves", "k_limb_matmul") if k in prof)
         lms = prof[lk][1]
         macs = winograd_leaf_macs(K, levels, nl, nl) if levels else K * M * N * nl * nl
@@ -969,12 +974,12 @@ def run_limb_kernels(args, W, world, rank, local):
         m.upload(Lp, Sp)
         mats[key] = m
     w = gbmm.DeviceMatrix(R, Cc, 33)
-    rec("mpz_add", "k_mpz_addsub", timed(lambda: gbmm.mpz_add(w, mats["u"], mats["v"])), E * (4 * (32 + 32 + 33) + 12))
-    rec("mpz_sub", "k_mpz_addsub", timed(lambda: gbmm.mpz_sub(w, mats["u"], mats["v"])), E * (4 * (32 + 32 + 33) + 12))
+    rec("mpz_add", "k_mpz_addsub_vec", timed(lambda: gbmm.mpz_add(w, mats["u"], mats["v"])), E * (4 * (32 + 32 + 33) + 12))
+    rec("mpz_sub", "k_mpz_addsub_vec", timed(lambda: gbmm.mpz_sub(w, mats["u"], mats["v"])), E * (4 * (32 + 32 + 33) + 12))
     p = gbmm.DeviceMatrix(R, Cc, 33)
-    rec("mpz_mul", "k_mpz_mulops", timed(lambda: gbmm.mpz_mul(p, mats["s"], mats["t"])),
+    rec("mpz_mul", "k_mpz_mulops_sm", timed(lambda: gbmm.mpz_mul(p, mats["s"], mats["t"])),
         E * (4 * (16 + 16 + 32) + 12), 16 * 16 * E)
-    rec("mpz_addmul", "k_mpz_mulops", timed(lambda: gbmm.mpz_addmul(p, mats["s"], mats["t"])),
+    rec("mpz_addmul", "k_mpz_mulops_sm", timed(lambda: gbmm.mpz_addmul(p, mats["s"], mats["t"])),
         E * (4 * (16 + 16 + 33 + 33) + 16), 16 * 16 * E)
     if rank != 0:
         return 0
