@@ -2272,6 +2272,7 @@ static inline unsigned grid1(int64_t n, int bs) { return (unsigned)((n + bs - 1)
 // CTA size of the on-chip mpn products for `words` shared-memory words per
 // operand: the largest of 128, 64, 32 whose staging fits, 0 when none does
 constexpr size_t MPN_SM_MAX_BYTES = 200 * 1024;
+constexpr size_t SM_SHARED_BYTES = 228 * 1024;  // an SM's; a CTA takes 1 KB more than it asked for
 static int sm_threads(size_t words) {
     for (int nt = 128; nt >= 32; nt >>= 1)
         if ((size_t)nt * words * 4 <= MPN_SM_MAX_BYTES) return nt;
@@ -2915,8 +2916,14 @@ extern "C" gbmm_status gbmm_mpn_mul_basecase(uint32_t *rp, const uint32_t *up, i
     }
     const int vu = vec16(up, ld), vv = vec16(vp, ld);
     const size_t words8 = (size_t)sm_stride_b<8>(un) + sm_stride_b<8>(vn);
-    const bool by8 = sm_block(un, vn) == 8 && (size_t)nt * words8 * 4 <= MPN_SM_MAX_BYTES;
-    const size_t smem = (size_t)nt * (by8 ? words8 : (size_t)sm_stride(un) + sm_stride(vn)) * 4;
+    const size_t words4 = (size_t)sm_stride(un) + sm_stride(vn);
+    // blocks of 8 pad the strings further; where that costs an SM a CTA of a grid that fills them,
+    // blocks of 4 are faster (40000 products, us by 8 and by 4: 96 x 41 limbs 67 and 56, 176 x 41
+    // 138 and 126; 104 x 48, two CTAs either way, 74 and 79)
+    auto ctas = [&](size_t words) { return std::min<int64_t>(5, SM_SHARED_BYTES / (nt * words * 4 + 1024)); };
+    const bool by8 = sm_block(un, vn) == 8 && (size_t)nt * words8 * 4 <= MPN_SM_MAX_BYTES &&
+                     (ctas(words8) == ctas(words4) || (nb + nt - 1) / nt <= num_sms() * ctas(words8));
+    const size_t smem = (size_t)nt * (by8 ? words8 : words4) * 4;
     LaunchScope ls_("k_mpn_mul_basecase_sm", as_stream(stream));
 #define BASECASE_SM(NT_, B_)                                                                                    \
     do {                                                                                                        \
