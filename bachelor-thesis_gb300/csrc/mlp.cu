@@ -262,6 +262,17 @@ int model_choose(gbmm_handle h, int m, int k, int n, int la, int lb) {
     int best = -1;
     for (int o = 0; o < NO; o++) {
         if (!plan_admissible(o, m, k, n, la, lb) || md->head_samples[o] < MIN_HEAD_SAMPLES) continue;
+        // Winograd's tree keeps 7/8 of the product's multiplications a level, so its time is bounded
+        // by the plain product's, whose head knows far more shapes: none of 158 trees timed on
+        // 448 uneven products was below the bound, and small rectangular ones are up to six
+        // times above it, which their head misses now and then
+        const Plan p = plan_of(o);
+        if (p.path == GBMM_PATH_LIMB && p.method == GBMM_METHOD_WINOGRAD &&
+            md->head_samples[GBMM_PLAN_LIMB_NAIVE] >= MIN_HEAD_SAMPLES) {
+            float bound = y[GBMM_PLAN_LIMB_NAIVE];
+            for (int d = std::min(std::min(m, k), n); d > p.cutoff; d /= 2) bound -= 0.19265f;  // log2(8/7)
+            y[o] = std::max(y[o], bound);
+        }
         if (best < 0 || y[o] < y[best]) best = o;
     }
     const int base = heuristic_plan(m, k, n, la, lb);
