@@ -1650,8 +1650,8 @@ extern "C" gbmm_status gbmm_mpn_mul(gbmm_handle h, uint32_t *rp, const uint32_t 
     if (un < vn || vn < 1) return set_error(GBMM_ERR_INVALID, "mpn_mul needs un >= vn >= 1");
     const int s = un >> 1, n = un - s, t = vn - n;
     // The on-chip basecase beats the on-chip Toom-2.2 wherever it fits (measured on
-    // 2^16 to 2^18 operand pairs: Toom at 0.70x its speed at 64 limbs, 0.80x at 128,
-    // 0.86x at 192): the Karatsuba split's additions cost more than the quarter of
+    // 2^16 to 2^18 operand pairs: Toom at 0.63x its speed at 64 limbs, 0.68x at 128,
+    // 0.72x at 192): the Karatsuba split's additions cost more than the quarter of
     // the MACs it saves.  Longer balanced operands take Toom-2.2.
     const bool toom = !mpn_basecase_on_chip(un, vn) && 4 * un < 5 * vn && 0 < t && t <= s;
     if (!toom) return gbmm_mpn_mul_basecase(rp, up, un, vp, vn, ld, nb, h->stream);

@@ -123,8 +123,8 @@ __device__ __forceinline__ uint64_t sdesc_hankel(uint32_t saddr) {
            ((uint64_t)1 << 46);
 }
 
-// What bounds it: the tensor pipe (an MMA of 256 columns, M = 128, K = 16 takes 128
-// clocks) beside the 16 KB of plain rows each K step brings into shared memory.  Every
+// What bounds it: the tensor pipe (83 % busy at 256^3, 2048 bits; an MMA of 256 columns, M = 128,
+// K = 16 takes 128 clocks) beside the 16 KB of plain rows each K step brings into shared memory.  Every
 // MMA covers the tile's W columns: restricting an MMA to the columns that its digits
 // reach halves the multiplications, but every change of the column range drains the
 // pipe (measured at 256^3, 2048 bits: 4.5 ms with exact ranges, 3.7 ms with one range

@@ -302,11 +302,14 @@ __device__ __forceinline__ void tmem_relinquish_pair() {
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
-// Arrive on an mbarrier of another CTA of the cluster.  What it hands over is tensor
-// memory, whose reads tcgen05.wait::ld and tcgen05.fence have ordered, or shared memory of this
-// CTA behind a proxy fence; a release spelled out at cluster scope would also wait for
-// the thread's global accesses (1300 clocks an arrival in the converters of k_crt_residue2, a
-// fifth of the time of the pairs' epilogues).
+// Arrive on an mbarrier of another CTA of the cluster, for hand-overs whose order does not rest
+// on the arrival's own release: the caller has ordered its side before it, tensor-memory reads
+// by tcgen05.wait::ld and tcgen05.fence::before_thread_sync, writes to its own shared memory
+// that the pair's MMA (the async proxy) will read by fence.proxy.async in every writing thread
+// and a warp sync; the waiting side issues tcgen05.fence::after_thread_sync.  It is not for
+// generic-proxy data that the other CTA's threads read: that takes a release at cluster
+// scope, which also waits for the thread's global accesses (1300 clocks an arrival in the
+// converters of k_crt_residue2, a fifth of the time of the pairs' epilogues).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster) : "memory");
 }
