@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(256) k_mpn_addsub_n_vec(uint4 *rp, const uint4
 // batches with at least this many operands take the one-thread-per-operand kernel
 constexpr int64_t ADDSUB_SERIAL_MIN_OPS = 16384;
 // ... and with four per thread when that still leaves eight warps per SM
-constexpr int64_t ADDSUB_VEC_MIN_OPS = 152 * 8 * 32 * 4;
+static int64_t addsub_vec_min_ops() { return (int64_t)num_sms() * 8 * 32 * 4; }
 
 // ---- mul_1 family: one thread per operand, serial over limbs (coalesced) -----------
 template <int OP>  // 0 mul_1, 1 addmul_1, 2 submul_1
@@ -1047,7 +1047,7 @@ __global__ void k_mpz_addsub(MatArgs W, MatArgs U, MatArgs V, int sub, int64_t c
 // in the same pass.  When w and the product have opposite signs the merge is a
 // two's complement subtraction; a final borrow means |uv| > |w| and the
 // written limbs are negated in place.
-__device__ __forceinline__ void mulops_entry(const MatArgs &W, const MatArgs &U, const MatArgs &V, int op, int64_t e, int su,
+__device__ __forceinline__ void mulops_one(const MatArgs &W, const MatArgs &U, const MatArgs &V, int op, int64_t e, int su,
                                              int sv, int sw, uint32_t *err) {
     const int64_t iw = ent(W, e);
     const int un = min(iabs_d(su), U.nlimbs), vn = min(iabs_d(sv), V.nlimbs);
@@ -1122,7 +1122,7 @@ __device__ __forceinline__ void mulops_entry(const MatArgs &W, const MatArgs &U,
 __global__ void k_mpz_mulops(MatArgs W, MatArgs U, MatArgs V, int op, int64_t count, uint32_t *err) {
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= count) return;
-    mulops_entry(W, U, V, op, e, U.sizes[ent(U, e)], V.sizes[ent(V, e)], op == 0 ? 0 : W.sizes[ent(W, e)], err);
+    mulops_one(W, U, V, op, e, U.sizes[ent(U, e)], V.sizes[ent(V, e)], op == 0 ? 0 : W.sizes[ent(W, e)], err);
 }
 
 // The same operations with the operands staged on chip (as k_mpn_mul_basecase_sm): a CTA
@@ -1149,7 +1149,7 @@ constexpr int MPZ_DIRECT = 8;
 // out of line: its registers would cost the staged product's loop 4 % (700 x 700 limbs)
 __device__ __noinline__ void mulops_short(MatArgs W, MatArgs U, MatArgs V, int op, int64_t e, int su, int sv, int sw,
                                           uint32_t *err) {
-    mulops_entry(W, U, V, op, e, su, sv, sw, err);
+    mulops_one(W, U, V, op, e, su, sv, sw, err);
 }
 
 // Limbs [0, n) of entries e0 .. e0 + NT - 1 into dst[t * SS + i], zeros above an entry's size
@@ -2515,7 +2515,7 @@ double limb_rate(int la, int lb, int64_t entries) {
     if (cfg.G == 1) return 1.9 * std::min(1.0, entries / 41000.0);
     const bool thin = cfg.thinA || cfg.thinB;
     const double rate = cfg.R == 8 ? 4.8 : cfg.R == 4 ? (thin ? 2.7 : 3.4) : (thin ? 1.4 : 1.85);
-    return rate * std::min(1.0, (double)entries * cfg.Gp / (152.0 * 512));
+    return rate * std::min(1.0, (double)entries * cfg.Gp / (num_sms() * 512.0));
 }
 
 static size_t mm_smem(const MMCfg &c) {
@@ -2765,7 +2765,7 @@ static gbmm_status addsub_n_entry(uint32_t *rp, const uint32_t *up, const uint32
     GBMM_TRY(check_batch(rp, up, ld, nb, n));
     if (!vp || !cy) return set_error(GBMM_ERR_INVALID, "null pointer");
     if (nb == 0) return GBMM_OK;
-    if (nb >= ADDSUB_VEC_MIN_OPS && vec16(rp, ld) && vec16(up, ld) && vec16(vp, ld) && vec16(cy, 4)) {
+    if (nb >= addsub_vec_min_ops() && vec16(rp, ld) && vec16(up, ld) && vec16(vp, ld) && vec16(cy, 4)) {
         LaunchScope ls_("k_mpn_addsub_n_vec", as_stream(stream));
         k_mpn_addsub_n_vec<SUB><<<grid1(nb / 4 + nb % 4, 256), 256, 0, as_stream(stream)>>>(
             (uint4 *)rp, (const uint4 *)up, (const uint4 *)vp, n, ld / 4, nb, (uint4 *)cy);
