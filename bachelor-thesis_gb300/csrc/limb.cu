@@ -1048,19 +1048,19 @@ __global__ void k_mpz_addsub(MatArgs W, MatArgs U, MatArgs V, int sub, int64_t c
 // two's complement subtraction; a final borrow means |uv| > |w| and the
 // written limbs are negated in place.
 __device__ __forceinline__ void mulops_one(const MatArgs &W, const MatArgs &U, const MatArgs &V, int op, int64_t e, int su,
-                                             int sv, int sw, uint32_t *err) {
+                                           int sv, int sw, uint32_t *err) {
     const int64_t iw = ent(W, e);
     const int un = min(iabs_d(su), U.nlimbs), vn = min(iabs_d(sv), V.nlimbs);
     const uint32_t *up = U.limbs + ent(U, e), *vp = V.limbs + ent(V, e);
     uint32_t *wp = W.limbs + iw;
     const int64_t ws = W.ld;
-    const int wn = iabs_d(sw);
+    const int cap = W.nlimbs;
+    const int wn = min(iabs_d(sw), cap);
     int pneg = (su < 0) ^ (sv < 0);
     if (op == 2) pneg ^= 1;
     const int pn = (un && vn) ? un + vn : 0;
     const int subtract = wn && pn && ((sw < 0) != pneg);
     const int rn = (pn > wn ? pn : wn) + (subtract ? 0 : 1);
-    const int cap = W.nlimbs;
     // Result limbs [0, rn).  Limbs of w beyond wn are zero by invariant.  Limbs
     // at t >= cap are not stored; hi_nz / hi_ones remember whether any of them
     // is nonzero / all of them are all-ones, which decides overflow below.
