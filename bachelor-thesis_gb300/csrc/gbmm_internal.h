@@ -86,8 +86,8 @@ gbmm_status launch_split_sizes(const gbmm_mat &x, int h, int32_t *lo, int32_t *h
 gbmm_status launch_add_shifted(const gbmm_mat &w, const gbmm_mat &u, const gbmm_mat &v, int sh, cudaStream_t s);
 // whether the per-entry product kernel handles la x lb limb entries
 bool limb_kernel_fits(int la, int lb);
-// measured rate of that kernel on long sums, in 10^12 32-bit MAC/s, for `entries` results
-double limb_rate(int la, int lb, int64_t entries);
+// its estimated time in microseconds for `entries` sums of k products (1e30: it does not take them)
+double limb_us(int la, int lb, int k, int64_t entries);
 // whether the batched basecase product stages un x vn limb operands on chip
 bool mpn_basecase_on_chip(int un, int vn);
 
@@ -117,7 +117,10 @@ gbmm_status launch_wino_combine(const WinoTree &t, int d, cudaStream_t s);
 // handle's workspace has no room
 int ltc_wino_levels(int N, int levels, int la, int lb);
 bool ltc_wino_fits(int hh, int la, int lb, int64_t leaves, size_t room);
-bool ltc_pays(int m, int k, int n, int la, int lb, int64_t leaves);
+// (slack: also when their estimate is up to that factor above the per-entry kernel's; for
+// leaves above the cutoff, whose alternative is a deeper tree)
+constexpr double LTC_SHALLOW = 1.25;
+bool ltc_pays(int m, int k, int n, int la, int lb, int64_t leaves, double slack = 1.0);
 size_t ltc_ws(int m, int k, int n, int la, int lb, int64_t leaves);
 gbmm_status ltc_matmul(gbmm_handle h, const gbmm_mat &c, const gbmm_mat &a, const gbmm_mat &b, int accumulate,
                        cudaStream_t s, bool *done);

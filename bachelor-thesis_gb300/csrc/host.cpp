@@ -968,6 +968,7 @@ static int64_t pow7_h(int l) {
 // launch, then the combinations of every level bottom up (kernels in limb.cu).
 // Same products and sums as rec_winograd down to its leaves, so the same exact result.
 gbmm_status rec_winograd_bf(RecCtx &c, gbmm_mat C, gbmm_mat A, gbmm_mat B, int N, int levels) {
+    const int full = levels;
     if (c.h->limb_tc) {
         // fewer levels where that is faster on the tensor cores and the workspace, which was
         // reserved for all of them, holds the larger leaves' operands
@@ -1005,7 +1006,8 @@ gbmm_status rec_winograd_bf(RecCtx &c, gbmm_mat C, gbmm_mat A, gbmm_mat B, int N
     if (st == GBMM_OK) {
         bool done = false;
         const int hl = N >> levels;
-        if (c.h->limb_tc && ltc_pays(hl, hl, hl, t.capSA, t.capSB, np)) st = ltc_wino_leaves(c.h, t, np, c.s, &done);
+        if (c.h->limb_tc && ltc_pays(hl, hl, hl, t.capSA, t.capSB, np, levels < full ? LTC_SHALLOW : 1.0))
+            st = ltc_wino_leaves(c.h, t, np, c.s, &done);
         if (st == GBMM_OK && !done) st = launch_wino_leaves(t, c.s);
     }
     for (int d = levels; d >= 1 && st == GBMM_OK; d--) st = launch_wino_combine(t, d, c.s);
@@ -1397,10 +1399,11 @@ size_t limb_tc_extra(const Plan &p, int la, int lb, int m, int k, int n) {
     size_t x = 0;
     if (ltc_pays(m, k, n, la + up, lb + up, 1)) x = ltc_ws(m, k, n, la + up, lb + up, 1) + 4096;
     if (p.method == GBMM_METHOD_WINOGRAD && m == k && k == n) {
-        int L = levels_for(m, p.cutoff);
-        if (L >= 1 && L <= WINO_MAX_LEVELS) L = ltc_wino_levels(m, L, la + 1, lb + 1);
+        const int full = levels_for(m, p.cutoff);
+        const int L = full >= 1 && full <= WINO_MAX_LEVELS ? ltc_wino_levels(m, full, la + 1, lb + 1) : full;
         const int hl = m >> L;
-        if (L >= 1 && L <= WINO_MAX_LEVELS && ltc_pays(hl, hl, hl, la + 1, lb + 1, pow7_h(L))) {
+        if (L >= 1 && L <= WINO_MAX_LEVELS &&
+            ltc_pays(hl, hl, hl, la + 1, lb + 1, pow7_h(L), L < full ? LTC_SHALLOW : 1.0)) {
             const size_t per = ltc_ws(hl, hl, hl, la + 1, lb + 1, 1) + 4096;
             x = std::max(x, per * (size_t)std::min<int64_t>(pow7_h(L), std::max<int64_t>(64, (int64_t)(WINO_BYTES / per))));
         }

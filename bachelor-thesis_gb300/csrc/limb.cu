@@ -2508,14 +2508,29 @@ bool limb_kernel_fits(int la, int lb) {
     return choose_mm(la, lb, cfg);
 }
 
-double limb_rate(int la, int lb, int64_t entries) {
-    MMCfg cfg;
-    if (!choose_mm_for(la, lb, entries, cfg)) return 1.0;
-    // one thread per entry: it takes about 40 thousand entries to fill the GPU
-    if (cfg.G == 1) return 1.9 * std::min(1.0, entries / 41000.0);
+// Rates in 10^12 32-bit MAC/s over whole blocks of limbs, and terms k that an entry's set-up and
+// epilogue cost, fitted to 785 products (1 to 4000 rows and columns, 1 to 600 terms, 1 to 176
+// limbs); long sums of square operands run at up to 1.4 times these.
+double limb_us(int la, int lb, int k, int64_t entries) {
+    MMCfg cfg, many;
+    if (!choose_mm(la, lb, many) || !choose_mm_for(la, lb, entries, cfg)) return 1e30;
     const bool thin = cfg.thinA || cfg.thinB;
-    const double rate = cfg.R == 8 ? 4.8 : cfg.R == 4 ? (thin ? 2.7 : 3.4) : (thin ? 1.4 : 1.85);
-    return rate * std::min(1.0, (double)entries * cfg.Gp / (num_sms() * 512.0));
+    const double fill = std::min(1.0, (double)entries * cfg.Gp / (num_sms() * 512.0));
+    double rate, terms = 16.0, pa = cfg.thinA ? la : cfg.La, pb = cfg.thinB ? lb : cfg.Lb;
+    if (many.G == 1) {
+        // one thread per entry, which takes about 40 thousand entries to fill the GPU, or few entries
+        // in blocks of 2 x 2 limbs
+        rate = cfg.G == 1 ? 1.9 * std::min(1.0, entries / 41000.0) : (thin ? 1.4 : 1.85) * fill;
+        terms = 6.0;
+        pa = la;
+        pb = lb;
+    } else if (cfg.R == 8) {
+        rate = 4.56 * fill;
+        terms = 9.0;
+    } else {
+        rate = (cfg.R == 4 ? (thin ? 2.15 : 2.4) : (thin ? 1.05 : 1.3)) * fill;
+    }
+    return 10.0 + (double)entries * (k + terms) * pa * pb / (rate * 1e6);
 }
 
 static size_t mm_smem(const MMCfg &c) {

@@ -605,10 +605,13 @@ size_t ltc_ws(int m, int k, int n, int la, int lb, int64_t leaves) {
 }
 
 // Estimated time of both forms in microseconds; the tensor form is taken when it is
-// faster.  Tensor form: 30 us of launches and pipeline fill, then per tile and term k 800
+// faster.  Tensor form: 23.5 us of launches and pipeline fill, then per tile and term k 800
 // clocks (the Hankel operand's hand-over) plus the MMAs of the chunks the tile reads, over the
-// tiles one SM runs.  CUDA cores: 10 us plus the multiplications at the rate of the
-// per-entry kernel's block edge (limb_rate), less on short sums.  Measured (us, CUDA cores / tensor):
+// tiles one SM runs, and the finish: 0.215 us a limb of an entry (one thread takes them one after
+// the other) or its traffic at 7.4 TB/s of L2.  CUDA cores: limb_us.  Over 1285 products of 1 to 600
+// terms the choice costs 1.5 % against the faster form of each, and five take more than 1.08 times the CUDA
+// cores' time (1.17 at most; with a constant for the finish 72, 2.5 at most: 16 x 20 x 64 entries of
+// 128 and 16 limbs 28 on the CUDA cores, 65 here).  Measured (us, CUDA cores / tensor):
 // 32^3 32 limbs 24 / 63, 64^3 16 limbs 59 / 61, 64^3 33 limbs 141 / 95, 128^3 16 limbs 330 / 90,
 // 128^3 64 limbs 1813 / 385, 256^3 8 limbs 575 / 163, 256^3 64 limbs 14002 / 2371,
 // 256 x 256 x 16 32 limbs 341 / 420 (16 columns use 16 of 128 lanes), 200 x 40 x 60 16 limbs 113 / 53.
@@ -631,24 +634,23 @@ static double ltc_tensor_us(const LtcArgs &a, int k) {
     }
     nblk /= a.nW;
     const double waves = (double)((a.nitems + num_sms() - 1) / num_sms());
-    return 30.0 + waves * k * (800.0 + 1.1 * nblk * a.W / 2) / 2070.0;
+    const double limbs = a.T / 4;
+    return 23.5 + waves * k * (800.0 + 1.1 * nblk * a.W / 2) / 2070.0 + 0.215 * limbs + a.went * limbs * 16 / 7.4e6;
 }
-static double ltc_cores_us(int m, int k, int n, int la, int lb, int64_t leaves) {
-    return 10.0 + (double)leaves * m * n * (k + 16.0) * la * lb / (limb_rate(la, lb, leaves * m * n) * 1e6);
-}
-bool ltc_pays(int m, int k, int n, int la, int lb, int64_t leaves) {
+bool ltc_pays(int m, int k, int n, int la, int lb, int64_t leaves, double slack) {
     if (m < 1 || k < 1 || n < 1 || la < 1 || lb < 1 || t_ltc_mode == 0) return false;
     LtcArgs a;
     ltc_shape(a, m, k, n, la, lb, leaves);
     if (!ltc_allowed(a, k, n, leaves)) return false;
     if (t_ltc_mode == 1) return true;
-    return ltc_tensor_us(a, k) < 0.95 * ltc_cores_us(m, k, n, la, lb, leaves);
+    return ltc_tensor_us(a, k) < slack * limb_us(la, lb, k, leaves * m * n);
 }
 
 // Levels of a Winograd tree (1 .. levels, the depth that the cutoff gives) whose sums,
 // leaf products and combinations together are estimated fastest.  Each level has 7/8 of the
 // multiplications, but leaves of fewer than 128 columns leave lanes of the MMAs idle, and
-// the sums and combinations of a level take about 16 us plus their traffic; so on the
+// the sums and combinations of a level take about 16 us plus their traffic; above the
+// cutoff leaves count whose estimate is within LTC_SHALLOW of the CUDA cores'.  So on the
 // tensor cores the tree usually stops at blocks of 64 or more, on the CUDA cores at the
 // cutoff.  Products, us (levels, and before at the cutoff's depth): 64^3 16 limbs cutoff 16 98 (1; 151 at 2),
 // 128^3 32 limbs cutoff 32 389 (1; 623 at 2), 256^3 64 limbs cutoff 32 3001 (1; 8560 at 3),
@@ -664,8 +666,9 @@ int ltc_wino_levels(int N, int levels, int la, int lb) {
         sums += 16.0 + np * e * 4.0 * 19.0 * (la + lb) / 4e6;
         LtcArgs a;
         ltc_shape(a, hh, hh, hh, la, lb, 7 * np);
-        double t = d == levels ? ltc_cores_us(hh, hh, hh, la, lb, 7 * np) : 1e30;
-        if (hh <= ltc_kmax(la, lb) && ltc_pays(hh, hh, hh, la, lb, 7 * np)) t = std::min(t, ltc_tensor_us(a, hh));
+        double t = d == levels ? limb_us(la, lb, hh, 7 * np * hh * hh) : 1e30;
+        if (hh <= ltc_kmax(la, lb) && ltc_pays(hh, hh, hh, la, lb, 7 * np, d < levels ? LTC_SHALLOW : 1.0))
+            t = std::min(t, ltc_tensor_us(a, hh));
         if (sums + t < best) {
             best = sums + t;
             pick = d;
