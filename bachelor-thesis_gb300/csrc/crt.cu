@@ -3152,30 +3152,38 @@ gbmm_status crt_group_launch(crt_group *g, const char *d_blob, cudaStream_t s, c
                             group_at<ProductJob>(d_blob, g->sprod), err));
         GBMM_CUDA_TRY(cudaGetLastError());
     }
-    // the products with post steps first: their shifted adds then run on s2 while
-    // the other reconstructions do
-    for (int f = 1; f >= 0; f--) {
-        for (int d = 1; d >= 0; d--) {
-            const crt_group::Sect &sec = g->srec[2 * f + d];
-            if (!sec.n) continue;
-            ReconArgs none;
-            memset(&none, 0, sizeof none);
-            auto kern = d ? k_crt_recon<REC_STAGES_PAIR, true, true, 8> : k_crt_recon<REC_STAGES_PAIR, true, true, 7>;
-            GBMM_TRY(set_smem((const void *)kern, g->smem_rec));
-            LaunchScope ls_("k_crt_recon", s);
-            GBMM_TRY(launch_pairs(kern, REC_THREADS, sec.total, g->smem_rec, s, zmap, zmap, none,
-                                  group_at<ReconJob>(d_blob, sec), err));
-        }
-        if (f == 1 && !g->post.empty()) {
-            cudaStream_t sp = s;
-            if (s2 && ev) {
-                GBMM_CUDA_TRY(cudaEventRecord(ev, s));
-                GBMM_CUDA_TRY(cudaStreamWaitEvent(s2, ev, 0));
-                sp = s2;
-            }
-            for (auto &fn : g->post) GBMM_TRY(fn(sp));
-        }
+    // The products with post steps first: their shifted adds then run on s2 while
+    // the other reconstructions do.  With s2 the two table forms run side by side too: an entry's N
+    // tiles follow one another, so on few entries a launch takes as long as the longest entry
+    // however little it has to do (9 products of up to 36 rows and 13489 bits, us: 288 one after the
+    // other, 233 side by side; 24 of up to 150 rows and 15092 bits 808 and 692).
+    const bool side = s2 && ev;
+    if (side && (g->srec[0].n || g->srec[2].n) && (g->srec[1].n || g->srec[3].n)) {
+        GBMM_CUDA_TRY(cudaEventRecord(ev, s));
+        GBMM_CUDA_TRY(cudaStreamWaitEvent(s2, ev, 0));
     }
+    auto recon = [&](int f, int d, cudaStream_t rs) -> gbmm_status {
+        const crt_group::Sect &sec = g->srec[2 * f + d];
+        if (!sec.n) return GBMM_OK;
+        ReconArgs none;
+        memset(&none, 0, sizeof none);
+        auto kern = d ? k_crt_recon<REC_STAGES_PAIR, true, true, 8> : k_crt_recon<REC_STAGES_PAIR, true, true, 7>;
+        GBMM_TRY(set_smem((const void *)kern, g->smem_rec));
+        LaunchScope ls_("k_crt_recon", rs);
+        return launch_pairs(kern, REC_THREADS, sec.total, g->smem_rec, rs, zmap, zmap, none, group_at<ReconJob>(d_blob, sec),
+                            err);
+    };
+    // base-128 tables beside base-256 ones, on s2 (where there are both)
+    const cudaStream_t s7 = side && (g->srec[1].n || g->srec[3].n) ? s2 : s;
+    GBMM_TRY(recon(1, 1, s));
+    GBMM_TRY(recon(1, 0, s7));
+    if (side && !g->post.empty()) GBMM_CUDA_TRY(cudaEventRecord(ev, s));
+    GBMM_TRY(recon(0, 0, s7));
+    if (!g->post.empty()) {
+        if (side) GBMM_CUDA_TRY(cudaStreamWaitEvent(s2, ev, 0));
+        for (auto &fn : g->post) GBMM_TRY(fn(side ? s2 : s));
+    }
+    GBMM_TRY(recon(0, 1, s));
     return GBMM_OK;
 }
 

@@ -169,7 +169,8 @@ void crt_group_post(crt_group *g, std::function<gbmm_status(cudaStream_t)> f);
 size_t crt_group_ws(int la, int lb, int m, int k, int n);
 // the stage records as one blob (built once every product is added); it goes to
 // device memory 128-byte aligned, and crt_group_launch reads it there.  The post
-// steps run on s2 (after `ev`, recorded on s) when s2 is given, else on s.
+// steps and the reconstructions by base-128 tables beside base-256 ones run on s2 (after `ev`,
+// recorded on s) when s2 is given, else on s; the caller joins both.
 const std::vector<char> &crt_group_blob(crt_group *g);
 gbmm_status crt_group_launch(crt_group *g, const char *d_blob, cudaStream_t s, cudaStream_t s2, cudaEvent_t ev);
 // Stage hooks the host-buffer pipeline hands to one single-pass CRT product
