@@ -2242,13 +2242,46 @@ static void build_tables_host(int P, crt_tables_host &o, int db = 7) {
     }
 }
 
+// Whether the columns of the top base-256 digits stay below the bound: the Mod / p share their
+// leading digits, the moduli being close together, so these columns alone can pass it (36 of the
+// moduli counts up to 940, all from 739 on).  Read off Mod's top 13 to 14 bytes before a table is
+// built: building base 256, then base 128 took 9.9 ms at 922 moduli, base 128 alone 7.5.
+static bool top_digits_fit(int P) {
+    if (2 * P * 128 * 128 < (1 << 24)) return true;
+    const auto &pr = primes_desc();
+    unsigned __int128 mod = 1;  // Mod without its low bytes
+    for (int i = 0; i < P; i++)
+        for (mod *= pr[i]; mod >> 112;) mod >>= 8;
+    int64_t sum[16] = {};
+    for (int i = 0; i < P; i++) {
+        unsigned __int128 q = mod / (unsigned)pr[i] >> 32;  // (the low bytes lack what was dropped)
+        for (int t = 0, c = 0; t < 12; t++, q >>= 8) {
+            const int v = (int)(q & 255u) + c;
+            c = v >= 128;
+            const int d = std::abs(v - (c << 8));
+            sum[t] += d;      // the low digit's factor
+            sum[t + 1] += d;  // the high digit's, 256 times it
+        }
+    }
+    return 128 * *std::max_element(sum, sum + 16) < (1 << 24);
+}
+
+// The table of P moduli in the larger digits that its columns allow; returns the builds it took.
+static int build_tables_fit(int P, crt_tables_host &o) {
+    int builds = 0;
+    if (P <= RECON256_MAX_P && top_digits_fit(P)) {
+        build_tables_host(P, o, 8);
+        builds++;
+        if (o.bound < 16777216.0) return builds;
+        o = crt_tables_host();
+    }
+    build_tables_host(P, o, 7);
+    return builds + 1;
+}
+
 static gbmm_status build_tables(crt_tables *t, int P) {
     crt_tables_host o;
-    if (P <= RECON256_MAX_P) build_tables_host(P, o, 8);
-    if (P > RECON256_MAX_P || o.bound >= 16777216.0) {
-        o = crt_tables_host();
-        build_tables_host(P, o, 7);
-    }
+    build_tables_fit(P, o);
     t->db = o.db;
     t->P = o.P;
     t->Pp = o.Pp;
@@ -3288,6 +3321,15 @@ extern "C" uint64_t gbmmx_table_build(int32_t P, double *ms) {
     mix(o.vtab.data(), o.vtab.size() * 4);
     mix(o.mods.data(), o.mods.size() * sizeof(ModConst));
     return h;
+}
+
+// Test hook: bits of a digit of the table that P moduli get, and the builds that took.
+extern "C" int32_t gbmmx_table_digits(int32_t P, int32_t *builds) {
+    if (P < 1 || P > 2 * CMOD_PAIRS) return 0;
+    crt_tables_host o;
+    const int n = build_tables_fit(P, o);
+    if (builds) *builds = n;
+    return o.db;
 }
 
 // Test hook: launch the four stages' kernels with programmatic stream
